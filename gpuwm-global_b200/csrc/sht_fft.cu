@@ -15,6 +15,22 @@
 // into a length-L complex sequence and inverted; the result equals
 // irfft(nlon * W) of the reference (transform.py:1654-1702), which discards
 // Imag(W_0) and has no Nyquist term because T < nlon/2.
+//
+// Any even nlon in FP32 and FP64 (the register kernels of sht_fft_fast.cu
+// take nlon = 64 F in FP32).  A CTA transforms 2^lr rows of one latitude pair
+// together, held row-innermost in shared memory ([k][row]): every thread
+// keeps one row through all passes, so no pass divides an index by a run-time
+// row or butterfly count, shared accesses are consecutive, and the threads of
+// one butterfly column read their twiddles as broadcasts.  What bounds it is
+// the chain of passes, a barrier apart, so the radix plan takes the fewest
+// passes, radices up to 16, and three CTAs (two in FP64) share an SM.  Against
+// a kernel that held rows one after another, divided indices in every pass and
+// had 24 of 256 threads busy in a radix-16 pass (forward / inverse): T62 x 161
+// planes in FP64 on 94 x 192, 94 / 58 -> 19 / 19 us; T300 x 41 planes in FP32
+// on 452 x 960, 162 / 171 -> 73 / 67 us (1.6 TB/s); T21, one plane, 12.8 /
+// 13.6 -> 3.4 / 3.8 us.
+#include <algorithm>
+
 #include "sht_plan.h"
 
 namespace sht {
@@ -33,414 +49,515 @@ __device__ __forceinline__ V2<T> csub(V2<T> a, V2<T> b) { return mk2<T>(a.x - b.
 template <typename T>
 __device__ __forceinline__ V2<T> cconj(V2<T> a) { return mk2<T>(a.x, -a.y); }
 // multiply by -i (forward) or +i (inverse)
-template <typename T>
-__device__ __forceinline__ V2<T> rot90(V2<T> a, bool inv) {
-  return inv ? mk2<T>(-a.y, a.x) : mk2<T>(a.y, -a.x);
+template <typename T, bool INV>
+__device__ __forceinline__ V2<T> rot90(V2<T> a) {
+  return INV ? mk2<T>(-a.y, a.x) : mk2<T>(a.y, -a.x);
+}
+// multiply by (c, -s) forward, (c, s) inverse
+template <typename T, bool INV>
+__device__ __forceinline__ V2<T> turn(V2<T> a, double c, double s) {
+  return cmul<T>(a, mk2<T>(T(c), INV ? T(s) : T(-s)));
 }
 
-// In-register DFTs of small radix.  Forward uses exp(-2 pi i rs/R).
-template <typename T>
-__device__ __forceinline__ void dft2(V2<T>* v) {
-  V2<T> a = v[0], b = v[1];
-  v[0] = cadd<T>(a, b);
-  v[1] = csub<T>(a, b);
+// In-register DFTs, forward with exp(-2 pi i rs / R), natural order in and out.
+template <typename T, bool INV>
+__device__ __forceinline__ void dft2(V2<T>& a, V2<T>& b) {
+  const V2<T> t = a;
+  a = cadd<T>(t, b);
+  b = csub<T>(t, b);
 }
-template <typename T>
-__device__ __forceinline__ void dft3(V2<T>* v, bool inv) {
-  const T c1 = T(-0.5);
-  const T s1 = inv ? T(0.86602540378443864676) : T(-0.86602540378443864676);
-  V2<T> a = v[0], b = v[1], c = v[2];
-  V2<T> t1 = cadd<T>(b, c), t2 = csub<T>(b, c);
-  v[0] = cadd<T>(a, t1);
-  V2<T> m1 = mk2<T>(a.x + c1 * t1.x, a.y + c1 * t1.y);
-  V2<T> m2 = mk2<T>(-s1 * t2.y, s1 * t2.x);  // i * s1 * t2
-  v[1] = cadd<T>(m1, m2);
-  v[2] = csub<T>(m1, m2);
-}
-template <typename T>
-__device__ __forceinline__ void dft4(V2<T>* v, bool inv) {
-  V2<T> a0 = cadd<T>(v[0], v[2]), a1 = csub<T>(v[0], v[2]);
-  V2<T> b0 = cadd<T>(v[1], v[3]), b1 = rot90<T>(csub<T>(v[1], v[3]), inv);
+template <typename T, bool INV>
+__device__ __forceinline__ void dft4(V2<T>* v) {
+  const V2<T> a0 = cadd<T>(v[0], v[2]), a1 = csub<T>(v[0], v[2]);
+  const V2<T> b0 = cadd<T>(v[1], v[3]), b1 = rot90<T, INV>(csub<T>(v[1], v[3]));
   v[0] = cadd<T>(a0, b0);
   v[2] = csub<T>(a0, b0);
   v[1] = cadd<T>(a1, b1);
   v[3] = csub<T>(a1, b1);
 }
-template <typename T>
-__device__ __forceinline__ void dft5(V2<T>* v, bool inv) {
-  const T c1 = T(0.30901699437494742410), c2 = T(-0.80901699437494742410);
-  const T s1 = inv ? T(0.95105651629515357212) : T(-0.95105651629515357212);
-  const T s2 = inv ? T(0.58778525229247312917) : T(-0.58778525229247312917);
-  V2<T> a = v[0];
-  V2<T> t1 = cadd<T>(v[1], v[4]), t2 = csub<T>(v[1], v[4]);
-  V2<T> t3 = cadd<T>(v[2], v[3]), t4 = csub<T>(v[2], v[3]);
-  v[0] = mk2<T>(a.x + t1.x + t3.x, a.y + t1.y + t3.y);
-  V2<T> r1 = mk2<T>(a.x + c1 * t1.x + c2 * t3.x, a.y + c1 * t1.y + c2 * t3.y);
-  V2<T> r2 = mk2<T>(a.x + c2 * t1.x + c1 * t3.x, a.y + c2 * t1.y + c1 * t3.y);
-  // i*(s1 t2 + s2 t4) and i*(s2 t2 - s1 t4)
-  V2<T> i1 = mk2<T>(-(s1 * t2.y + s2 * t4.y), s1 * t2.x + s2 * t4.x);
-  V2<T> i2 = mk2<T>(-(s2 * t2.y - s1 * t4.y), s2 * t2.x - s1 * t4.x);
-  v[1] = cadd<T>(r1, i1);
-  v[4] = csub<T>(r1, i1);
-  v[2] = cadd<T>(r2, i2);
-  v[3] = csub<T>(r2, i2);
-}
-template <typename T>
-__device__ __forceinline__ void dft8(V2<T>* v, bool inv) {
-  // radix-2 x 4: even/odd halves then combine with exp(-2 pi i k/8).
+template <typename T, bool INV>
+__device__ __forceinline__ void dft8(V2<T>* v) {
   V2<T> e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
-  dft4<T>(e, inv);
-  dft4<T>(o, inv);
-  const T r = T(0.70710678118654752440);
-  // w^1 = (r, -r) forward, (r, r) inverse; w^2 = -i / +i; w^3 = (-r, -r) / (-r, r)
-  o[1] = cmul<T>(o[1], mk2<T>(r, inv ? r : -r));
-  o[2] = rot90<T>(o[2], inv);
-  o[3] = cmul<T>(o[3], mk2<T>(-r, inv ? r : -r));
+  dft4<T, INV>(e);
+  dft4<T, INV>(o);
+  constexpr double r = 0.70710678118654752440;
+  o[1] = turn<T, INV>(o[1], r, r);
+  o[2] = rot90<T, INV>(o[2]);
+  o[3] = turn<T, INV>(o[3], -r, r);
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     v[k] = cadd<T>(e[k], o[k]);
     v[k + 4] = csub<T>(e[k], o[k]);
   }
 }
-template <typename T>
-__device__ __forceinline__ void dft16(V2<T>* v, const V2<T>* w16, bool inv) {
-  // 4 x 4: columns, twiddle, rows.  w16[k] = exp(-2 pi i k / 16).
-  V2<T> a[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) a[i][j] = v[j * 4 + i];
-    dft4<T>(a[i], inv);
+
+// cos and sin of 2 pi k / R, k <= R / 2, of the odd prime radices.
+template <int R> struct OddTrig;
+template <> struct OddTrig<3> {
+  static __device__ __forceinline__ double c(int k) { const double t[] = {1.0, -0.5}; return t[k]; }
+  static __device__ __forceinline__ double s(int k) { const double t[] = {0.0, 0.866025403784438646764}; return t[k]; }
+};
+template <> struct OddTrig<5> {
+  static __device__ __forceinline__ double c(int k) {
+    const double t[] = {1.0, 0.309016994374947424102, -0.809016994374947424102};
+    return t[k];
   }
+  static __device__ __forceinline__ double s(int k) {
+    const double t[] = {0.0, 0.951056516295153572116, 0.587785252292473129169};
+    return t[k];
+  }
+};
+template <> struct OddTrig<7> {
+  static __device__ __forceinline__ double c(int k) {
+    const double t[] = {1.0, 0.623489801858733530525, -0.222520933956314404289, -0.900968867902419126236};
+    return t[k];
+  }
+  static __device__ __forceinline__ double s(int k) {
+    const double t[] = {0.0, 0.781831482468029808708, 0.974927912181823607018, 0.433883739117558120476};
+    return t[k];
+  }
+};
+template <> struct OddTrig<11> {
+  static __device__ __forceinline__ double c(int k) {
+    const double t[] = {1.0, 0.841253532831181168862, 0.415415013001886425529,
+                        -0.142314838273285140444, -0.654860733945285064057, -0.95949297361449738989};
+    return t[k];
+  }
+  static __device__ __forceinline__ double s(int k) {
+    const double t[] = {0.0, 0.540640817455597582108, 0.909631995354518371412,
+                        0.989821441880932732376, 0.755749574354258283774, 0.281732556841429697711};
+    return t[k];
+  }
+};
+template <> struct OddTrig<13> {
+  static __device__ __forceinline__ double c(int k) {
+    const double t[] = {1.0, 0.8854560256532098959, 0.568064746731155802512, 0.120536680255323053349,
+                        -0.35460488704253562597, -0.748510748171101098635, -0.970941817426052027157};
+    return t[k];
+  }
+  static __device__ __forceinline__ double s(int k) {
+    const double t[] = {0.0, 0.464723172043768545656, 0.82298386589365639458, 0.992708874098053992801,
+                        0.93501624268541482344, 0.663122658240795202377, 0.239315664287557767149};
+    return t[k];
+  }
+};
+// Odd prime R by pairs: with t_i = v_i + v_{R-i} and u_i = v_i - v_{R-i},
+// X_k, X_{R-k} = v_0 + sum_i cos(ik) t_i -+ i sum_i sin(ik) u_i.
+template <typename T, bool INV, int R>
+__device__ __forceinline__ void dft_odd(V2<T>* v) {
+  constexpr int H = R / 2;
+  V2<T> t[H], u[H];
+  V2<T> sum = v[0];
 #pragma unroll
-  for (int i = 1; i < 4; ++i)
+  for (int i = 1; i <= H; ++i) {
+    t[i - 1] = cadd<T>(v[i], v[R - i]);
+    u[i - 1] = csub<T>(v[i], v[R - i]);
+    sum = cadd<T>(sum, t[i - 1]);
+  }
+  const V2<T> v0 = v[0];
+  v[0] = sum;
 #pragma unroll
-    for (int j = 1; j < 4; ++j) {
-      V2<T> t = w16[i * j];
-      a[i][j] = cmul<T>(a[i][j], inv ? cconj<T>(t) : t);
+  for (int k = 1; k <= H; ++k) {
+    V2<T> a = v0, b = mk2<T>(T(0), T(0));
+#pragma unroll
+    for (int i = 1; i <= H; ++i) {
+      const int e = (i * k) % R;
+      const T c = T(OddTrig<R>::c(e <= H ? e : R - e));
+      const T s = T(e <= H ? OddTrig<R>::s(e) : -OddTrig<R>::s(R - e));
+      a.x += c * t[i - 1].x;
+      a.y += c * t[i - 1].y;
+      b.x += s * u[i - 1].x;
+      b.y += s * u[i - 1].y;
     }
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    V2<T> b[4] = {a[0][j], a[1][j], a[2][j], a[3][j]};
-    dft4<T>(b, inv);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) v[i * 4 + j] = b[i];
+    const V2<T> ib = rot90<T, INV>(b);
+    v[k] = cadd<T>(a, ib);
+    v[R - k] = csub<T>(a, ib);
   }
 }
 
+template <typename T, bool INV, int R>
+__device__ __forceinline__ void dft(V2<T>* v);
+
+// R = A B with A and B coprime (Good-Thomas): no twiddles; element
+// (B a + A b) mod R in, (B Bi k1 + A Ai k2) mod R out, Bi = B^-1 mod A.
+constexpr int inverse_mod(int x, int n) {
+  for (int i = 1; i < n; ++i)
+    if ((x * i) % n == 1) return i;
+  return 1;
+}
+template <typename T, bool INV, int A, int B>
+__device__ __forceinline__ void dft_coprime(V2<T>* v) {
+  constexpr int R = A * B, EB = B * inverse_mod(B % A, A), EA = A * inverse_mod(A % B, B);
+  V2<T> w[A][B];
+#pragma unroll
+  for (int a = 0; a < A; ++a) {
+#pragma unroll
+    for (int b = 0; b < B; ++b) w[a][b] = v[(B * a + A * b) % R];
+    dft<T, INV, B>(w[a]);
+  }
+#pragma unroll
+  for (int b = 0; b < B; ++b) {
+    V2<T> c[A];
+#pragma unroll
+    for (int a = 0; a < A; ++a) c[a] = w[a][b];
+    dft<T, INV, A>(c);
+#pragma unroll
+    for (int a = 0; a < A; ++a) v[(EB * a + EA * b) % R] = c[a];
+  }
+}
+// R = A x A: columns, twiddles exp(-2 pi i ij / R), rows.
+template <typename T, bool INV, int A>
+__device__ __forceinline__ void dft_square(V2<T>* v) {
+  V2<T> w[A][A];
+#pragma unroll
+  for (int i = 0; i < A; ++i) {
+#pragma unroll
+    for (int j = 0; j < A; ++j) w[i][j] = v[j * A + i];
+    dft<T, INV, A>(w[i]);
+  }
+  if constexpr (A == 3) {
+    w[1][1] = turn<T, INV>(w[1][1], 0.766044443118978035202, 0.642787609686539326323);
+    w[1][2] = turn<T, INV>(w[1][2], 0.173648177666930348852, 0.984807753012208059367);
+    w[2][1] = turn<T, INV>(w[2][1], 0.173648177666930348852, 0.984807753012208059367);
+    w[2][2] = turn<T, INV>(w[2][2], -0.939692620785908384054, 0.342020143325668733044);
+  } else {
+    constexpr double c1 = 0.923879532511286756128, s1 = 0.382683432365089771728;
+    constexpr double r = 0.70710678118654752440;
+    w[1][1] = turn<T, INV>(w[1][1], c1, s1);
+    w[1][2] = turn<T, INV>(w[1][2], r, r);
+    w[1][3] = turn<T, INV>(w[1][3], s1, c1);
+    w[2][1] = turn<T, INV>(w[2][1], r, r);
+    w[2][2] = rot90<T, INV>(w[2][2]);
+    w[2][3] = turn<T, INV>(w[2][3], -r, r);
+    w[3][1] = turn<T, INV>(w[3][1], s1, c1);
+    w[3][2] = turn<T, INV>(w[3][2], -r, r);
+    w[3][3] = turn<T, INV>(w[3][3], -c1, -s1);
+  }
+#pragma unroll
+  for (int j = 0; j < A; ++j) {
+    V2<T> c[A];
+#pragma unroll
+    for (int i = 0; i < A; ++i) c[i] = w[i][j];
+    dft<T, INV, A>(c);
+#pragma unroll
+    for (int i = 0; i < A; ++i) v[i * A + j] = c[i];
+  }
+}
+template <typename T, bool INV, int R>
+__device__ __forceinline__ void dft(V2<T>* v) {
+  if constexpr (R == 2) dft2<T, INV>(v[0], v[1]);
+  else if constexpr (R == 4) dft4<T, INV>(v);
+  else if constexpr (R == 8) dft8<T, INV>(v);
+  else if constexpr (R == 6) dft_coprime<T, INV, 2, 3>(v);
+  else if constexpr (R == 10) dft_coprime<T, INV, 2, 5>(v);
+  else if constexpr (R == 12) dft_coprime<T, INV, 4, 3>(v);
+  else if constexpr (R == 15) dft_coprime<T, INV, 3, 5>(v);
+  else if constexpr (R == 9) dft_square<T, INV, 3>(v);
+  else if constexpr (R == 16) dft_square<T, INV, 4>(v);
+  else dft_odd<T, INV, R>(v);
+}
+
+// ------------------------------------------------------------------ passes
+constexpr int kMaxPass = 24;
+struct FftPass {
+  int R;           // radix
+  int Ns;          // product of the earlier radices
+  int nb;          // butterflies per row, L / R
+  int stride;      // twiddle stride, L / (Ns R)
+  unsigned magic;  // ceil(2^32 / Ns): j / Ns = umulhi(j, magic) for j < 2^16, Ns > 1
+};
 struct FftShape {
-  int L;        // complex length nlon/2
-  int Lp;       // padded row stride in the shared buffers
-  int nrad;
-  int rad[24];  // radix sequence
+  int L;     // complex length nlon / 2
+  int lc;    // log2 of the waist columns (plane, field) of a CTA
+  int rs;    // shared row stride: entry k of row g lies at k * rs + g
+  int npass;
+  int tw_shared;  // 1: the twiddle table is staged in shared memory
+  FftPass pass[kMaxPass];
 };
 
-// One Stockham pass (radix R, Ns = product of earlier radices) over `rows`
-// rows held in shared memory; twiddles from the table exp(-2 pi i k / L).
-template <typename T, int R>
-__device__ void pass_fixed(const V2<T>* in, V2<T>* out, const FftShape& f, int Ns, int rows,
-                           const V2<T>* __restrict__ tw, const V2<T>* w16, bool inv) {
-  const int nb = f.L / R;
-  const int stride = f.L / (Ns * R);
-  for (int t = threadIdx.x; t < rows * nb; t += blockDim.x) {
-    int g = t / nb, j = t - g * nb;
-    const V2<T>* src = in + g * f.Lp;
-    V2<T>* dst = out + g * f.Lp;
-    int k = j % Ns;
+// One Stockham pass; thread -> row g = tid % rows (fixed), butterflies
+// j = tid / rows, + blockDim / rows, ...
+template <typename T, bool INV, int R>
+__device__ __forceinline__ void pass_fixed(const V2<T>* in, V2<T>* out, const FftShape& f,
+                                           const FftPass& p, int lr, const V2<T>* tw) {
+  const int row = threadIdx.x & ((1 << lr) - 1), step = blockDim.x >> lr;
+  const int nb = p.nb, Ns = p.Ns, rs = f.rs;
+  for (int j = threadIdx.x >> lr; j < nb; j += step) {
+    const V2<T>* src = in + j * rs + row;
     V2<T> v[R];
 #pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = src[j + r * nb];
+    for (int r = 0; r < R; ++r) v[r] = src[r * nb * rs];
+    const int q = Ns > 1 ? (int)__umulhi((unsigned)j, p.magic) : j;
+    const int k = j - q * Ns;
     if (Ns > 1) {
+      const V2<T>* w = tw + k * p.stride;
 #pragma unroll
       for (int r = 1; r < R; ++r) {
-        V2<T> w = tw[k * r * stride];
-        v[r] = cmul<T>(v[r], inv ? cconj<T>(w) : w);
+        const V2<T> t = w[k * (r - 1) * p.stride];
+        v[r] = cmul<T>(v[r], INV ? cconj<T>(t) : t);
       }
     }
-    if (R == 2) dft2<T>(v);
-    if (R == 3) dft3<T>(v, inv);
-    if (R == 4) dft4<T>(v, inv);
-    if (R == 5) dft5<T>(v, inv);
-    if (R == 8) dft8<T>(v, inv);
-    if (R == 16) dft16<T>(v, w16, inv);
-    int base = (j / Ns) * Ns * R + k;
+    dft<T, INV, R>(v);
+    V2<T>* dst = out + (q * Ns * R + k) * rs + row;
 #pragma unroll
-    for (int r = 0; r < R; ++r) dst[base + r * Ns] = v[r];
+    for (int r = 0; r < R; ++r) dst[r * Ns * rs] = v[r];
   }
 }
 
-// Generic odd-prime radix: direct DFT of the twiddled inputs.
-template <typename T>
-__device__ void pass_generic(const V2<T>* in, V2<T>* out, const FftShape& f, int Ns, int R,
-                             int rows, const V2<T>* __restrict__ tw, bool inv) {
-  const int nb = f.L / R;
-  const int stride = f.L / (Ns * R);
-  const int rstride = f.L / R;
-  for (int t = threadIdx.x; t < rows * nb; t += blockDim.x) {
-    int g = t / nb, j = t - g * nb;
-    const V2<T>* src = in + g * f.Lp;
-    V2<T>* dst = out + g * f.Lp;
-    int k = j % Ns;
-    int base = (j / Ns) * Ns * R + k;
-    for (int s = 0; s < R; ++s) {
-      V2<T> acc = mk2<T>(T(0), T(0));
-      for (int r = 0; r < R; ++r) {
-        V2<T> v = src[j + r * nb];
-        int idx = (k * r * stride + ((r * s) % R) * rstride) % f.L;
-        V2<T> w = tw[idx];
-        v = cmul<T>(v, inv ? cconj<T>(w) : w);
-        acc = cadd<T>(acc, v);
-      }
-      dst[base + s * Ns] = acc;
+// Any other prime radix: direct DFT of the twiddled inputs.
+template <typename T, bool INV>
+__device__ __noinline__ void pass_generic(const V2<T>* in, V2<T>* out, const FftShape& f,
+                                          const FftPass& p, int lr, const V2<T>* tw) {
+  const int row = threadIdx.x & ((1 << lr) - 1), step = blockDim.x >> lr;
+  const int nb = p.nb, Ns = p.Ns, R = p.R, rs = f.rs;
+  for (int e = threadIdx.x >> lr; e < f.L; e += step) {
+    const int s = e / nb, j = e - s * nb;  // output s of butterfly j
+    const int q = Ns > 1 ? (int)__umulhi((unsigned)j, p.magic) : j;
+    const int k = j - q * Ns;
+    const int inc = (k * p.stride + s * nb) % f.L;  // twiddle and DFT phase per input
+    V2<T> acc = mk2<T>(T(0), T(0));
+    for (int r = 0, idx = 0; r < R; ++r) {
+      const V2<T> w = tw[idx];
+      acc = cadd<T>(acc, cmul<T>(in[(j + r * nb) * rs + row], INV ? cconj<T>(w) : w));
+      idx += inc;
+      if (idx >= f.L) idx -= f.L;
     }
+    out[(q * Ns * R + k + s * Ns) * rs + row] = acc;
   }
 }
 
-// Runs the radix sequence; returns the buffer that holds the result.
-template <typename T>
-__device__ V2<T>* run_passes(V2<T>* a, V2<T>* b, const FftShape& f, int rows,
-                             const V2<T>* __restrict__ tw, const V2<T>* w16, bool inv) {
-  int Ns = 1;
-  for (int p = 0; p < f.nrad; ++p) {
-    int R = f.rad[p];
-    switch (R) {
-      case 2: pass_fixed<T, 2>(a, b, f, Ns, rows, tw, w16, inv); break;
-      case 3: pass_fixed<T, 3>(a, b, f, Ns, rows, tw, w16, inv); break;
-      case 4: pass_fixed<T, 4>(a, b, f, Ns, rows, tw, w16, inv); break;
-      case 5: pass_fixed<T, 5>(a, b, f, Ns, rows, tw, w16, inv); break;
-      case 8: pass_fixed<T, 8>(a, b, f, Ns, rows, tw, w16, inv); break;
-      case 16: pass_fixed<T, 16>(a, b, f, Ns, rows, tw, w16, inv); break;
-      default: pass_generic<T>(a, b, f, Ns, R, rows, tw, inv); break;
+// Runs the passes (a barrier after each); returns the buffer with the result.
+template <typename T, bool INV>
+__device__ __forceinline__ V2<T>* run_passes(V2<T>* a, V2<T>* b, const FftShape& f, int lr,
+                                             const V2<T>* tw) {
+  for (int i = 0; i < f.npass; ++i) {
+    const FftPass& p = f.pass[i];
+    switch (p.R) {
+      case 2: pass_fixed<T, INV, 2>(a, b, f, p, lr, tw); break;
+      case 3: pass_fixed<T, INV, 3>(a, b, f, p, lr, tw); break;
+      case 4: pass_fixed<T, INV, 4>(a, b, f, p, lr, tw); break;
+      case 5: pass_fixed<T, INV, 5>(a, b, f, p, lr, tw); break;
+      case 6: pass_fixed<T, INV, 6>(a, b, f, p, lr, tw); break;
+      case 7: pass_fixed<T, INV, 7>(a, b, f, p, lr, tw); break;
+      case 8: pass_fixed<T, INV, 8>(a, b, f, p, lr, tw); break;
+      case 9: pass_fixed<T, INV, 9>(a, b, f, p, lr, tw); break;
+      case 10: pass_fixed<T, INV, 10>(a, b, f, p, lr, tw); break;
+      case 11: pass_fixed<T, INV, 11>(a, b, f, p, lr, tw); break;
+      case 12: pass_fixed<T, INV, 12>(a, b, f, p, lr, tw); break;
+      case 13: pass_fixed<T, INV, 13>(a, b, f, p, lr, tw); break;
+      case 15: pass_fixed<T, INV, 15>(a, b, f, p, lr, tw); break;
+      case 16: pass_fixed<T, INV, 16>(a, b, f, p, lr, tw); break;
+      default: pass_generic<T, INV>(a, b, f, p, lr, tw); break;
     }
     __syncthreads();
     V2<T>* t = a;
     a = b;
     b = t;
-    Ns *= R;
   }
   return a;
 }
 
+// The twiddle table exp(-2 pi i k / L): its shared copy (filled here; the
+// caller's next barrier publishes it) or the table in global memory.
+template <typename T>
+__device__ __forceinline__ const V2<T>* stage_twiddles(const FftShape& f, V2<T>* room,
+                                                       const V2<T>* __restrict__ tw_l) {
+  if (!f.tw_shared) return tw_l;
+  for (int k = threadIdx.x; k < f.L; k += blockDim.x) room[k] = tw_l[k];
+  return room;
+}
+
+// ----------------------------------------------------------------- forward
 struct FoldArgs {
   FftShape f;
   int nlat, nlon, T, H, nlat_odd;
-  int G;        // planes per CTA
-  int F;        // fields stacked per plane (1 scalar, 2 for (u, v))
-  int64_t planes;
+  int F;         // fields stacked per plane (1 scalar, 2 for (u, v))
+  int64_t cols;  // waist columns, planes * F
 };
 
-template <typename T>
-__device__ void load_w16(V2<T>* w16, const V2<T>* tw, int L) {
-  if (threadIdx.x < 16) {
-    // exp(-2 pi i k/16) = tw[k L/16] when 16 | L, else computed
-    if (L % 16 == 0) {
-      w16[threadIdx.x] = tw[threadIdx.x * (L / 16)];
-    } else {
-      double s, c;
-      sincospi(-2.0 * threadIdx.x / 16.0, &s, &c);
-      w16[threadIdx.x] = mk2<T>(T(c), T(s));
-    }
-  }
-}
-
 // grid (planes, nlat, nlon) per field -> waist [m][s][h][r], r = (p*F + f)*2 + c.
+// Row g of a CTA: side g >> lc (the latitude, its mirror) of column g % 2^lc.
 template <typename T>
-__global__ void forward_fold_kernel(FoldArgs a, const T* __restrict__ g0,
-                                    const T* __restrict__ g1, const V2<T>* __restrict__ tw_l,
-                                    const V2<T>* __restrict__ tw_n, T* __restrict__ wfold,
-                                    float* __restrict__ rowmax) {
-  extern __shared__ unsigned char smem_raw[];
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) forward_fold_kernel(
+    const __grid_constant__ FoldArgs a, const T* __restrict__ g0, const T* __restrict__ g1,
+    const V2<T>* __restrict__ tw_l, const V2<T>* __restrict__ tw_n, T* __restrict__ wfold,
+    float* __restrict__ rowmax) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int L = a.f.L, lc = a.f.lc, lr = lc + 1, rs = a.f.rs;
   V2<T>* bufA = reinterpret_cast<V2<T>*>(smem_raw);
-  const int h = blockIdx.x;
-  const int64_t p0 = (int64_t)blockIdx.y * a.G;
+  V2<T>* bufB = bufA + L * rs;
+  const int h = blockIdx.y;
+  const int64_t c0 = (int64_t)blockIdx.x << lc;
   const bool eq = a.nlat_odd && h == a.H - 1;
-  const int rpp = eq ? 1 : 2;              // rows per (plane, field)
-  const int rows = a.G * a.F * rpp;
-  const int Lp = a.f.Lp;
-  V2<T>* bufB = bufA + rows * Lp;
-  __shared__ V2<T> w16[16];
-  load_w16<T>(w16, tw_l, a.f.L);
-
-  // Load rows: row index ((gp*F + f)*rpp + side).
-  for (int t = threadIdx.x; t < rows * a.f.L; t += blockDim.x) {
-    int row = t / a.f.L, k = t - row * a.f.L;
-    int side = row % rpp, pf = row / rpp;
-    int f = pf % a.F, gp = pf / a.F;
-    int64_t plane = p0 + gp;
-    V2<T> v = mk2<T>(T(0), T(0));
-    if (plane < a.planes) {
-      int j = side ? (a.nlat - 1 - h) : h;
-      const T* src = (f ? g1 : g0) + (plane * a.nlat + j) * (int64_t)a.nlon;
-      v = reinterpret_cast<const V2<T>*>(src)[k];
-    }
-    bufA[row * Lp + k] = v;
+  const int fsh = a.F - 1;  // log2 of the field count (1 or 2)
+  const V2<T>* tw = stage_twiddles<T>(a.f, bufB + L * rs, tw_l);
+  // Loads: four neighbouring k of a row per quad of lanes (one 32-byte
+  // sector in FP32), rows across the quads; each thread stays on one row.
+  {
+    const int row = (threadIdx.x >> 2) & ((1 << lr) - 1);
+    const int64_t col = min(c0 + (row & ((1 << lc) - 1)), a.cols - 1);  // past the end: any live column
+    const int j = (row >> lc) && !eq ? a.nlat - 1 - h : h;
+    const V2<T>* src = reinterpret_cast<const V2<T>*>(
+        ((col & fsh) ? g1 : g0) + ((col >> fsh) * a.nlat + j) * (int64_t)a.nlon);
+    const int kstep = blockDim.x >> lr;
+#pragma unroll 4
+    for (int k = ((threadIdx.x >> (2 + lr)) << 2) + (threadIdx.x & 3); k < L; k += kstep)
+      bufA[k * rs + row] = src[k];
   }
   __syncthreads();
-  V2<T>* Z = run_passes<T>(bufA, bufB, a.f, rows, tw_l, w16, false);
+  const V2<T>* Z = run_passes<T, false>(bufA, bufB, a.f, lr, tw);
 
-  // Untangle, scale, fold, write.  Thread -> (m, gp, f) with (gp, f) fastest.
-  const int L = a.f.L;
-  const int nper = a.G * a.F;
-  const int64_t R = a.planes * a.F * 2;
-  const T inv_n = T(1) / T(a.nlon);
+  // Untangle, scale, fold, write.  Thread -> (m, column), columns fastest.
+  const int q = threadIdx.x & ((1 << lc) - 1), mstep = blockDim.x >> lc;
+  const T half_inv_n = T(0.5) / T(a.nlon);
   V2<T>* out = reinterpret_cast<V2<T>*>(wfold);
-  float mre = 0.f, mim = 0.f;  // this thread's column maxima (pf = tid % nper)
-  for (int t = threadIdx.x; t < (a.T + 1) * nper; t += blockDim.x) {
-    int m = t / nper, pf = t - m * nper;
-    int gp = pf / a.F;
-    if (p0 + gp >= a.planes) continue;
-    V2<T> X[2];
-    V2<T> w = tw_n[m];
-    for (int side = 0; side < rpp; ++side) {
-      const V2<T>* zr = Z + (pf * rpp + side) * Lp;
-      V2<T> zk = zr[m];
-      V2<T> zc = cconj<T>(zr[m == 0 ? 0 : L - m]);
-      V2<T> ev = cadd<T>(zk, zc);   // 2 * even part
-      V2<T> od = csub<T>(zk, zc);   // 2 * i * odd part
-      // X = (ev - i w od) / 2
-      V2<T> t1 = cmul<T>(w, od);
-      V2<T> xm = mk2<T>(T(0.5) * (ev.x + t1.y), T(0.5) * (ev.y - t1.x));
-      X[side] = mk2<T>(xm.x * inv_n, xm.y * inv_n);
+  const V2<T>*z0 = Z + q, *z1 = Z + q + (1 << lc);
+  const bool live = c0 + q < a.cols;
+  float mre = 0.f, mim = 0.f;  // this thread's column maxima
+  if (live) {
+    const int64_t dsd = (int64_t)a.H * a.cols;  // S row -> D row of the same order
+    V2<T>* dst = out + ((int64_t)(2 * (threadIdx.x >> lc)) * a.H + h) * a.cols + c0 + q;
+    for (int m = threadIdx.x >> lc; m <= a.T; m += mstep, dst += 2 * mstep * dsd) {
+      const V2<T> w = tw_n[m];
+      const int mc = m == 0 ? 0 : L - m;
+      V2<T> X[2];
+#pragma unroll
+      for (int sd = 0; sd < 2; ++sd) {
+        const V2<T>* z = sd ? z1 : z0;
+        const V2<T> zk = z[m * rs], zc = cconj<T>(z[mc * rs]);
+        const V2<T> ev = cadd<T>(zk, zc);  // 2 * even part
+        const V2<T> od = csub<T>(zk, zc);  // 2 * i * odd part
+        const V2<T> t = cmul<T>(w, od);    // X = (ev - i w od) / 2
+        X[sd] = mk2<T>((ev.x + t.y) * half_inv_n, (ev.y - t.x) * half_inv_n);
+      }
+      const V2<T> S = eq ? X[0] : cadd<T>(X[0], X[1]);
+      const V2<T> D = eq ? mk2<T>(T(0), T(0)) : csub<T>(X[0], X[1]);
+      dst[0] = S;
+      dst[dsd] = D;
+      mre = fmaxf(mre, (float)fmax(fabs(S.x), fabs(D.x)));
+      mim = fmaxf(mim, (float)fmax(fabs(S.y), fabs(D.y)));
     }
-    V2<T> S, D;
-    if (rpp == 2) {
-      S = cadd<T>(X[0], X[1]);
-      D = csub<T>(X[0], X[1]);
-    } else {
-      S = X[0];
-      D = mk2<T>(T(0), T(0));
-    }
-    int64_t rr = (p0 * a.F + pf);  // complex column index = r/2
-    int64_t base0 = ((int64_t)(m * 2 + 0) * a.H + h) * (R / 2) + rr;
-    int64_t base1 = ((int64_t)(m * 2 + 1) * a.H + h) * (R / 2) + rr;
-    out[base0] = S;
-    out[base1] = D;
-    mre = fmaxf(mre, (float)fmax(fabs(S.x), fabs(D.x)));
-    mim = fmaxf(mim, (float)fmax(fabs(S.y), fabs(D.y)));
   }
-  if (rowmax != nullptr) {
-    const int pf = threadIdx.x % nper;  // fixed per thread: blockDim % nper == 0
-    rowmax_merge(rowmax, p0 * a.F + pf, p0 + pf / a.F < a.planes, mre, mim, nper);
-  }
+  if (rowmax != nullptr) rowmax_merge(rowmax, c0 + q, live, mre, mim, 1 << lc);
 }
 
+// ----------------------------------------------------------------- inverse
 struct UnfoldArgs {
-  FftShape f;
+  FftShape f;  // 2^lc planes per CTA
   int nlat, nlon, T, H, nlat_odd;
-  int G;
-  int mode;
+  int zonal;   // NF = 1: multiply by i m
   int64_t planes;
   double radius;
 };
 
-// waist(s) -> grid rows.  Waist row index r = (p*F + f)*2 + c with F = 2
-// (psi, chi) in the wind mode and F = 1 otherwise.
-template <typename T>
-__global__ void inverse_unfold_kernel(UnfoldArgs a, const T* __restrict__ wP,
-                                      const T* __restrict__ wD, const double* __restrict__ coslat,
-                                      const V2<T>* __restrict__ tw_l,
-                                      const V2<T>* __restrict__ tw_n, T* __restrict__ out0,
-                                      T* __restrict__ out1) {
-  extern __shared__ unsigned char smem_raw[];
+// waist(s) -> grid rows.  NF waist columns per plane: 1 (scalar, zonal,
+// meridional), 2 (gradient: the P and dP syntheses of one field), 4 (wind: P
+// and dP of psi and chi, stored (psi, chi) per plane).  Row g of a CTA:
+// output field g >> (lc + 1), side (g >> lc) & 1, plane g % 2^lc.
+template <typename T, int NF>
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) inverse_unfold_kernel(
+    const __grid_constant__ UnfoldArgs a, const T* __restrict__ wP, const T* __restrict__ wD,
+    const double* __restrict__ coslat, const V2<T>* __restrict__ tw_l,
+    const V2<T>* __restrict__ tw_n, T* __restrict__ out0, T* __restrict__ out1) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int NO = NF == 1 ? 1 : 2;  // output fields
+  constexpr int FW = NF == 4 ? 2 : 1;  // waist columns per plane and buffer
+  const int L = a.f.L, lc = a.f.lc, lr = lc + NO, rs = a.f.rs;
   V2<T>* bufA = reinterpret_cast<V2<T>*>(smem_raw);
-  const int h = blockIdx.x;
-  const int64_t p0 = (int64_t)blockIdx.y * a.G;
+  V2<T>* bufB = bufA + L * rs;
+  const int h = blockIdx.y;
+  const int64_t p0 = (int64_t)blockIdx.x << lc;
   const bool eq = a.nlat_odd && h == a.H - 1;
-  const int rpp = eq ? 1 : 2;
-  const int NO = (a.mode == kUnfoldGradient || a.mode == kUnfoldWind) ? 2 : 1;
-  const int FW = a.mode == kUnfoldWind ? 2 : 1;  // fields per plane in the waist
-  const int rows = a.G * NO * rpp;
-  const int Lp = a.f.Lp;
-  const int L = a.f.L;
-  V2<T>* bufB = bufA + rows * Lp;
-  __shared__ V2<T> w16[16];
-  load_w16<T>(w16, tw_l, L);
-  const int64_t Rc = a.planes * FW;  // complex columns per waist row block
-  const V2<T>* P2 = reinterpret_cast<const V2<T>*>(wP);
-  const V2<T>* D2 = reinterpret_cast<const V2<T>*>(wD);
-  const T inv_a = T(1.0 / a.radius);
+  const V2<T>* tw = stage_twiddles<T>(a.f, bufB + L * rs, tw_l);
 
-  // Stage 1: Fourier coefficients X_row[m] (m <= T) into bufB, row index
-  // ((gp*NO + o)*rpp + side).
-  for (int t = threadIdx.x; t < (a.T + 1) * a.G; t += blockDim.x) {
-    int m = t / a.G, gp = t - m * a.G;
-    int64_t plane = p0 + gp;
-    if (plane >= a.planes) continue;
-    int j[2] = {h, a.nlat - 1 - h};
-    for (int side = 0; side < rpp; ++side) {
-      T sgn = side ? T(-1) : T(1);
-      T cl = T(coslat[j[side]]);
-      T im_over = T(m) / (T(a.radius) * cl);  // m / (a cos phi)
-      auto fetch = [&](const V2<T>* w, int f) {
-        int64_t c0 = ((int64_t)(m * 2 + 0) * a.H + h) * Rc + plane * FW + f;
-        int64_t c1 = ((int64_t)(m * 2 + 1) * a.H + h) * Rc + plane * FW + f;
-        V2<T> s = w[c0], d = w[c1];
-        return mk2<T>(s.x + sgn * d.x, s.y + sgn * d.y);
-      };
-      V2<T> o0, o1 = mk2<T>(T(0), T(0));
-      if (a.mode == kUnfoldScalar || a.mode == kUnfoldMeridional) {
-        o0 = fetch(P2, 0);
-      } else if (a.mode == kUnfoldZonal) {
-        V2<T> x = fetch(P2, 0);
-        o0 = mk2<T>(-T(m) * x.y, T(m) * x.x);
-      } else if (a.mode == kUnfoldGradient) {
-        V2<T> x = fetch(P2, 0);
-        V2<T> y = fetch(D2, 0);
-        o0 = mk2<T>(-T(m) * x.y, T(m) * x.x);  // i m X (metric factor after the FFT)
-        o1 = y;                                 // dP synthesis (/a after the FFT)
-      } else {  // wind: u = -dpsi/a + i m chi/(a cos); v = i m psi/(a cos) + dchi/a
-        V2<T> xp = fetch(P2, 0), xc = fetch(P2, 1);
-        V2<T> dp = fetch(D2, 0), dc = fetch(D2, 1);
-        o0 = mk2<T>(-dp.x * inv_a - im_over * xc.y, -dp.y * inv_a + im_over * xc.x);
-        o1 = mk2<T>(-im_over * xp.y + dc.x * inv_a, im_over * xp.x + dc.y * inv_a);
+  // Unfold, combine and entangle: thread -> (k <= L / 2, plane), which reads
+  // the waist at orders k and L - k and forms Z[k] and Z[L - k] of every
+  // output row: Z[k] = A + conj(C) + i conj(w_k) (A - conj(C)) with A = X[k],
+  // C = X[L - k], and Z[L - k] from the same three (w_{L-k} = -conj(w_k)).
+  {
+    const int q = threadIdx.x & ((1 << lc) - 1), kstep = blockDim.x >> lc;
+    const int64_t plane = min(p0 + q, a.planes - 1);  // past the end: transformed, not stored
+    const int64_t Rc = a.planes * FW;
+    const V2<T>* P2 = reinterpret_cast<const V2<T>*>(wP) + (int64_t)h * Rc + plane * FW;
+    const V2<T>* D2 = reinterpret_cast<const V2<T>*>(wD) + (int64_t)h * Rc + plane * FW;
+    const int64_t dsd = (int64_t)a.H * Rc;  // S row -> D row of the same order
+    const T inv_a = T(1.0 / a.radius);
+    T ie[2] = {T(0), T(0)};  // 1 / (a cos phi) of the two sides
+    if constexpr (NF != 1) {
+      ie[0] = T(1) / (T(a.radius) * T(coslat[h]));
+      ie[1] = T(1) / (T(a.radius) * T(coslat[a.nlat - 1 - h]));
+    }
+    // x[o][sd]: order m of output field o on side sd
+    auto order_values = [&](int m, V2<T>(&x)[NO][2]) {
+      V2<T> S[NF], D[NF];
+      const int64_t at = 2 * m * dsd;
+#pragma unroll
+      for (int k = 0; k < NF; ++k) {
+        const V2<T>* w = (NF == 1 || k < NF / 2 ? P2 : D2) + at + (NF == 4 ? (k & 1) : 0);
+        S[k] = w[0];
+        D[k] = w[dsd];
       }
-      bufB[((gp * NO + 0) * rpp + side) * Lp + m] = o0;
-      if (NO == 2) bufB[((gp * NO + 1) * rpp + side) * Lp + m] = o1;
+      const T mf = T(m);
+#pragma unroll
+      for (int sd = 0; sd < 2; ++sd) {
+        V2<T> v[NF];
+#pragma unroll
+        for (int k = 0; k < NF; ++k) v[k] = sd ? csub<T>(S[k], D[k]) : cadd<T>(S[k], D[k]);
+        if constexpr (NF == 1) {
+          x[0][sd] = a.zonal ? mk2<T>(-mf * v[0].y, mf * v[0].x) : v[0];
+        } else if constexpr (NF == 2) {
+          // east: i m P / (a cos phi); north: dP / a
+          x[0][sd] = mk2<T>(-mf * v[0].y * ie[sd], mf * v[0].x * ie[sd]);
+          x[1][sd] = mk2<T>(v[1].x * inv_a, v[1].y * inv_a);
+        } else {
+          // v = {P psi, P chi, dP psi, dP chi}: u = -dpsi/a + i m chi/(a cos),
+          // v = i m psi/(a cos) + dchi/a
+          const T im = mf * ie[sd];
+          x[0][sd] = mk2<T>(-v[2].x * inv_a - im * v[1].y, -v[2].y * inv_a + im * v[1].x);
+          x[1][sd] = mk2<T>(-im * v[0].y + v[3].x * inv_a, im * v[0].x + v[3].y * inv_a);
+        }
+      }
+    };
+    for (int k = threadIdx.x >> lc; 2 * k <= L; k += kstep) {
+      const int kc = L - k;
+      V2<T> A[NO][2], C[NO][2];
+#pragma unroll
+      for (int o = 0; o < NO; ++o)
+        A[o][0] = A[o][1] = C[o][0] = C[o][1] = mk2<T>(T(0), T(0));
+      if (k <= a.T) order_values(k, A);
+      if (k > 0 && kc <= a.T) order_values(kc, C);
+      if (k == 0) {  // irfft reads only the real part of order 0
+#pragma unroll
+        for (int o = 0; o < NO; ++o) A[o][0].y = A[o][1].y = T(0);
+      }
+      const V2<T> w = cconj<T>(tw_n[k]);  // exp(+2 pi i k / N)
+#pragma unroll
+      for (int o = 0; o < NO; ++o)
+#pragma unroll
+        for (int sd = 0; sd < 2; ++sd) {
+          V2<T>* row = bufA + (((o * 2 + sd) << lc) + q);
+          const V2<T> p = A[o][sd], c = C[o][sd];
+          const V2<T> sm = mk2<T>(p.x + c.x, p.y - c.y), df = mk2<T>(p.x - c.x, p.y + c.y);
+          const V2<T> t = cmul<T>(w, df);
+          row[k * rs] = mk2<T>(sm.x - t.y, sm.y + t.x);
+          if (k > 0 && kc != k) row[kc * rs] = mk2<T>(sm.x + t.y, t.x - sm.y);
+        }
     }
   }
   __syncthreads();
-  // Stage 2: entangle into Z[k], k < L, in bufA.
-  for (int t = threadIdx.x; t < rows * L; t += blockDim.x) {
-    int row = t / L, k = t - row * L;
-    int gp = row / (NO * rpp);
-    V2<T> z = mk2<T>(T(0), T(0));
-    if (p0 + gp < a.planes) {
-      const V2<T>* xr = bufB + row * Lp;
-      V2<T> xk = k <= a.T ? xr[k] : mk2<T>(T(0), T(0));
-      int kc = L - k;
-      V2<T> xc = (k > 0 && kc <= a.T) ? cconj<T>(xr[kc]) : mk2<T>(T(0), T(0));
-      if (k == 0) xk.y = T(0);  // irfft reads only the real part of bin 0
-      V2<T> s = cadd<T>(xk, xc), d = csub<T>(xk, xc);
-      V2<T> w = cconj<T>(tw_n[k]);  // exp(+2 pi i k / N)
-      V2<T> wd = cmul<T>(w, d);
-      z = mk2<T>(s.x - wd.y, s.y + wd.x);  // s + i w d
-    }
-    bufA[row * Lp + k] = z;
-  }
-  __syncthreads();
-  V2<T>* zr = run_passes<T>(bufA, bufB, a.f, rows, tw_l, w16, true);
+  const V2<T>* Z = run_passes<T, true>(bufA, bufB, a.f, lr, tw);
 
-  // Stage 3: write rows with per-row scaling.
-  for (int t = threadIdx.x; t < rows * L; t += blockDim.x) {
-    int row = t / L, k = t - row * L;
-    int side = row % rpp, o = (row / rpp) % NO, gp = row / (NO * rpp);
-    int64_t plane = p0 + gp;
-    if (plane >= a.planes) continue;
-    int j = side ? (a.nlat - 1 - h) : h;
-    V2<T> v = zr[row * Lp + k];
-    if (a.mode == kUnfoldGradient) {
-      if (o == 0) {
-        T den = T(a.radius) * T(coslat[j]);
-        v.x = v.x / den;
-        v.y = v.y / den;
-      } else {
-        v.x = v.x / T(a.radius);
-        v.y = v.y / T(a.radius);
-      }
-    }
-    T* dst = (o ? out1 : out0) + (plane * a.nlat + j) * (int64_t)a.nlon;
-    reinterpret_cast<V2<T>*>(dst)[k] = v;
-  }
+  // Store: four neighbouring k of a row per quad of lanes, as the forward's loads.
+  const int row = (threadIdx.x >> 2) & ((1 << lr) - 1);
+  const int64_t plane = p0 + (row & ((1 << lc) - 1));
+  const int side = (row >> lc) & 1, o = row >> (lc + 1);
+  if (plane >= a.planes || (eq && side)) return;
+  V2<T>* dst = reinterpret_cast<V2<T>*>(
+      (o ? out1 : out0) + (plane * a.nlat + (side ? a.nlat - 1 - h : h)) * (int64_t)a.nlon);
+  const int kstep = blockDim.x >> lr;
+#pragma unroll 4
+  for (int k = ((threadIdx.x >> (2 + lr)) << 2) + (threadIdx.x & 3); k < L; k += kstep)
+    dst[k] = Z[k * rs + row];
 }
 
 __global__ void twiddle_kernel(int L, int N, double2* tl, double2* tn) {
@@ -462,21 +579,75 @@ __global__ void twiddle_cast_kernel(const double2* in, float2* out, int n) {
   if (k < n) out[k] = make_float2((float)in[k].x, (float)in[k].y);
 }
 
-FftShape make_shape(const sht_plan* p) {
-  FftShape f{};
-  f.L = p->L;
-  f.Lp = p->L;
-  f.nrad = (int)p->radices.size();
-  for (int i = 0; i < f.nrad; ++i) f.rad[i] = p->radices[i];
-  return f;
+// The radix sequence of length L: the fewest passes of radices 2 .. 16 (13
+// and below the prime ones), and among those the smallest sum of radices
+// (the widest passes); other primes by the direct pass.
+std::vector<int> radix_plan(int L) {
+  std::vector<int> rest;
+  int r = L;
+  for (int q = 2; r > 1 && q <= 13; ++q)
+    while (r % q == 0) r /= q;
+  const int smooth = L / r;
+  for (int q = 17; r > 1; q += 2)
+    while (r % q == 0) { rest.push_back(q); r /= q; }
+  constexpr int kRadix[] = {16, 15, 13, 12, 11, 10, 9, 8, 7, 6, 5, 4, 3, 2};
+  std::vector<int> best, now;
+  auto sum = [](const std::vector<int>& v) { int s = 0; for (int x : v) s += x; return s; };
+  auto walk = [&](auto&& self, int n, int most) -> void {
+    if (n == 1) {
+      if (best.empty() || now.size() < best.size() || (now.size() == best.size() && sum(now) < sum(best))) best = now;
+      return;
+    }
+    if (!best.empty() && now.size() + 1 > best.size()) return;
+    for (int q : kRadix)
+      if (q <= most && n % q == 0) {
+        now.push_back(q);
+        self(self, n / q, q);
+        now.pop_back();
+      }
+  };
+  walk(walk, smooth, 16);
+  best.insert(best.end(), rest.begin(), rest.end());
+  return best;
 }
 
+// Columns of a CTA: as many as leave room for three CTAs per SM (two in FP64;
+// two buffers of 2 no columns rows each), at most 8 (in FP32 64-byte pieces of
+// every waist row) and no more than the call has; fewer when the launch would
+// leave SMs without a CTA.
 template <typename T>
-int rows_budget() { return sizeof(T) == 8 ? 4 : 8; }
-
-template <typename T>
-size_t smem_bytes(const sht_plan* p, int rows) {
-  return (size_t)2 * rows * p->L * sizeof(V2<T>);
+FftShape make_shape(const sht_plan* p, int64_t cols, int no, size_t* smem, int* threads) {
+  constexpr size_t kTarget = (sizeof(T) == 4 ? 74 : 100) * 1024, kMost = 227 * 1024;
+  FftShape f{};
+  f.L = p->L;
+  f.npass = (int)p->radices.size();
+  int Ns = 1;
+  for (int i = 0; i < f.npass; ++i) {
+    const int R = p->radices[i];
+    f.pass[i] = {R, Ns, p->L / R, p->L / (Ns * R),
+                 Ns > 1 ? (unsigned)(((uint64_t)1 << 32) / Ns + 1) : 0u};
+    Ns *= R;
+  }
+  // FP32 rows of 16 (FP64: 8) and more fill a whole bank sweep per k: the
+  // quad's four k of the load and store phases then fall on the same banks
+  // unless the row stride is padded.
+  constexpr int kSlots = sizeof(T) == 4 ? 16 : 8;
+  auto stride = [&](int lc) {
+    const int rows = (2 * no) << lc;
+    return rows >= kSlots ? rows + kSlots / 4 : rows;
+  };
+  auto bytes = [&](int lc) { return (size_t)2 * stride(lc) * p->L * sizeof(V2<T>); };
+  const size_t table = (size_t)p->L * sizeof(V2<T>);
+  int lc = 0;
+  while (lc < 3 && ((int64_t)1 << lc) < cols && bytes(lc + 1) + table <= kTarget) ++lc;
+  while (lc > 0 && p->H * div_up(cols, (int64_t)1 << lc) < 2 * 148) --lc;
+  f.lc = lc;
+  f.rs = stride(lc);
+  f.tw_shared = bytes(lc) + table <= kMost ? 1 : 0;
+  *smem = bytes(lc) + (f.tw_shared ? table : 0);
+  const int work = ((2 * no) << lc) * p->L;  // elements; about eight per thread and pass
+  *threads = std::max(work >= 1536 ? 256 : (work >= 768 ? 128 : 64), 4 * ((2 * no) << lc));
+  return f;
 }
 
 template <typename K>
@@ -488,20 +659,9 @@ void allow_smem(K kernel, size_t bytes) {
 }  // namespace
 
 void build_fft(sht_plan* p, cudaStream_t s) {
-  // Radix plan: 16s, 8, 4, 2, then 3s, 5s, then any other primes.
-  int L = p->L;
-  std::vector<int> rad;
-  int r = L;
-  while (r % 16 == 0) { rad.push_back(16); r /= 16; }
-  if (r % 8 == 0) { rad.push_back(8); r /= 8; }
-  if (r % 4 == 0) { rad.push_back(4); r /= 4; }
-  if (r % 2 == 0) { rad.push_back(2); r /= 2; }
-  while (r % 3 == 0) { rad.push_back(3); r /= 3; }
-  while (r % 5 == 0) { rad.push_back(5); r /= 5; }
-  for (int q = 7; r > 1; q += 2)
-    while (r % q == 0) { rad.push_back(q); r /= q; }
-  SHT_REQUIRE(rad.size() <= 24, "nlon has too many prime factors");
-  p->radices = rad;
+  const int L = p->L;
+  p->radices = radix_plan(L);
+  SHT_REQUIRE(p->radices.size() <= kMaxPass, "nlon has too many prime factors");
   p->fast_fft = fast_fft_supported(p) && !p->force_generic_fft;
   if (p->fast_fft) fast_fft_init_constants(s);
 
@@ -538,23 +698,30 @@ void launch_forward_fold(const sht_plan* p, const T* g0, const T* g1, int64_t pl
   }
   // g0 (and g1 for a stacked (u, v) pair) are (planes, nlat, nlon) grids.
   const int fields = g1 ? 2 : 1;
-  FoldArgs a{};
-  a.f = make_shape(p);
-  a.nlat = p->nlat;
-  a.nlon = p->nlon;
-  a.T = p->T;
-  a.H = p->H;
-  a.nlat_odd = p->nlat_odd;
-  a.F = fields;
-  a.G = std::max(1, rows_budget<T>() / (2 * fields));
-  a.planes = planes;
-  int rows = a.G * a.F * 2;
-  size_t sm = smem_bytes<T>(p, rows);
+  size_t sm = 0;
+  int threads = 0;
+  const FftShape f = make_shape<T>(p, planes * fields, 1, &sm, &threads);
+  const FoldArgs a{f, p->nlat, p->nlon, p->T, p->H, p->nlat_odd ? 1 : 0, fields, planes * fields};
   allow_smem(forward_fold_kernel<T>, sm);
-  dim3 grid_dim((unsigned)p->H, (unsigned)div_up(planes, a.G));
-  SHT_REQUIRE(rowmax == nullptr || 256 % (a.G * a.F) == 0, "row maxima need 256 % (G F) == 0");
-  forward_fold_kernel<T><<<grid_dim, 256, sm, s>>>(a, g0, g1 ? g1 : g0, (const V2<T>*)p->tw_l,
+  const dim3 grid((unsigned)div_up(a.cols, (int64_t)1 << f.lc), (unsigned)p->H);
+  forward_fold_kernel<T><<<grid, threads, sm, s>>>(a, g0, g1 ? g1 : g0, (const V2<T>*)p->tw_l,
                                                    (const V2<T>*)p->tw_n, wfold, rowmax);
+  SHT_CUDA_OR_THROW(cudaGetLastError());
+}
+
+template <typename T, int NF>
+void launch_unfold(const sht_plan* p, int mode, const T* wP, const T* wD, int64_t planes, T* out0,
+                   T* out1, cudaStream_t s) {
+  size_t sm = 0;
+  int threads = 0;
+  const FftShape f = make_shape<T>(p, planes, NF == 1 ? 1 : 2, &sm, &threads);
+  const UnfoldArgs a{f, p->nlat, p->nlon, p->T, p->H, p->nlat_odd ? 1 : 0,
+                     mode == kUnfoldZonal ? 1 : 0, planes, p->radius};
+  allow_smem(inverse_unfold_kernel<T, NF>, sm);
+  const dim3 grid((unsigned)div_up(planes, (int64_t)1 << f.lc), (unsigned)p->H);
+  inverse_unfold_kernel<T, NF><<<grid, threads, sm, s>>>(
+      a, wP, wD ? wD : wP, p->d_coslat, (const V2<T>*)p->tw_l, (const V2<T>*)p->tw_n, out0,
+      out1 ? out1 : out0);
   SHT_CUDA_OR_THROW(cudaGetLastError());
 }
 
@@ -567,26 +734,12 @@ void launch_inverse_unfold(const sht_plan* p, int mode, const T* wP, const T* wD
       return;
     }
   }
-  UnfoldArgs a{};
-  a.f = make_shape(p);
-  a.nlat = p->nlat;
-  a.nlon = p->nlon;
-  a.T = p->T;
-  a.H = p->H;
-  a.nlat_odd = p->nlat_odd;
-  a.mode = mode;
-  a.planes = planes;
-  a.radius = p->radius;
-  int NO = (mode == kUnfoldGradient || mode == kUnfoldWind) ? 2 : 1;
-  a.G = std::max(1, rows_budget<T>() / (2 * NO));
-  int rows = a.G * NO * 2;
-  size_t sm = smem_bytes<T>(p, rows);
-  allow_smem(inverse_unfold_kernel<T>, sm);
-  dim3 grid_dim((unsigned)p->H, (unsigned)div_up(planes, a.G));
-  inverse_unfold_kernel<T><<<grid_dim, 256, sm, s>>>(a, wP, wD, p->d_coslat,
-                                                     (const V2<T>*)p->tw_l,
-                                                     (const V2<T>*)p->tw_n, out0, out1);
-  SHT_CUDA_OR_THROW(cudaGetLastError());
+  if (mode == kUnfoldWind)
+    launch_unfold<T, 4>(p, mode, wP, wD, planes, out0, out1, s);
+  else if (mode == kUnfoldGradient)
+    launch_unfold<T, 2>(p, mode, wP, wD, planes, out0, out1, s);
+  else
+    launch_unfold<T, 1>(p, mode, wP, wD, planes, out0, out1, s);
 }
 
 template void launch_forward_fold<float>(const sht_plan*, const float*, const float*, int64_t,
