@@ -162,9 +162,23 @@ void contract(sht_plan* p, int kind, const T* data, T* out, int64_t R, cudaStrea
   launch_gemm_simt<T>(p, dir, flip, static_cast<const T*>(table_ptr(p, kind)), data, out, R, s);
 }
 
+// Two contractions of one direction in one SIMT launch.
+template <typename T>
+void simt_pair(sht_plan* p, int kind0, const T* data0, T* out0, int kind1, const T* data1, T* out1,
+               int64_t R, cudaStream_t s) {
+  const int dir = table_dir(kind0);
+  KernelScope scope(p, dir == 0 ? SHT_KIND_LEGENDRE_SYNTHESIS : SHT_KIND_LEGENDRE_ANALYSIS, s);
+  const int flip[2] = {table_flip(kind0), table_flip(kind1)};
+  const T* table[2] = {static_cast<const T*>(table_ptr(p, kind0)),
+                       static_cast<const T*>(table_ptr(p, kind1))};
+  const T* data[2] = {data0, data1};
+  T* out[2] = {out0, out1};
+  launch_gemm_simt_groups<T>(p, dir, 2, flip, table, data, out, R, s);
+}
+
 // Two contractions of the same data (P and dP/dphi tables of a gradient or
 // wind synthesis; rotational and shear tables of a vordiv analysis): one
-// tensor-core launch over the merged tiles on the split path.
+// launch over both tables.
 template <typename T>
 void contract2(sht_plan* p, int kind0, T* out0, int kind1, T* out1, const T* data, int64_t R,
                cudaStream_t s) {
@@ -179,8 +193,7 @@ void contract2(sht_plan* p, int kind0, T* out0, int kind1, T* out1, const T* dat
       return;
     }
   }
-  contract<T>(p, kind0, data, out0, R, s);
-  contract<T>(p, kind1, data, out1, R, s);
+  simt_pair<T>(p, kind0, data, out0, kind1, data, out1, R, s);
 }
 
 // Two contractions of different operands, each with its own row maxima (the
@@ -200,8 +213,7 @@ void contract_pair(sht_plan* p, int kind0, const T* data0, const float* rm0, T* 
       return;
     }
   }
-  contract<T>(p, kind0, data0, out0, R, s);
-  contract<T>(p, kind1, data1, out1, R, s);
+  simt_pair<T>(p, kind0, data0, out0, kind1, data1, out1, R, s);
 }
 
 template <typename T>

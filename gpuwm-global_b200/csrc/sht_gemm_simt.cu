@@ -3,7 +3,9 @@
 // Tab[k][x] * D[k][r], with the plane/component rows r innermost in both the
 // data and the output.  One launch covers the whole triangle: the work list
 // holds (block, x-tile) items sorted by descending cost, so the large low-m
-// blocks start first and the ragged high-m tail fills in behind them.  This
+// blocks start first and the ragged high-m tail fills in behind them; the row
+// blocks (and the tables of a two-table call) of one item are neighbours in
+// the grid, so its table and data tiles come from L2 after the first.  This
 // replaces the reference's per-band dense strided-batched GEMMs
 // (transform.py:1178-1274), which multiply the zeros above the triangle too.
 #include <algorithm>
@@ -14,161 +16,212 @@
 namespace sht {
 namespace {
 
-// Tile shapes (x columns of the table x r data rows per CTA).  FP32 has two,
-// chosen at run time (SHT_TUNE_SIMT_TILE): 128 x 128, and 64 x 128, whose
-// narrower column tiles waste less on the ragged analysis blocks (X = the
-// degrees of one order and parity) at the price of more table loads.
-template <typename T, bool NARROW> struct SimtCfg;
-template <> struct SimtCfg<float, false> {
-  static constexpr int BX = 128, BR = 128, BK = 8, TMX = 8, TMR = 8, VW = 4;
-  using V = float4;
+// Tiles in units of V, the elements of 16 bytes (4 floats, 2 doubles).  A
+// thread holds 2 V columns of the table x GN V data rows, a warp 4 x 8 such
+// threads (8 V columns x 8 GN V rows), a CTA WX warps side by side.  The 16-byte
+// pieces a thread owns are interleaved across its warp (piece g of lane l at
+// (g * lanes + l) * V), so every shared load of a warp is one contiguous
+// stretch.  Bound by the FMA pipe (62 / 70 % busy at T511, analysis /
+// synthesis) and the shared loads that feed it (65 %): FP32 issues packed pairs
+// (fma.rn.f32x2), which halves the issue slots of the multiply-adds, and 8 x 8
+// outputs per thread leave 16 warps on an SM; 8 x 16 with 8 warps measured the
+// same at T511 and 10 to 25 % slower at T255 and T126, where the chain per tile
+// is short.  Analysis + synthesis against one element per instruction in
+// 128 x 128 tiles of 256 threads loaded through registers: T511 x 200 planes
+// 2716 -> 1921 us (42 TF/s), T255 x 161 planes 444 -> 264 us, T126 x 200 planes
+// 103 -> 70 us.  Each output element is one chain of fused multiply-adds over
+// ascending k from zero, whatever the tile, so every tile shape returns the
+// same bits.
+template <typename T> struct SimtCfg {
+  static constexpr int V = 16 / (int)sizeof(T);
+  static constexpr int BK = 16;  // contraction rows per stage
+  static constexpr int S = 3;    // stages
+  static constexpr int G = 2;    // row pieces per thread of a whole row block
 };
-template <> struct SimtCfg<float, true> {
-  static constexpr int BX = 64, BR = 128, BK = 8, TMX = 4, TMR = 8, VW = 4;
-  using V = float4;
+// Columns of a CTA (WX = 2 or 4 warps) and rows of a row block (GN pieces).
+template <typename T> constexpr int tile_x(int wx) { return 8 * SimtCfg<T>::V * wx; }
+template <typename T> constexpr int tile_r(int gn) { return 8 * SimtCfg<T>::V * gn; }
+
+// One table of a launch; the groups of a launch share the item list and R.
+template <typename T> struct SimtGroup {
+  const ShtGemmDesc* descs;
+  const T* table;
+  const T* data;
+  T* out;
 };
-template <> struct SimtCfg<double, false> {
-  static constexpr int BX = 64, BR = 64, BK = 8, TMX = 4, TMR = 4, VW = 2;
-  using V = double2;
+template <typename T> struct SimtArgs {
+  SimtGroup<T> g[2];
+  const ShtGemmItem* items;
+  int ng;      // groups (1 or 2)
+  int nrb;     // row blocks of tile_r(G)
+  bool half;   // the last one holds at most tile_r(1) rows
+  int64_t R;
 };
 
-template <typename T, bool NARROW>
-__global__ void __launch_bounds__(256, 2) gemm_simt_kernel(const ShtGemmDesc* __restrict__ descs,
-                                                        const ShtGemmItem* __restrict__ items,
-                                                        const T* __restrict__ table,
-                                                        const T* __restrict__ data,
-                                                        T* __restrict__ out, int64_t R) {
-  using C = SimtCfg<T, NARROW>;
-  constexpr int BX = C::BX, BR = C::BR, BK = C::BK, TMX = C::TMX, TMR = C::TMR, VW = C::VW;
-  constexpr int NTX = BX / TMX, NTR = BR / TMR;  // 16 x 16 threads
-  constexpr int GX = TMX / VW, GR = TMR / VW;     // vector groups per thread
-  static_assert(NTX * NTR == 256, "256 threads");
+template <int BYTES>
+__device__ __forceinline__ void cp_async(uint32_t dst, const void* src, bool live) {
+  const uint32_t n = live ? BYTES : 0;  // the rest of the piece is zero-filled
+  if constexpr (BYTES == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+}
 
-  const ShtGemmItem it = items[blockIdx.x];
-  const ShtGemmDesc d = descs[it.problem];
-  const int x0 = it.x0;
-  const int64_t r0 = (int64_t)blockIdx.y * BR;
-  const T* __restrict__ Tb = table + d.t_off;
-  const T* __restrict__ Db = data + d.d_row * R;
-  T* __restrict__ Cb = out + d.c_row * R;
+// One CTA tile.  DB: bytes of a data-row copy, 16 where every data row starts
+// on a 16-byte boundary and 8 otherwise (FP32 with an odd plane count).
+template <typename T, int WX, int GN, int DB>
+__device__ __forceinline__ void simt_tile(const SimtGroup<T>& G, const ShtGemmDesc& d, int x0,
+                                          int64_t r0, int64_t R, T* smem) {
+  constexpr int V = SimtCfg<T>::V, BK = SimtCfg<T>::BK, S = SimtCfg<T>::S;
+  constexpr int BX = tile_x<T>(WX), BR = tile_r<T>(GN), NT = 32 * WX;
+  const T* __restrict__ Tb = G.table + d.t_off;
+  const T* __restrict__ Db = G.data + d.d_row * R;
+  T* sA = smem;                // [S][BK][BX]
+  T* sB = smem + S * BK * BX;  // [S][BK][BR]
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int lx = lane >> 3, lr = lane & 7;
+  // A warp whose columns lie wholly past the problem (the ragged x tail of an
+  // analysis block) skips its arithmetic.
+  const bool busy = x0 + warp * 8 * V < d.X;
 
-  __shared__ __align__(16) T As[2][BK][BX];
-  __shared__ __align__(16) T Bs[2][BK][BR];
-
-  const int tid = threadIdx.x;
-  // Thread -> a TMX x TMR block of contiguous x and r.  Warp w covers the
-  // rows wr * BR/4 .. +BR/4 (wr = w % 4) and the columns wx * BX/2 .. +BX/2
-  // (wx = w / 4); lane -> (lr = lane % 4, lx = lane / 4) within it.  A warp
-  // whose rows or columns lie wholly past the problem's extent (the ragged x
-  // tail of an analysis block, the last partial row block) skips its FFMAs:
-  // the issue slots go to the other warps and CTAs of the SM.
-  const int warp = tid >> 5, lane = tid & 31;
-  const int r_base = (warp & 3) * (BR / 4) + (lane & 3) * TMR;
-  const int x_base = (warp >> 2) * (BX / 2) + (lane >> 2) * TMX;
-  static_assert(4 * TMR * 4 == BR && 8 * TMX * 2 == BX, "warp tiling covers the block");
-  const bool busy = x0 + (warp >> 2) * (BX / 2) < d.X && r0 + (warp & 3) * (BR / 4) < R;
-
-  // Global-load mapping: each tile is BK x B{X,R} = 8 x 128 (or 8 x 64);
-  // thread loads LPT consecutive elements of one k-row.
-  constexpr int LPT_A = BK * BX / 256, LPT_B = BK * BR / 256;
-  const int la_k = tid / (BX / LPT_A), la_x = (tid % (BX / LPT_A)) * LPT_A;
-  const int lb_k = tid / (BR / LPT_B), lb_r = (tid % (BR / LPT_B)) * LPT_B;
-
-  T ra[LPT_A], rb[LPT_B];
-  auto load_global = [&](int k0) {
-    int k = k0 + la_k;
+  auto load_stage = [&](int kt) {
+    const int buf = kt % S, k0 = kt * BK;
+    constexpr int AP = BX / V;  // pieces per table row
 #pragma unroll
-    for (int i = 0; i < LPT_A; ++i) {
-      int x = x0 + la_x + i;
-      ra[i] = (k < d.K && x < d.X) ? Tb[(int64_t)k * d.ldt + x] : T(0);
+    for (int e = tid; e < BK * AP; e += NT) {
+      const int k = e / AP, x = (e % AP) * V;
+      const bool live = k0 + k < d.K && x0 + x < d.ldt;
+      cp_async<16>((uint32_t)__cvta_generic_to_shared(sA + (buf * BK + k) * BX + x),
+                   live ? Tb + (int64_t)(k0 + k) * d.ldt + x0 + x : Tb, live);
     }
-    k = k0 + lb_k;
+    constexpr int DV = DB / (int)sizeof(T), BP = BR / DV;
 #pragma unroll
-    for (int i = 0; i < LPT_B; ++i) {
-      int64_t r = r0 + lb_r + i;
-      rb[i] = (k < d.K && r < R) ? Db[(int64_t)k * R + r] : T(0);
+    for (int e = tid; e < BK * BP; e += NT) {
+      const int k = e / BP, r = (e % BP) * DV;
+      const bool live = k0 + k < d.K && r0 + r < R;
+      cp_async<DB>((uint32_t)__cvta_generic_to_shared(sB + (buf * BK + k) * BR + r),
+                   live ? Db + (int64_t)(k0 + k) * R + r0 + r : Db, live);
     }
   };
-  auto store_shared = [&](int buf) {
-#pragma unroll
-    for (int i = 0; i < LPT_A; ++i) As[buf][la_k][la_x + i] = ra[i];
-#pragma unroll
-    for (int i = 0; i < LPT_B; ++i) Bs[buf][lb_k][lb_r + i] = rb[i];
-  };
 
-  T acc[TMX][TMR];
+  // FP32: acc[i][j] holds the pair of rows (2j, 2j + 1) of column i.
+  using Acc = std::conditional_t<sizeof(T) == 4, float2, double>;
+  constexpr int NJ = sizeof(T) == 4 ? GN * V / 2 : GN * V;
+  Acc acc[2 * V][NJ];
 #pragma unroll
-  for (int i = 0; i < TMX; ++i)
+  for (int i = 0; i < 2 * V; ++i)
 #pragma unroll
-    for (int j = 0; j < TMR; ++j) acc[i][j] = T(0);
+    for (int j = 0; j < NJ; ++j) {
+      if constexpr (sizeof(T) == 4) acc[i][j] = make_float2(0.f, 0.f);
+      else acc[i][j] = 0.0;
+    }
 
   const int nk = (d.K + BK - 1) / BK;
-  load_global(0);
-  store_shared(0);
-  __syncthreads();
-  for (int kt = 0; kt < nk; ++kt) {
-    const int buf = kt & 1;
-    if (kt + 1 < nk) load_global((kt + 1) * BK);
-    if (busy) {
 #pragma unroll
-      for (int kk = 0; kk < BK; ++kk) {
-        T a[TMX], b[TMR];
-#pragma unroll
-        for (int g = 0; g < GX; ++g) {
-          typename C::V v = *reinterpret_cast<const typename C::V*>(&As[buf][kk][x_base + g * VW]);
-          const T* pv = reinterpret_cast<const T*>(&v);
-#pragma unroll
-          for (int u = 0; u < VW; ++u) a[g * VW + u] = pv[u];
-        }
-#pragma unroll
-        for (int g = 0; g < GR; ++g) {
-          typename C::V v = *reinterpret_cast<const typename C::V*>(&Bs[buf][kk][r_base + g * VW]);
-          const T* pv = reinterpret_cast<const T*>(&v);
-#pragma unroll
-          for (int u = 0; u < VW; ++u) b[g * VW + u] = pv[u];
-        }
-#pragma unroll
-        for (int i = 0; i < TMX; ++i)
-#pragma unroll
-          for (int j = 0; j < TMR; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
-      }
-    }
-    if (kt + 1 < nk) {
-      store_shared(buf ^ 1);
-    }
-    __syncthreads();
+  for (int kt = 0; kt < S - 1; ++kt) {
+    if (kt < nk) load_stage(kt);
+    asm volatile("cp.async.commit_group;" ::: "memory");
   }
-
-  // Epilogue: C[x][r], r innermost.
+  for (int kt = 0; kt < nk; ++kt) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(S - 2) : "memory");
+    __syncthreads();  // stage kt has landed; every warp is done with stage kt - 1
+    if (kt + S - 1 < nk) load_stage(kt + S - 1);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    if (!busy) continue;
+    const T* pa = sA + (kt % S) * BK * BX + warp * 8 * V + lx * V;
+    const T* pb = sB + (kt % S) * BK * BR + lr * V;
+#pragma unroll 8
+    for (int kk = 0; kk < BK; ++kk) {
+      if constexpr (sizeof(T) == 4) {
+        float a[8];
+        float2 b[NJ];
 #pragma unroll
-  for (int i = 0; i < TMX; ++i) {
-      int x = x0 + x_base + i;
-      if (x >= d.X) continue;
-      T* crow = Cb + (int64_t)x * R;
-#pragma unroll
-      for (int gr = 0; gr < GR; ++gr) {
-        int64_t r = r0 + r_base + gr * VW;
-        const T* av = &acc[i][gr * VW];
-        if (r + VW <= R && (R % VW) == 0) {
-          typename C::V v;
-          T* pv = reinterpret_cast<T*>(&v);
-#pragma unroll
-          for (int w = 0; w < VW; ++w) pv[w] = av[w];
-          *reinterpret_cast<typename C::V*>(crow + r) = v;
-        } else {
-#pragma unroll
-          for (int w = 0; w < VW; ++w)
-            if (r + w < R) crow[r + w] = av[w];
+        for (int g = 0; g < 2; ++g) {
+          const float4 v = *reinterpret_cast<const float4*>(pa + kk * BX + g * 4 * V);
+          a[4 * g] = v.x; a[4 * g + 1] = v.y; a[4 * g + 2] = v.z; a[4 * g + 3] = v.w;
         }
+#pragma unroll
+        for (int g = 0; g < GN; ++g) {
+          const float4 v = *reinterpret_cast<const float4*>(pb + kk * BR + g * 8 * V);
+          b[2 * g] = make_float2(v.x, v.y);
+          b[2 * g + 1] = make_float2(v.z, v.w);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+          for (int j = 0; j < NJ; ++j) acc[i][j] = __ffma2_rn(make_float2(a[i], a[i]), b[j], acc[i][j]);
+      } else {
+        double a[4], b[NJ];
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+          const double2 v = *reinterpret_cast<const double2*>(pa + kk * BX + g * 4 * V);
+          a[2 * g] = v.x; a[2 * g + 1] = v.y;
+        }
+#pragma unroll
+        for (int g = 0; g < GN; ++g) {
+          const double2 v = *reinterpret_cast<const double2*>(pb + kk * BR + g * 8 * V);
+          b[2 * g] = v.x; b[2 * g + 1] = v.y;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < NJ; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
       }
     }
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+
+  // Epilogue: C[x][r], r innermost, in pieces of 16 (or 8) bytes.
+  if (!busy) return;
+  T* __restrict__ Cb = G.out + d.c_row * R;
+#pragma unroll
+  for (int i = 0; i < 2 * V; ++i) {
+    const int x = x0 + warp * 8 * V + (i / V) * 4 * V + lx * V + i % V;
+    if (x >= d.X) continue;
+    T* crow = Cb + (int64_t)x * R;
+#pragma unroll
+    for (int g = 0; g < GN; ++g) {
+      const int64_t r = r0 + g * 8 * V + lr * V;
+      if constexpr (sizeof(T) == 4) {
+        const float2 u = acc[i][2 * g], w = acc[i][2 * g + 1];
+        if constexpr (DB == 16) {
+          if (r < R) *reinterpret_cast<float4*>(crow + r) = make_float4(u.x, u.y, w.x, w.y);
+        } else {
+          if (r < R) *reinterpret_cast<float2*>(crow + r) = u;
+          if (r + 2 < R) *reinterpret_cast<float2*>(crow + r + 2) = w;
+        }
+      } else {
+        if (r < R) *reinterpret_cast<double2*>(crow + r) = make_double2(acc[i][2 * g], acc[i][2 * g + 1]);
+      }
+    }
+  }
+}
+
+// Block -> (item, row block, group), groups fastest.  A last row block at most
+// half full runs with half the rows per thread.
+template <typename T, int WX, int DB>
+__global__ void __launch_bounds__(32 * WX, 16 / WX) gemm_simt_kernel(const __grid_constant__ SimtArgs<T> a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  T* smem = reinterpret_cast<T*>(smem_raw);
+  constexpr int G = SimtCfg<T>::G;
+  unsigned b = blockIdx.x;
+  const SimtGroup<T>& grp = a.g[a.ng == 2 ? (b & 1) : 0];
+  if (a.ng == 2) b >>= 1;
+  const int rb = (int)(b % (unsigned)a.nrb);
+  const ShtGemmItem it = a.items[b / (unsigned)a.nrb];
+  const ShtGemmDesc d = grp.descs[it.problem];
+  const int64_t r0 = (int64_t)rb * tile_r<T>(G);
+  if (a.half && rb == a.nrb - 1)
+    simt_tile<T, WX, 1, DB>(grp, d, it.x0, r0, a.R, smem);
+  else
+    simt_tile<T, WX, G, DB>(grp, d, it.x0, r0, a.R, smem);
 }
 
 }  // namespace
 
 void build_gemm_items(sht_plan* p) {
   const int T = p->T;
-  const int bx = p->prec == SHT_PREC_F64 ? SimtCfg<double, false>::BX : SimtCfg<float, false>::BX;
+  const int bx = p->prec == SHT_PREC_F64 ? tile_x<double>(4) : tile_x<float>(4);
   p->gemm_bx = bx;
   // Every (m, q) is a problem, including the empty parity-1 block of m = T:
   // its synthesis item has K = 0 and writes the zeros the inverse FFT reads
@@ -228,7 +281,7 @@ void build_gemm_items(sht_plan* p) {
   for (int dir = 0; dir < 2; ++dir) {
     item_list(dir, bx, &p->d_items[dir], &p->n_items[dir]);
     if (p->prec != SHT_PREC_F64)
-      item_list(dir, SimtCfg<float, true>::BX, &p->d_items_narrow[dir], &p->n_items_narrow[dir]);
+      item_list(dir, tile_x<float>(2), &p->d_items_narrow[dir], &p->n_items_narrow[dir]);
     for (int f = 0; f < 2; ++f) {
       auto& v = p->h_desc[dir][f];
       SHT_CUDA_OR_THROW(cudaMalloc(&p->d_desc[dir][f], sizeof(ShtGemmDesc) * std::max<size_t>(v.size(), 1)));
@@ -237,34 +290,71 @@ void build_gemm_items(sht_plan* p) {
   }
 }
 
+namespace {
+
+template <typename T, int WX, int DB>
+void launch_simt(const SimtArgs<T>& a, int n_items, cudaStream_t s) {
+  using C = SimtCfg<T>;
+  const size_t sm = sizeof(T) * C::S * C::BK * (tile_x<T>(WX) + tile_r<T>(C::G));
+  const int64_t blocks = (int64_t)n_items * a.nrb * a.ng;
+  SHT_REQUIRE(blocks < ((int64_t)1 << 31), "too many planes for one launch");
+  SHT_CUDA_OR_THROW(cudaFuncSetAttribute(gemm_simt_kernel<T, WX, DB>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  gemm_simt_kernel<T, WX, DB><<<(unsigned)blocks, 32 * WX, sm, s>>>(a);
+  SHT_CUDA_OR_THROW(cudaGetLastError());
+}
+
+}  // namespace
+
+template <typename T>
+void launch_gemm_simt_groups(const sht_plan* p, int direction, int ngroups, const int* flip,
+                             const T* const* table, const T* const* data, T* const* out,
+                             int64_t R, cudaStream_t s) {
+  // 64-wide tiles waste less of the ragged analysis blocks and hold twice as
+  // many CTAs; from 256 latitude pairs on the 128-wide ones' fewer table and
+  // data reloads make up for it (T511 x 200 planes 1921 against 1955 us; T255 x
+  // 161 planes 292 against 264, T126 x 200 planes 76 against 70).
+  const bool narrow = std::is_same<T, float>::value && (p->tune_simt_tile == 1 || p->H < 256);
+  const int n_items = narrow ? p->n_items_narrow[direction] : p->n_items[direction];
+  if (n_items == 0 || R == 0) return;
+  SHT_REQUIRE(ngroups == 1 || ngroups == 2, "one or two tables per SIMT launch");
+  SHT_REQUIRE(p->gemm_bx == tile_x<T>(4), "SIMT work list built for another tile width");
+  SimtArgs<T> a{};
+  for (int g = 0; g < ngroups; ++g)
+    a.g[g] = {p->d_desc[direction][flip[g]], table[g], data[g], out[g]};
+  a.items = narrow ? p->d_items_narrow[direction] : p->d_items[direction];
+  SHT_REQUIRE(a.items != nullptr, "SIMT work list not built");
+  a.ng = ngroups;
+  a.R = R;
+  const int whole = tile_r<T>(SimtCfg<T>::G);
+  a.nrb = (int)div_up(R, whole);
+  a.half = R % whole != 0 && R % whole <= whole / 2;
+  if constexpr (std::is_same<T, float>::value) {
+    const bool aligned = R % 4 == 0;
+    if (narrow && aligned) launch_simt<T, 2, 16>(a, n_items, s);
+    else if (narrow) launch_simt<T, 2, 8>(a, n_items, s);
+    else if (aligned) launch_simt<T, 4, 16>(a, n_items, s);
+    else launch_simt<T, 4, 8>(a, n_items, s);
+  } else {
+    launch_simt<T, 4, 16>(a, n_items, s);  // R is even: every data row is 16-byte aligned
+  }
+}
+
 template <typename T>
 void launch_gemm_simt(const sht_plan* p, int direction, int flip, const T* table, const T* data,
                       T* out, int64_t R, cudaStream_t s) {
-  if (p->n_items[direction] == 0 || R == 0) return;
-  if constexpr (std::is_same<T, float>::value) {
-    if (p->tune_simt_tile == 1) {
-      SHT_REQUIRE(p->d_items_narrow[direction] != nullptr, "narrow SIMT work list not built");
-      using C = SimtCfg<float, true>;
-      dim3 grid((unsigned)p->n_items_narrow[direction], (unsigned)div_up(R, C::BR));
-      SHT_REQUIRE(grid.y <= 65535, "too many planes for one launch");
-      gemm_simt_kernel<float, true><<<grid, 256, 0, s>>>(
-          p->d_desc[direction][flip], p->d_items_narrow[direction], table, data, out, R);
-      SHT_CUDA_OR_THROW(cudaGetLastError());
-      return;
-    }
-  }
-  using C = SimtCfg<T, false>;
-  SHT_REQUIRE(p->gemm_bx == C::BX, "SIMT work list built for another tile width");
-  dim3 grid((unsigned)p->n_items[direction], (unsigned)div_up(R, C::BR));
-  SHT_REQUIRE(grid.y <= 65535, "too many planes for one launch");
-  gemm_simt_kernel<T, false><<<grid, 256, 0, s>>>(p->d_desc[direction][flip], p->d_items[direction],
-                                                  table, data, out, R);
-  SHT_CUDA_OR_THROW(cudaGetLastError());
+  launch_gemm_simt_groups<T>(p, direction, 1, &flip, &table, &data, &out, R, s);
 }
 
 template void launch_gemm_simt<float>(const sht_plan*, int, int, const float*, const float*,
                                       float*, int64_t, cudaStream_t);
 template void launch_gemm_simt<double>(const sht_plan*, int, int, const double*, const double*,
                                        double*, int64_t, cudaStream_t);
+template void launch_gemm_simt_groups<float>(const sht_plan*, int, int, const int*,
+                                             const float* const*, const float* const*,
+                                             float* const*, int64_t, cudaStream_t);
+template void launch_gemm_simt_groups<double>(const sht_plan*, int, int, const int*,
+                                              const double* const*, const double* const*,
+                                              double* const*, int64_t, cudaStream_t);
 
 }  // namespace sht

@@ -66,7 +66,7 @@ struct sht_plan {
   int tune_contraction = 0;  // 1: FP32 SIMT contraction on a split16 plan
   int tune_tile_order = 0;   // tensor-core tile order (0: row blocks innermost, 1: column tiles)
   int tune_tc_ctas = 0;      // tensor-core CTAs per launch (0: one per SM)
-  int tune_simt_tile = 0;    // FP32 SIMT column tile (0: 128 wide; 1: 64 wide)
+  int tune_simt_tile = 0;    // FP32 SIMT column tile (0: by size, 128 or 64 wide; 1: 64 wide)
   int tune_accumulators = 0; // tensor-core accumulators (0: three K segments; 1: one, double-buffered;
                              // 2: two K segments, data operand in TMEM)
 
@@ -151,6 +151,11 @@ void build_gemm_items(sht_plan* p);
 template <typename T>
 void launch_gemm_simt(const sht_plan* p, int direction, int flip, const T* table,
                       const T* data, T* out, int64_t R, cudaStream_t s);
+// Two tables of one direction in one launch (R rows each).
+template <typename T>
+void launch_gemm_simt_groups(const sht_plan* p, int direction, int ngroups, const int* flip,
+                             const T* const* table, const T* const* data, T* const* out,
+                             int64_t R, cudaStream_t s);
 
 // Pack / unpack / elementwise (sht_pack.cu).
 enum PackMode { kPackPlain = 0, kPackInvLap = 1 };
