@@ -133,7 +133,7 @@ void ensure_scratch(sht_plan* p, int64_t R) {
     SHT_CUDA_OR_THROW(cudaMalloc(&p->wfold[i], p->elem() * std::max<int64_t>(p->wfold_elems(R), 1)));
     SHT_CUDA_OR_THROW(cudaMalloc(&p->cfold[i], p->elem() * std::max<int64_t>(p->cfold_elems(R), 1)));
   }
-  SHT_CUDA_OR_THROW(cudaMalloc(&p->rowmax, sizeof(float) * std::max<int64_t>(R, 1)));
+  SHT_CUDA_OR_THROW(cudaMalloc(&p->rowmax, sizeof(float) * (R + 4)));
   p->scratch_rows = R;
 }
 
@@ -218,45 +218,45 @@ void contract_pair(sht_plan* p, int kind0, const T* data0, const float* rm0, T* 
 
 template <typename T>
 void do_forward(sht_plan* p, const T* grid, int64_t planes, T* coeff, cudaStream_t s) {
-  const int64_t R = 2 * planes;
+  const int64_t ldc = padded_cols(planes), R = 2 * ldc;
   ensure_scratch(p, R);
   T* w = static_cast<T*>(p->wfold[0]);
   T* c = static_cast<T*>(p->cfold[0]);
   {
     float* rm = rowmax_for(p, R, s);
     KernelScope k(p, SHT_KIND_FFT_FORWARD, s);
-    launch_forward_fold<T>(p, grid, nullptr, planes, w, s, rm);
+    launch_forward_fold<T>(p, grid, nullptr, planes, ldc, w, s, rm);
   }
   contract<T>(p, kAnalysis, w, c, R, s);
   {
     KernelScope k(p, SHT_KIND_UNPACK, s);
-    launch_unpack<T>(p, kUnpackScalar, c, nullptr, planes, coeff, nullptr, s);
+    launch_unpack<T>(p, kUnpackScalar, c, nullptr, planes, ldc, coeff, nullptr, s);
   }
 }
 
 template <typename T>
 void do_synthesis(sht_plan* p, int kind, int mode, const T* coeff, int64_t planes, T* grid,
                   cudaStream_t s) {
-  const int64_t R = 2 * planes;
+  const int64_t ldc = padded_cols(planes), R = 2 * ldc;
   ensure_scratch(p, R);
   T* w = static_cast<T*>(p->wfold[0]);
   T* c = static_cast<T*>(p->cfold[0]);
   {
     float* rm = rowmax_for(p, R, s);
     KernelScope k(p, SHT_KIND_PACK, s);
-    launch_pack<T>(p, coeff, nullptr, planes, kPackPlain, c, s, rm);
+    launch_pack<T>(p, coeff, nullptr, planes, ldc, kPackPlain, c, s, rm);
   }
   contract<T>(p, kind, c, w, R, s);
   {
     KernelScope k(p, SHT_KIND_FFT_INVERSE, s);
-    launch_inverse_unfold<T>(p, mode, w, nullptr, planes, grid, nullptr, s);
+    launch_inverse_unfold<T>(p, mode, w, nullptr, planes, ldc, grid, nullptr, s);
   }
 }
 
 template <typename T>
 void do_gradient(sht_plan* p, const T* coeff, int64_t planes, T* east, T* north,
                  cudaStream_t s) {
-  const int64_t R = 2 * planes;
+  const int64_t ldc = padded_cols(planes), R = 2 * ldc;
   ensure_scratch(p, R);
   T* c = static_cast<T*>(p->cfold[0]);
   T* w0 = static_cast<T*>(p->wfold[0]);
@@ -264,19 +264,19 @@ void do_gradient(sht_plan* p, const T* coeff, int64_t planes, T* east, T* north,
   {
     float* rm = rowmax_for(p, R, s);
     KernelScope k(p, SHT_KIND_PACK, s);
-    launch_pack<T>(p, coeff, nullptr, planes, kPackPlain, c, s, rm);
+    launch_pack<T>(p, coeff, nullptr, planes, ldc, kPackPlain, c, s, rm);
   }
   contract2<T>(p, kBasis, w0, kDBasis, w1, c, R, s);
   {
     KernelScope k(p, SHT_KIND_FFT_INVERSE, s);
-    launch_inverse_unfold<T>(p, kUnfoldGradient, w0, w1, planes, east, north, s);
+    launch_inverse_unfold<T>(p, kUnfoldGradient, w0, w1, planes, ldc, east, north, s);
   }
 }
 
 template <typename T>
 void do_wind(sht_plan* p, const T* vort, const T* div, int64_t planes, T* u, T* v,
              cudaStream_t s) {
-  const int64_t R = 4 * planes;
+  const int64_t ldc = 2 * planes, R = 2 * ldc;
   ensure_scratch(p, R);
   T* c = static_cast<T*>(p->cfold[0]);
   T* w0 = static_cast<T*>(p->wfold[0]);
@@ -284,19 +284,19 @@ void do_wind(sht_plan* p, const T* vort, const T* div, int64_t planes, T* u, T* 
   {
     float* rm = rowmax_for(p, R, s);
     KernelScope k(p, SHT_KIND_PACK, s);
-    launch_pack<T>(p, vort, div, planes, kPackInvLap, c, s, rm);
+    launch_pack<T>(p, vort, div, planes, ldc, kPackInvLap, c, s, rm);
   }
   contract2<T>(p, kBasis, w0, kDBasis, w1, c, R, s);
   {
     KernelScope k(p, SHT_KIND_FFT_INVERSE, s);
-    launch_inverse_unfold<T>(p, kUnfoldWind, w0, w1, planes, u, v, s);
+    launch_inverse_unfold<T>(p, kUnfoldWind, w0, w1, planes, ldc, u, v, s);
   }
 }
 
 template <typename T>
 void do_vordiv(sht_plan* p, const T* u, const T* v, int64_t planes, T* vort, T* div,
                cudaStream_t s) {
-  const int64_t R = 4 * planes;
+  const int64_t ldc = 2 * planes, R = 2 * ldc;
   ensure_scratch(p, R);
   T* w = static_cast<T*>(p->wfold[0]);
   T* c0 = static_cast<T*>(p->cfold[0]);
@@ -304,12 +304,12 @@ void do_vordiv(sht_plan* p, const T* u, const T* v, int64_t planes, T* vort, T* 
   {
     float* rm = rowmax_for(p, R, s);
     KernelScope k(p, SHT_KIND_FFT_FORWARD, s);
-    launch_forward_fold<T>(p, u, v, planes, w, s, rm);
+    launch_forward_fold<T>(p, u, v, planes, ldc, w, s, rm);
   }
   contract2<T>(p, kRot, c0, kShear, c1, w, R, s);
   {
     KernelScope k(p, SHT_KIND_UNPACK, s);
-    launch_unpack<T>(p, kUnpackVorDiv, c0, c1, planes, vort, div, s);
+    launch_unpack<T>(p, kUnpackVorDiv, c0, c1, planes, ldc, vort, div, s);
   }
 }
 
@@ -321,7 +321,7 @@ void do_vordiv(sht_plan* p, const T* u, const T* v, int64_t planes, T* vort, T* 
 template <typename T>
 void do_vordiv_waist(sht_plan* p, const T* waist, int64_t planes, T* vort, T* div,
                      cudaStream_t s) {
-  const int64_t R = 4 * planes;
+  const int64_t ldc = 2 * planes, R = 2 * ldc;
   ensure_scratch(p, R);
   T* w = static_cast<T*>(p->wfold[0]);
   T* c0 = static_cast<T*>(p->cfold[0]);
@@ -329,12 +329,12 @@ void do_vordiv_waist(sht_plan* p, const T* waist, int64_t planes, T* vort, T* di
   {
     float* rm = rowmax_for(p, R, s);
     KernelScope k(p, SHT_KIND_PACK, s);
-    launch_waist_import<T>(p, waist, 2 * planes, 1.0, w, rm, s, 2);
+    launch_waist_import<T>(p, waist, 2 * planes, ldc, 1.0, w, rm, s, 2);
   }
   contract2<T>(p, kRot, c0, kShear, c1, w, R, s);
   {
     KernelScope k(p, SHT_KIND_UNPACK, s);
-    launch_unpack<T>(p, kUnpackVorDiv, c0, c1, planes, vort, div, s);
+    launch_unpack<T>(p, kUnpackVorDiv, c0, c1, planes, ldc, vort, div, s);
   }
 }
 
@@ -343,8 +343,8 @@ void do_vordiv_waist(sht_plan* p, const T* waist, int64_t planes, T* vort, T* di
 // on the v half only, each contraction at half the rows of the full pair.
 template <typename T>
 void do_divergence_waist(sht_plan* p, const T* waist, int64_t planes, T* div, cudaStream_t s) {
-  const int64_t R = 2 * planes;
-  ensure_scratch(p, 2 * R);
+  const int64_t ldc = padded_cols(planes), R = 2 * ldc;
+  ensure_scratch(p, 4 * planes);  // rowmax holds four rows more: 2 R of them here
   T* wu = static_cast<T*>(p->wfold[0]);
   T* wv = static_cast<T*>(p->wfold[1]);
   T* c0 = static_cast<T*>(p->cfold[0]);
@@ -353,14 +353,14 @@ void do_divergence_waist(sht_plan* p, const T* waist, int64_t planes, T* div, cu
   {
     float* rm = rowmax_for(p, 2 * R, s);
     KernelScope k(p, SHT_KIND_PACK, s);
-    launch_waist_import<T>(p, waist, planes, 1.0, wu, rm, s);
-    launch_waist_import<T>(p, waist + 2 * per_field, planes, 1.0, wv, rm ? rm + R : nullptr, s);
+    launch_waist_import<T>(p, waist, planes, ldc, 1.0, wu, rm, s);
+    launch_waist_import<T>(p, waist + 2 * per_field, planes, ldc, 1.0, wv, rm ? rm + R : nullptr, s);
   }
   const float* rm = uses_tc(p) ? p->rowmax : nullptr;
   contract_pair<T>(p, kRot, wu, rm, c0, kShear, wv, rm ? rm + R : nullptr, c1, R, s);
   {
     KernelScope k(p, SHT_KIND_UNPACK, s);
-    launch_unpack<T>(p, kUnpackDiv, c0, c1, planes, div, nullptr, s);
+    launch_unpack<T>(p, kUnpackDiv, c0, c1, planes, ldc, div, nullptr, s);
   }
 }
 
@@ -371,7 +371,7 @@ template <typename T>
 void do_helmholtz_synthesis(sht_plan* p, const sht_vertical* op, double tau_w, const T* div,
                             const T* theta, const T* lnps, T* odiv, T* otheta, T* olnps,
                             T* grid, cudaStream_t s) {
-  const int64_t planes = op->nlev, R = 2 * planes;
+  const int64_t planes = op->nlev, ldc = padded_cols(planes), R = 2 * ldc;
   ensure_scratch(p, R);
   T* c = static_cast<T*>(p->cfold[0]);
   T* w = static_cast<T*>(p->wfold[0]);
@@ -379,12 +379,12 @@ void do_helmholtz_synthesis(sht_plan* p, const sht_vertical* op, double tau_w, c
     float* rm = rowmax_for(p, R, s);
     KernelScope k(p, SHT_KIND_HELMHOLTZ, s);
     launch_semi_implicit<T>(p, op->nlev, static_cast<const T*>(op->mats), op->thermo, kSemiSolve,
-                            tau_w, 1.0, div, theta, lnps, odiv, otheta, olnps, nullptr, c, rm, s);
+                            tau_w, 1.0, div, theta, lnps, odiv, otheta, olnps, nullptr, c, ldc, rm, s);
   }
   contract<T>(p, kBasis, c, w, R, s);
   {
     KernelScope k(p, SHT_KIND_FFT_INVERSE, s);
-    launch_inverse_unfold<T>(p, kUnfoldScalar, w, nullptr, planes, grid, nullptr, s);
+    launch_inverse_unfold<T>(p, kUnfoldScalar, w, nullptr, planes, ldc, grid, nullptr, s);
   }
 }
 
@@ -408,12 +408,12 @@ void contract_batch(sht_batch* b, int kind, T* const* data, T* const* out, cudaS
       TcGroupSpec g[kMaxTcGroups];
       for (int i = 0; i < n; ++i)
         g[i] = {b->plans[i], dir, table_flip(kind), kind, data[i], b->plans[i]->rowmax, out[i],
-                2 * b->planes[i]};
+                2 * padded_cols(b->planes[i])};
       launch_gemm_tc_groups(g, n, b->cache, s);
       return;
     }
   }
-  for (int i = 0; i < n; ++i) contract<T>(b->plans[i], kind, data[i], out[i], 2 * b->planes[i], s);
+  for (int i = 0; i < n; ++i) contract<T>(b->plans[i], kind, data[i], out[i], 2 * padded_cols(b->planes[i]), s);
 }
 
 template <typename T>
@@ -423,19 +423,19 @@ void do_batch_forward(sht_batch* b, const void* const* grids, void* const* coeff
   T* c[kMaxTcGroups];
   for (int i = 0; i < n; ++i) {
     sht_plan* p = b->plans[i];
-    const int64_t planes = b->planes[i], R = 2 * planes;
+    const int64_t planes = b->planes[i], ldc = padded_cols(planes), R = 2 * ldc;
     ensure_scratch(p, R);
     w[i] = static_cast<T*>(p->wfold[0]);
     c[i] = static_cast<T*>(p->cfold[0]);
     float* rm = rowmax_for(p, R, s);
     KernelScope k(p, SHT_KIND_FFT_FORWARD, s);
-    launch_forward_fold<T>(p, static_cast<const T*>(grids[i]), nullptr, planes, w[i], s, rm);
+    launch_forward_fold<T>(p, static_cast<const T*>(grids[i]), nullptr, planes, ldc, w[i], s, rm);
   }
   contract_batch<T>(b, kAnalysis, w, c, s);
   for (int i = 0; i < n; ++i) {
     KernelScope k(b->plans[i], SHT_KIND_UNPACK, s);
     launch_unpack<T>(b->plans[i], kUnpackScalar, c[i], nullptr, b->planes[i],
-                     static_cast<T*>(coeffs[i]), nullptr, s);
+                     padded_cols(b->planes[i]),                     static_cast<T*>(coeffs[i]), nullptr, s);
   }
 }
 
@@ -446,19 +446,19 @@ void do_batch_inverse(sht_batch* b, const void* const* coeffs, void* const* grid
   T* c[kMaxTcGroups];
   for (int i = 0; i < n; ++i) {
     sht_plan* p = b->plans[i];
-    const int64_t planes = b->planes[i], R = 2 * planes;
+    const int64_t planes = b->planes[i], ldc = padded_cols(planes), R = 2 * ldc;
     ensure_scratch(p, R);
     w[i] = static_cast<T*>(p->wfold[0]);
     c[i] = static_cast<T*>(p->cfold[0]);
     float* rm = rowmax_for(p, R, s);
     KernelScope k(p, SHT_KIND_PACK, s);
-    launch_pack<T>(p, static_cast<const T*>(coeffs[i]), nullptr, planes, kPackPlain, c[i], s, rm);
+    launch_pack<T>(p, static_cast<const T*>(coeffs[i]), nullptr, planes, ldc, kPackPlain, c[i], s, rm);
   }
   contract_batch<T>(b, kBasis, c, w, s);
   for (int i = 0; i < n; ++i) {
     KernelScope k(b->plans[i], SHT_KIND_FFT_INVERSE, s);
     launch_inverse_unfold<T>(b->plans[i], kUnfoldScalar, w[i], nullptr, b->planes[i],
-                             static_cast<T*>(grids[i]), nullptr, s);
+                             padded_cols(b->planes[i]),                             static_cast<T*>(grids[i]), nullptr, s);
   }
 }
 
@@ -651,7 +651,7 @@ void host_streamed(sht_plan* p, int op, const void* hin, int64_t planes, void* h
                            op == kHostRoundTrip ? (size_t)(chunk * ce) * es : 0,
                            (size_t)(chunk * out_e) * es};
   host_stream_prepare(p, bytes);
-  ensure_scratch(p, 2 * chunk);
+  ensure_scratch(p, 2 * padded_cols(chunk));
   auto& h = p->hs;
   p->last_stream = h.s_comp;
   try {
@@ -1127,7 +1127,7 @@ int sht_semi_implicit_map(sht_plan* plan, const sht_vertical* op, int mode, doub
                                             op->thermo, kmode, dt_w, uses_alpha ? alpha : 1.0,
                                             CP(divergence), CP(theta), CP(lnps),
                                             MP(out_divergence), MP(out_theta), MP(out_lnps),
-                                            static_cast<T*>(op->metric), nullptr, nullptr, s));
+                                            static_cast<T*>(op->metric), nullptr, 0, nullptr, s));
   });
 }
 
@@ -1315,14 +1315,15 @@ int sht_fourier_waist(sht_plan* plan, const void* grid, int64_t planes, void* wa
     check_ptr(grid, "grid");
     check_ptr(waist, "waist");
     SHT_TYPED(plan, {
-      ensure_scratch(plan, 2 * planes);
+      const int64_t ldc = padded_cols(planes);
+      ensure_scratch(plan, 2 * ldc);
       T* w = static_cast<T*>(plan->wfold[0]);
       {
         KernelScope k(plan, SHT_KIND_FFT_FORWARD, s);
-        launch_forward_fold<T>(plan, CP(grid), nullptr, planes, w, s, nullptr);
+        launch_forward_fold<T>(plan, CP(grid), nullptr, planes, ldc, w, s, nullptr);
       }
       KernelScope k(plan, SHT_KIND_UNPACK, s);
-      launch_waist_export<T>(plan, w, planes, 0.5, 0, MP(waist), s);
+      launch_waist_export<T>(plan, w, planes, ldc, 0.5, 0, MP(waist), s);
     });
   });
 }
@@ -1334,18 +1335,19 @@ int sht_contract_waist(sht_plan* plan, const void* waist, int64_t planes, void* 
     check_ptr(waist, "waist");
     check_ptr(coeff, "coeff");
     SHT_TYPED(plan, {
-      const int64_t R = 2 * planes;
+      const int64_t ldc = padded_cols(planes);
+      const int64_t R = 2 * ldc;
       ensure_scratch(plan, R);
       T* w = static_cast<T*>(plan->wfold[0]);
       T* c = static_cast<T*>(plan->cfold[0]);
       {
         float* rm = rowmax_for(plan, R, s);
         KernelScope k(plan, SHT_KIND_PACK, s);
-        launch_waist_import<T>(plan, CP(waist), planes, 1.0, w, rm, s);
+        launch_waist_import<T>(plan, CP(waist), planes, ldc, 1.0, w, rm, s);
       }
       contract<T>(plan, kAnalysis, w, c, R, s);
       KernelScope k(plan, SHT_KIND_UNPACK, s);
-      launch_unpack<T>(plan, kUnpackScalar, c, nullptr, planes, MP(coeff), nullptr, s);
+      launch_unpack<T>(plan, kUnpackScalar, c, nullptr, planes, ldc, MP(coeff), nullptr, s);
     });
   });
 }
@@ -1359,18 +1361,19 @@ int sht_contract_to_waist(sht_plan* plan, const void* coeff, int64_t planes, int
     SHT_REQUIRE(table == SHT_WAIST_BASIS || table == SHT_WAIST_DBASIS || table == SHT_WAIST_ZONAL,
                 "table must be SHT_WAIST_BASIS, SHT_WAIST_DBASIS or SHT_WAIST_ZONAL");
     SHT_TYPED(plan, {
-      const int64_t R = 2 * planes;
+      const int64_t ldc = padded_cols(planes);
+      const int64_t R = 2 * ldc;
       ensure_scratch(plan, R);
       T* w = static_cast<T*>(plan->wfold[0]);
       T* c = static_cast<T*>(plan->cfold[0]);
       {
         float* rm = rowmax_for(plan, R, s);
         KernelScope k(plan, SHT_KIND_PACK, s);
-        launch_pack<T>(plan, CP(coeff), nullptr, planes, kPackPlain, c, s, rm);
+        launch_pack<T>(plan, CP(coeff), nullptr, planes, ldc, kPackPlain, c, s, rm);
       }
       contract<T>(plan, table == SHT_WAIST_DBASIS ? kDBasis : kBasis, c, w, R, s);
       KernelScope k(plan, SHT_KIND_UNPACK, s);
-      launch_waist_export<T>(plan, w, planes, 1.0, table == SHT_WAIST_ZONAL ? 1 : 0, MP(waist), s);
+      launch_waist_export<T>(plan, w, planes, ldc, 1.0, table == SHT_WAIST_ZONAL ? 1 : 0, MP(waist), s);
     });
   });
 }
@@ -1382,14 +1385,15 @@ int sht_waist_to_grid(sht_plan* plan, const void* waist, int64_t planes, void* g
     check_ptr(waist, "waist");
     check_ptr(grid, "grid");
     SHT_TYPED(plan, {
-      ensure_scratch(plan, 2 * planes);
+      const int64_t ldc = padded_cols(planes);
+      ensure_scratch(plan, 2 * ldc);
       T* w = static_cast<T*>(plan->wfold[0]);
       {
         KernelScope k(plan, SHT_KIND_PACK, s);
-        launch_waist_import<T>(plan, CP(waist), planes, 0.5, w, nullptr, s);
+        launch_waist_import<T>(plan, CP(waist), planes, ldc, 0.5, w, nullptr, s);
       }
       KernelScope k(plan, SHT_KIND_FFT_INVERSE, s);
-      launch_inverse_unfold<T>(plan, kUnfoldScalar, w, nullptr, planes, MP(grid), nullptr, s);
+      launch_inverse_unfold<T>(plan, kUnfoldScalar, w, nullptr, planes, ldc, MP(grid), nullptr, s);
     });
   });
 }

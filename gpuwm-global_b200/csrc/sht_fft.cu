@@ -373,6 +373,7 @@ struct FoldArgs {
   int nlat, nlon, T, H, nlat_odd;
   int F;         // fields stacked per plane (1 scalar, 2 for (u, v))
   int64_t cols;  // waist columns, planes * F
+  int64_t ldc;   // their stride
 };
 
 // grid (planes, nlat, nlon) per field -> waist [m][s][h][r], r = (p*F + f)*2 + c.
@@ -415,8 +416,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) forward_fold_kern
   const bool live = c0 + q < a.cols;
   float mre = 0.f, mim = 0.f;  // this thread's column maxima
   if (live) {
-    const int64_t dsd = (int64_t)a.H * a.cols;  // S row -> D row of the same order
-    V2<T>* dst = out + ((int64_t)(2 * (threadIdx.x >> lc)) * a.H + h) * a.cols + c0 + q;
+    const int64_t dsd = (int64_t)a.H * a.ldc;  // S row -> D row of the same order
+    V2<T>* dst = out + ((int64_t)(2 * (threadIdx.x >> lc)) * a.H + h) * a.ldc + c0 + q;
     for (int m = threadIdx.x >> lc; m <= a.T; m += mstep, dst += 2 * mstep * dsd) {
       const V2<T> w = tw_n[m];
       const int mc = m == 0 ? 0 : L - m;
@@ -447,6 +448,7 @@ struct UnfoldArgs {
   int nlat, nlon, T, H, nlat_odd;
   int zonal;   // NF = 1: multiply by i m
   int64_t planes;
+  int64_t ldc;  // waist column stride
   double radius;
 };
 
@@ -477,10 +479,9 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) inverse_unfold_ke
   {
     const int q = threadIdx.x & ((1 << lc) - 1), kstep = blockDim.x >> lc;
     const int64_t plane = min(p0 + q, a.planes - 1);  // past the end: transformed, not stored
-    const int64_t Rc = a.planes * FW;
-    const V2<T>* P2 = reinterpret_cast<const V2<T>*>(wP) + (int64_t)h * Rc + plane * FW;
-    const V2<T>* D2 = reinterpret_cast<const V2<T>*>(wD) + (int64_t)h * Rc + plane * FW;
-    const int64_t dsd = (int64_t)a.H * Rc;  // S row -> D row of the same order
+    const V2<T>* P2 = reinterpret_cast<const V2<T>*>(wP) + (int64_t)h * a.ldc + plane * FW;
+    const V2<T>* D2 = reinterpret_cast<const V2<T>*>(wD) + (int64_t)h * a.ldc + plane * FW;
+    const int64_t dsd = (int64_t)a.H * a.ldc;  // S row -> D row of the same order
     const T inv_a = T(1.0 / a.radius);
     T ie[2] = {T(0), T(0)};  // 1 / (a cos phi) of the two sides
     if constexpr (NF != 1) {
@@ -689,10 +690,10 @@ void build_fft(sht_plan* p, cudaStream_t s) {
 
 template <typename T>
 void launch_forward_fold(const sht_plan* p, const T* g0, const T* g1, int64_t planes,
-                         T* wfold, cudaStream_t s, float* rowmax) {
+                         int64_t ldc, T* wfold, cudaStream_t s, float* rowmax) {
   if constexpr (sizeof(T) == 4) {
     if (p->fast_fft) {
-      fast_forward_fold(p, g0, g1, planes, wfold, s, rowmax);
+      fast_forward_fold(p, g0, g1, planes, ldc, wfold, s, rowmax);
       return;
     }
   }
@@ -701,7 +702,7 @@ void launch_forward_fold(const sht_plan* p, const T* g0, const T* g1, int64_t pl
   size_t sm = 0;
   int threads = 0;
   const FftShape f = make_shape<T>(p, planes * fields, 1, &sm, &threads);
-  const FoldArgs a{f, p->nlat, p->nlon, p->T, p->H, p->nlat_odd ? 1 : 0, fields, planes * fields};
+  const FoldArgs a{f, p->nlat, p->nlon, p->T, p->H, p->nlat_odd ? 1 : 0, fields, planes * fields, ldc};
   allow_smem(forward_fold_kernel<T>, sm);
   const dim3 grid((unsigned)div_up(a.cols, (int64_t)1 << f.lc), (unsigned)p->H);
   forward_fold_kernel<T><<<grid, threads, sm, s>>>(a, g0, g1 ? g1 : g0, (const V2<T>*)p->tw_l,
@@ -710,13 +711,13 @@ void launch_forward_fold(const sht_plan* p, const T* g0, const T* g1, int64_t pl
 }
 
 template <typename T, int NF>
-void launch_unfold(const sht_plan* p, int mode, const T* wP, const T* wD, int64_t planes, T* out0,
-                   T* out1, cudaStream_t s) {
+void launch_unfold(const sht_plan* p, int mode, const T* wP, const T* wD, int64_t planes,
+                   int64_t ldc, T* out0, T* out1, cudaStream_t s) {
   size_t sm = 0;
   int threads = 0;
   const FftShape f = make_shape<T>(p, planes, NF == 1 ? 1 : 2, &sm, &threads);
   const UnfoldArgs a{f, p->nlat, p->nlon, p->T, p->H, p->nlat_odd ? 1 : 0,
-                     mode == kUnfoldZonal ? 1 : 0, planes, p->radius};
+                     mode == kUnfoldZonal ? 1 : 0, planes, ldc, p->radius};
   allow_smem(inverse_unfold_kernel<T, NF>, sm);
   const dim3 grid((unsigned)div_up(planes, (int64_t)1 << f.lc), (unsigned)p->H);
   inverse_unfold_kernel<T, NF><<<grid, threads, sm, s>>>(
@@ -727,28 +728,28 @@ void launch_unfold(const sht_plan* p, int mode, const T* wP, const T* wD, int64_
 
 template <typename T>
 void launch_inverse_unfold(const sht_plan* p, int mode, const T* wP, const T* wD,
-                           int64_t planes, T* out0, T* out1, cudaStream_t s) {
+                           int64_t planes, int64_t ldc, T* out0, T* out1, cudaStream_t s) {
   if constexpr (sizeof(T) == 4) {
     if (p->fast_fft) {
-      fast_inverse_unfold(p, mode, wP, wD, planes, out0, out1, s);
+      fast_inverse_unfold(p, mode, wP, wD, planes, ldc, out0, out1, s);
       return;
     }
   }
   if (mode == kUnfoldWind)
-    launch_unfold<T, 4>(p, mode, wP, wD, planes, out0, out1, s);
+    launch_unfold<T, 4>(p, mode, wP, wD, planes, ldc, out0, out1, s);
   else if (mode == kUnfoldGradient)
-    launch_unfold<T, 2>(p, mode, wP, wD, planes, out0, out1, s);
+    launch_unfold<T, 2>(p, mode, wP, wD, planes, ldc, out0, out1, s);
   else
-    launch_unfold<T, 1>(p, mode, wP, wD, planes, out0, out1, s);
+    launch_unfold<T, 1>(p, mode, wP, wD, planes, ldc, out0, out1, s);
 }
 
-template void launch_forward_fold<float>(const sht_plan*, const float*, const float*, int64_t,
+template void launch_forward_fold<float>(const sht_plan*, const float*, const float*, int64_t, int64_t,
                                          float*, cudaStream_t, float*);
-template void launch_forward_fold<double>(const sht_plan*, const double*, const double*, int64_t,
+template void launch_forward_fold<double>(const sht_plan*, const double*, const double*, int64_t, int64_t,
                                           double*, cudaStream_t, float*);
 template void launch_inverse_unfold<float>(const sht_plan*, int, const float*, const float*,
-                                           int64_t, float*, float*, cudaStream_t);
+                                           int64_t, int64_t, float*, float*, cudaStream_t);
 template void launch_inverse_unfold<double>(const sht_plan*, int, const double*, const double*,
-                                            int64_t, double*, double*, cudaStream_t);
+                                            int64_t, int64_t, double*, double*, cudaStream_t);
 
 }  // namespace sht

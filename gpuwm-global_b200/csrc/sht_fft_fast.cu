@@ -250,30 +250,10 @@ __device__ __forceinline__ void warp_fft_rows(float2 (&z)[R][F], float2* reg, in
   __syncwarp();
 }
 
-// The L-point complex FFT of one warp's row: in registers z[j] = x[l + 32 j]
-// (lane l); out: the natural-order spectrum written to `reg` (length L).
-template <int F, bool INV>
-__device__ __forceinline__ void warp_fft(float2 (&z)[F], float2* reg, const float2* tws, int lane) {
-  float2(&z1)[1][F] = *reinterpret_cast<float2(*)[1][F]>(&z);
-  warp_fft_rows<F, 1, INV, false>(z1, reg, 0, tws, lane);
-}
-
-// A CTA runs kWarps warps, one grid row each: G planes x NF fields x the two
-// hemisphere rows (8 rows).
-constexpr int kWarps = 8;
-
-// An opaque copy of a pointer.  The inverse kernel reads its entangling
-// twiddles through it, so the compiler cannot hoist a whole row of them into
-// registers ahead of the butterflies (~20 registers per thread, one resident
-// CTA per SM fewer).
-__device__ __forceinline__ const float2* opaque(const float2* p) {
-  asm volatile("" : "+l"(p));
-  return p;
-}
-
 struct FastFoldArgs {
   int nlat, nlon, T, H, nlat_odd, F, G;  // F: fields per plane; G: planes per CTA
   int64_t planes;
+  int64_t ldc;  // waist column stride
   int pf_dist;  // latitude pairs ahead whose rows a CTA prefetches into L2 (0: none)
 };
 
@@ -353,7 +333,7 @@ __global__ void __launch_bounds__(W * 32, 24 / W) fast_forward_fold(FastFoldArgs
   // 0.5 / nlon: (x / 2) / nlon and x * (0.5 / nlon) round alike (both
   // scalings by 2 are exact).
   const float half_inv_n = 0.5f / (float)a.nlon;
-  const int64_t Rc = a.planes * a.F;  // complex columns per waist row
+  const int64_t Rc = a.ldc;           // waist column stride
   float mre = 0.f, mim = 0.f;         // this thread's column maxima
   const int T = TC >= 0 ? TC : a.T;   // compile-time on the linear grid
   // Thread -> column q (fixed: blockDim is a multiple of nper) and orders
@@ -398,129 +378,9 @@ __global__ void __launch_bounds__(W * 32, 24 / W) fast_forward_fold(FastFoldArgs
 struct FastUnfoldArgs {
   int nlat, nlon, T, H, nlat_odd, mode, G;
   int64_t planes;
+  int64_t ldc;  // waist column stride (even: 16-byte rows)
   float radius;
 };
-
-// waist(s) -> grid.  Warp w handles (row pair index po = w >> 1, side = w & 1)
-// with po = gp*NO + o (o: output field).  NF waist columns feed each
-// (m, plane): 1 (scalar, zonal, meridional), 2 (gradient: the P and dP
-// syntheses of one field), 4 (wind: P and dP of psi and chi).
-template <int FF, int NF>
-__global__ void __launch_bounds__(kWarps * 32) fast_inverse_unfold(FastUnfoldArgs a,
-                                                                   const float2* __restrict__ wP,
-                                                                   const float2* __restrict__ wD,
-                                                                   const double* __restrict__ coslat,
-                                                                   const float2* __restrict__ twL,
-                                                                   const float2* __restrict__ twN,
-                                                                   float* __restrict__ out0,
-                                                                   float* __restrict__ out1) {
-  constexpr int L = 32 * FF;
-  constexpr int NO = NF == 1 ? 1 : 2;
-  extern __shared__ float2 smem_dyn[];
-  auto smem = [&](int w) { return smem_dyn + w * WarpSmem<FF>::kFloats2; };
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // Plane blocks vary fastest over the grid: CTAs that run together touch
-  // adjacent slices of every waist row.
-  const int h = blockIdx.y;
-  const int64_t p0 = (int64_t)blockIdx.x * a.G;
-  const bool eq = a.nlat_odd && h == a.H - 1;
-  const int64_t Rc = a.planes * (NF == 4 ? 2 : 1);
-  const float inv_a = 1.0f / a.radius;
-  const int jmir = a.nlat - 1 - h;  // the mirror row (side 1)
-
-  float2* tws = smem_dyn + kWarps * WarpSmem<FF>::kFloats2;
-  load_lane_twiddles<FF>(tws, twL);
-  // Stage 1: Fourier coefficients of every output row into smem[row][m].
-  // Each thread first issues the waist loads of kBatch items (NF symmetric /
-  // antisymmetric pairs each), then combines them: the loads of a batch are
-  // in flight together instead of one dependent round trip per item.
-  constexpr int kBatch = NF == 4 ? 2 : 4;
-  constexpr int G = kWarps / 2 / NO;  // planes per CTA
-  const int total = (a.T + 1) * G;
-  for (int base = threadIdx.x; base < total; base += kBatch * blockDim.x) {
-    float2 S[kBatch][NF], D[kBatch][NF];
-#pragma unroll
-    for (int u = 0; u < kBatch; ++u) {
-      const int t = base + u * blockDim.x;
-      const int m = t / G, gp = t - m * G;
-      if (t < total && p0 + gp < a.planes) {
-        const int64_t r = (p0 + gp) * (NF == 4 ? 2 : 1);
-        const int64_t c0 = ((int64_t)(m * 2 + 0) * a.H + h) * Rc + r;
-        const int64_t c1 = ((int64_t)(m * 2 + 1) * a.H + h) * Rc + r;
-#pragma unroll
-        for (int k = 0; k < NF; ++k) {
-          const float2* w = (NF == 1 || k < NF / 2) ? wP : wD;
-          const int fld = NF == 4 ? (k & 1) : 0;
-          S[u][k] = __ldcs(w + c0 + fld);
-          D[u][k] = __ldcs(w + c1 + fld);
-        }
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < kBatch; ++u) {
-      const int t = base + u * blockDim.x;
-      const int m = t / G, gp = t - m * G;
-      if (t >= total || p0 + gp >= a.planes) continue;
-#pragma unroll
-      for (int sd = 0; sd < 2; ++sd) {
-        if (sd == 1 && eq) continue;
-        const float sgn = sd ? -1.f : 1.f;
-        float2 x[NF];
-#pragma unroll
-        for (int k = 0; k < NF; ++k)
-          x[k] = make_float2(S[u][k].x + sgn * D[u][k].x, S[u][k].y + sgn * D[u][k].y);
-        float2 o0, o1 = make_float2(0.f, 0.f);
-        if constexpr (NF == 1) {
-          o0 = a.mode == kUnfoldZonal ? make_float2(-(float)m * x[0].y, (float)m * x[0].x) : x[0];
-        } else if constexpr (NF == 2) {
-          o0 = make_float2(-(float)m * x[0].y, (float)m * x[0].x);
-          o1 = x[1];
-        } else {
-          // x = {P psi, P chi, dP psi, dP chi}
-          const float im_over = (float)m / (a.radius * (float)coslat[sd ? jmir : h]);
-          o0 = make_float2(-x[2].x * inv_a - im_over * x[1].y, -x[2].y * inv_a + im_over * x[1].x);
-          o1 = make_float2(-im_over * x[0].y + x[3].x * inv_a, im_over * x[0].x + x[3].y * inv_a);
-        }
-        smem((gp * NO + 0) * 2 + sd)[m] = o0;
-        if (NO == 2) smem((gp * NO + 1) * 2 + sd)[m] = o1;
-      }
-    }
-  }
-  __syncthreads();
-  const int po = warp >> 1, side = warp & 1;
-  const int o = po % NO, gp = po / NO;
-  const int64_t plane = p0 + gp;
-  if (po >= G * NO || plane >= a.planes || (eq && side == 1)) return;
-  float2* reg = smem(warp);
-  const float2* tn = opaque(twN);
-  // Stage 2: entangle z[k] for k = lane + 32 j straight into registers.
-  float2 z[FF];
-#pragma unroll
-  for (int i = 0; i < FF; ++i) {
-    int k = lane + 32 * i;
-    float2 xk = k <= a.T ? reg[k] : make_float2(0.f, 0.f);
-    int kc = L - k;
-    float2 xc = (k > 0 && kc <= a.T) ? cconjf(reg[kc]) : make_float2(0.f, 0.f);
-    if (k == 0) xk.y = 0.f;
-    float2 s = caddf(xk, xc), d = csubf(xk, xc);
-    float2 wd = cmulf(cconjf(tn[k]), d);
-    z[i] = make_float2(s.x - wd.y, s.y + wd.x);
-  }
-  __syncwarp();
-  warp_fft<FF, true>(z, reg, tws, lane);
-  // Stage 3: natural-order z[n] -> x[2n], x[2n+1] with the row scaling.
-  const int j = side ? jmir : h;
-  // The gradient divides the grid by (a cos phi) and by a, as the reference does.
-  const bool divide = NF == 2;
-  const float den = o == 0 ? a.radius * (float)coslat[j] : a.radius;
-  float2* dst = reinterpret_cast<float2*>((o ? out1 : out0) + (plane * a.nlat + j) * (int64_t)a.nlon);
-#pragma unroll 4
-  for (int i = 0; i < FF; ++i) {
-    float2 v = reg[lane + 32 * i];
-    if (divide) v = make_float2(v.x / den, v.y / den);
-    __stcs(dst + lane + 32 * i, v);
-  }
-}
 
 // The scalar inverse (one waist column per plane: scalar, zonal, meridional)
 // as a persistent kernel: each CTA walks a strided list of items (4 planes x
@@ -586,7 +446,7 @@ __global__ void __launch_bounds__(InvCfg<NF>::W * 32, 16 / InvCfg<NF>::W)
   float2* twn = tws + FF * 32;    // the entangling twiddles exp(-2 pi i k / nlon), k < L
   float2* stage = twn + 32 * FF;  // [buffer][s][m][CW] waist slices of the item in flight
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t Rc = NF == 4 ? 2 * a.planes : a.planes;  // waist columns per row
+  const int64_t Rc = a.ldc;  // waist column stride
   const int nms = 2 * (a.T + 1);
   const int64_t n_items = (int64_t)n_pb * a.H;
   // Item i: plane block i % n_pb (fastest: CTAs that run together touch
@@ -600,8 +460,7 @@ __global__ void __launch_bounds__(InvCfg<NF>::W * 32, 16 / InvCfg<NF>::W)
       const float2* w = b ? wD : wP;
       for (int e = threadIdx.x; e < nms * (CW / 2); e += blockDim.x) {
         const int c = e % (CW / 2), ms = e / (CW / 2);  // compile-time divisor
-        const int64_t valid = Rc - (c0 + 2 * c);  // columns that exist from this chunk on
-        const uint32_t bytes = valid >= 2 ? 16u : (valid == 1 ? 8u : 0u);
+        const uint32_t bytes = c0 + 2 * c < Rc ? 16u : 0u;  // Rc is even: whole chunks
         const float2* src = bytes ? w + ((int64_t)ms * a.H + h) * Rc + c0 + 2 * c : wP;
         // S (s = 0) and D (s = 1) in separate halves, orders contiguous.
         cp_async16(stage + ((b * 2 + (ms & 1)) * (a.T + 1) + (ms >> 1)) * CW + 2 * c, src, bytes);
@@ -758,14 +617,14 @@ int resident_ctas(K kernel, int threads, size_t sm) {
   return per_sm;
 }
 
-// The waist rows must be 16-byte aligned for cp.async: an even plane count.
+// The waist rows must be 16-byte aligned for cp.async: an even column stride.
 // One persistent CTA per resident slot.
 template <int FF, int NF, int TC>
 void launch_inv_pair_t(const sht_plan* p, int mode, const float* wP, const float* wD,
-                       int64_t planes, float* out0, float* out1, cudaStream_t s) {
+                       int64_t planes, int64_t ldc, float* out0, float* out1, cudaStream_t s) {
   constexpr int kW = InvCfg<NF>::W, NB = InvCfg<NF>::NB, R = RowsPerWarp<FF>::R;
   constexpr int GI = InvCfg<NF>::G * R, CW = NF == 4 ? 2 * GI : GI;
-  FastUnfoldArgs a{p->nlat, p->nlon, p->T, p->H, p->nlat_odd ? 1 : 0, mode, GI, planes,
+  FastUnfoldArgs a{p->nlat, p->nlon, p->T, p->H, p->nlat_odd ? 1 : 0, mode, GI, planes, ldc,
                    (float)p->radius};
   const int n_pb = (int)div_up(planes, GI);
   const size_t sm = sizeof(float2) * (kW * R * WarpSmem<FF>::kFloats2 + 2 * FF * 32 +
@@ -779,17 +638,15 @@ void launch_inv_pair_t(const sht_plan* p, int mode, const float* wP, const float
       (const float2*)p->tw_n, out0, out1 ? out1 : out0, n_pb);
   SHT_CUDA_OR_THROW(cudaGetLastError());
 }
-// The waist rows must be 16-byte aligned for cp.async: for NF = 1, 2 (one
-// waist column per plane) an even plane count; NF = 4 (two per plane) any.
 template <int FF, int NF>
 void launch_inv_pair(const sht_plan* p, int mode, const float* wP, const float* wD,
-                     int64_t planes, float* out0, float* out1, cudaStream_t s) {
+                     int64_t planes, int64_t ldc, float* out0, float* out1, cudaStream_t s) {
   // The linear grid's truncation, T + 1 = 2 nlon / 3 = 64 F / 3, when it is whole.
   constexpr int TLIN = (64 * FF) % 3 == 0 ? 64 * FF / 3 - 1 : -1;
   if (TLIN >= 0 && p->T == TLIN)
-    launch_inv_pair_t<FF, NF, TLIN>(p, mode, wP, wD, planes, out0, out1, s);
+    launch_inv_pair_t<FF, NF, TLIN>(p, mode, wP, wD, planes, ldc, out0, out1, s);
   else
-    launch_inv_pair_t<FF, NF, -1>(p, mode, wP, wD, planes, out0, out1, s);
+    launch_inv_pair_t<FF, NF, -1>(p, mode, wP, wD, planes, ldc, out0, out1, s);
 }
 
 // L2 prefetch of the rows one resident wave ahead in the forward FFT.
@@ -800,10 +657,10 @@ constexpr bool kFwdPrefetch = true;
 constexpr int kFwdWarps = 8;
 template <int FF, int TC>
 void launch_fwd_t(const sht_plan* p, const float* g0, const float* g1, int64_t planes,
-                  float* wfold, cudaStream_t s, float* rowmax) {
+                  int64_t ldc, float* wfold, cudaStream_t s, float* rowmax) {
   constexpr int W = kFwdWarps;
   constexpr int R = RowsPerWarp<FF>::R;
-  FastFoldArgs a{p->nlat, p->nlon, p->T, p->H, p->nlat_odd ? 1 : 0, g1 ? 2 : 1, 0, planes, 0};
+  FastFoldArgs a{p->nlat, p->nlon, p->T, p->H, p->nlat_odd ? 1 : 0, g1 ? 2 : 1, 0, planes, ldc, 0};
   a.G = W / 2 * R / a.F;  // planes per CTA
   dim3 grid((unsigned)div_up(planes, a.G), (unsigned)p->H);
   const size_t sm = sizeof(float2) * (W * R * WarpSmem<FF>::kFloats2 + FF * 32 + p->T + 1);
@@ -818,44 +675,25 @@ void launch_fwd_t(const sht_plan* p, const float* g0, const float* g1, int64_t p
   SHT_CUDA_OR_THROW(cudaGetLastError());
 }
 template <int FF>
-void launch_fwd(const sht_plan* p, const float* g0, const float* g1, int64_t planes, float* wfold,
-                cudaStream_t s, float* rowmax) {
+void launch_fwd(const sht_plan* p, const float* g0, const float* g1, int64_t planes, int64_t ldc,
+                float* wfold, cudaStream_t s, float* rowmax) {
   constexpr int TLIN = (64 * FF) % 3 == 0 ? 64 * FF / 3 - 1 : -1;  // T + 1 = 2 nlon / 3
   if (TLIN >= 0 && p->T == TLIN)
-    launch_fwd_t<FF, TLIN>(p, g0, g1, planes, wfold, s, rowmax);
+    launch_fwd_t<FF, TLIN>(p, g0, g1, planes, ldc, wfold, s, rowmax);
   else
-    launch_fwd_t<FF, -1>(p, g0, g1, planes, wfold, s, rowmax);
-}
-
-template <int FF, int NF>
-void launch_inv_nf(const sht_plan* p, int mode, const float* wP, const float* wD, int64_t planes,
-                   float* out0, float* out1, cudaStream_t s) {
-  constexpr int NO = NF == 1 ? 1 : 2;
-  FastUnfoldArgs a{p->nlat, p->nlon, p->T, p->H, p->nlat_odd ? 1 : 0, mode, kWarps / 2 / NO,
-                   planes, (float)p->radius};
-  dim3 grid((unsigned)div_up(planes, a.G), (unsigned)p->H);
-  const size_t sm = sizeof(float2) * (kWarps * WarpSmem<FF>::kFloats2 + FF * 32);
-  SHT_CUDA_OR_THROW(cudaFuncSetAttribute(fast_inverse_unfold<FF, NF>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  fast_inverse_unfold<FF, NF><<<grid, kWarps * 32, sm, s>>>(
-      a, (const float2*)wP, (const float2*)(wD ? wD : wP), p->d_coslat, (const float2*)p->tw_l,
-      (const float2*)p->tw_n, out0, out1 ? out1 : out0);
-  SHT_CUDA_OR_THROW(cudaGetLastError());
+    launch_fwd_t<FF, -1>(p, g0, g1, planes, ldc, wfold, s, rowmax);
 }
 
 template <int FF>
 void launch_inv(const sht_plan* p, int mode, const float* wP, const float* wD, int64_t planes,
-                float* out0, float* out1, cudaStream_t s) {
+                int64_t ldc, float* out0, float* out1, cudaStream_t s) {
+  SHT_REQUIRE(ldc % 2 == 0, "the inverse FFT reads 16-byte waist rows: an even column stride");
   if (mode == kUnfoldWind)
-    launch_inv_pair<FF, 4>(p, mode, wP, wD, planes, out0, out1, s);
-  else if (mode == kUnfoldGradient && planes % 2 == 0)
-    launch_inv_pair<FF, 2>(p, mode, wP, wD, planes, out0, out1, s);
+    launch_inv_pair<FF, 4>(p, mode, wP, wD, planes, ldc, out0, out1, s);
   else if (mode == kUnfoldGradient)
-    launch_inv_nf<FF, 2>(p, mode, wP, wD, planes, out0, out1, s);
-  else if (planes % 2 == 0)
-    launch_inv_pair<FF, 1>(p, mode, wP, wD, planes, out0, out1, s);
+    launch_inv_pair<FF, 2>(p, mode, wP, wD, planes, ldc, out0, out1, s);
   else
-    launch_inv_nf<FF, 1>(p, mode, wP, wD, planes, out0, out1, s);
+    launch_inv_pair<FF, 1>(p, mode, wP, wD, planes, ldc, out0, out1, s);
 }
 
 }  // namespace
@@ -880,31 +718,31 @@ void fast_fft_init_constants(cudaStream_t s) {
 }
 
 void fast_forward_fold(const sht_plan* p, const float* g0, const float* g1, int64_t planes,
-                       float* wfold, cudaStream_t s, float* rowmax) {
+                       int64_t ldc, float* wfold, cudaStream_t s, float* rowmax) {
   switch (p->L / 32) {
-    case 2: launch_fwd<2>(p, g0, g1, planes, wfold, s, rowmax); break;
-    case 3: launch_fwd<3>(p, g0, g1, planes, wfold, s, rowmax); break;
-    case 4: launch_fwd<4>(p, g0, g1, planes, wfold, s, rowmax); break;
-    case 6: launch_fwd<6>(p, g0, g1, planes, wfold, s, rowmax); break;
-    case 8: launch_fwd<8>(p, g0, g1, planes, wfold, s, rowmax); break;
-    case 12: launch_fwd<12>(p, g0, g1, planes, wfold, s, rowmax); break;
-    case 16: launch_fwd<16>(p, g0, g1, planes, wfold, s, rowmax); break;
-    case 24: launch_fwd<24>(p, g0, g1, planes, wfold, s, rowmax); break;
+    case 2: launch_fwd<2>(p, g0, g1, planes, ldc, wfold, s, rowmax); break;
+    case 3: launch_fwd<3>(p, g0, g1, planes, ldc, wfold, s, rowmax); break;
+    case 4: launch_fwd<4>(p, g0, g1, planes, ldc, wfold, s, rowmax); break;
+    case 6: launch_fwd<6>(p, g0, g1, planes, ldc, wfold, s, rowmax); break;
+    case 8: launch_fwd<8>(p, g0, g1, planes, ldc, wfold, s, rowmax); break;
+    case 12: launch_fwd<12>(p, g0, g1, planes, ldc, wfold, s, rowmax); break;
+    case 16: launch_fwd<16>(p, g0, g1, planes, ldc, wfold, s, rowmax); break;
+    case 24: launch_fwd<24>(p, g0, g1, planes, ldc, wfold, s, rowmax); break;
     default: throw Error{SHT_ERR_STATE, "fast FFT: unsupported length"};
   }
 }
 
 void fast_inverse_unfold(const sht_plan* p, int mode, const float* wP, const float* wD,
-                         int64_t planes, float* out0, float* out1, cudaStream_t s) {
+                         int64_t planes, int64_t ldc, float* out0, float* out1, cudaStream_t s) {
   switch (p->L / 32) {
-    case 2: launch_inv<2>(p, mode, wP, wD, planes, out0, out1, s); break;
-    case 3: launch_inv<3>(p, mode, wP, wD, planes, out0, out1, s); break;
-    case 4: launch_inv<4>(p, mode, wP, wD, planes, out0, out1, s); break;
-    case 6: launch_inv<6>(p, mode, wP, wD, planes, out0, out1, s); break;
-    case 8: launch_inv<8>(p, mode, wP, wD, planes, out0, out1, s); break;
-    case 12: launch_inv<12>(p, mode, wP, wD, planes, out0, out1, s); break;
-    case 16: launch_inv<16>(p, mode, wP, wD, planes, out0, out1, s); break;
-    case 24: launch_inv<24>(p, mode, wP, wD, planes, out0, out1, s); break;
+    case 2: launch_inv<2>(p, mode, wP, wD, planes, ldc, out0, out1, s); break;
+    case 3: launch_inv<3>(p, mode, wP, wD, planes, ldc, out0, out1, s); break;
+    case 4: launch_inv<4>(p, mode, wP, wD, planes, ldc, out0, out1, s); break;
+    case 6: launch_inv<6>(p, mode, wP, wD, planes, ldc, out0, out1, s); break;
+    case 8: launch_inv<8>(p, mode, wP, wD, planes, ldc, out0, out1, s); break;
+    case 12: launch_inv<12>(p, mode, wP, wD, planes, ldc, out0, out1, s); break;
+    case 16: launch_inv<16>(p, mode, wP, wD, planes, ldc, out0, out1, s); break;
+    case 24: launch_inv<24>(p, mode, wP, wD, planes, ldc, out0, out1, s); break;
     default: throw Error{SHT_ERR_STATE, "fast FFT: unsupported length"};
   }
 }

@@ -349,11 +349,9 @@ __device__ __forceinline__ float pow2_scale(float mx) {
 // operand with its row maxima, and the output.  A launch runs the merged,
 // cost-sorted tiles of up to kMaxTcGroups of them.
 struct alignas(64) TcGroup {
-  CUtensorMap data_map;    // the data operand as a [rows][R] FP32 tensor (when use_tma)
-  int use_tma;             // 1: the loader brings the data tiles in by TMA
+  CUtensorMap data_map;    // the data operand as a [rows][R] FP32 tensor
   const unsigned char* img;
   const float* colscale;
-  const float* data;
   const float* rowmax;     // per data row: max |value| (from the producer kernel)
   float* out;
   int64_t R;
@@ -550,7 +548,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
     // its stage finish): the data runs up to S stages ahead of the converted
     // operand ring, which is what keeps the tensor pipe fed across the
     // memory latency.
-    if (lane == 0 && a.g[0].use_tma) {
+    if (lane == 0) {
       int stage = 0;
       uint32_t phase = 0;
       int armed[S];
@@ -805,33 +803,24 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
       const int64_t R = G.R;
       const int64_t r = tl.r0 + rowi;
       const float sc = r < R ? row_scale(G, r) : 1.f;
-      const float* Db = G.data + tl.d_row * R;
       bool ok = true;
       for (int ks = 0; ks < tl.kst; ++ks) {
         float v[16];
-        if (G.use_tma) {
-          // Box q4 of the stage holds rows q4*32 .. +31 as 128-byte k rows,
-          // 16-byte chunks swizzled by k % 8.
-          ok = wait_bar(&pp.full_raw[stage], phase, pp, a.err, 8);
-          if (!ok) break;
-          const unsigned char* box = sRaw + stage * kRawStage + q4 * kRawBox;
+        // Box q4 of the stage holds rows q4*32 .. +31 as 128-byte k rows,
+        // 16-byte chunks swizzled by k % 8.
+        ok = wait_bar(&pp.full_raw[stage], phase, pp, a.err, 8);
+        if (!ok) break;
+        const unsigned char* box = sRaw + stage * kRawStage + q4 * kRawBox;
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const int kl = kh * 16 + i;
-            const float x = *reinterpret_cast<const float*>(
-                box + kl * 128 + ((((lane >> 2) ^ (kl & 7))) << 4) + (lane & 3) * 4);
-            v[i] = ks * BK + kl < tl.K ? x : 0.f;  // rows past K belong to the next problem
-          }
-          __syncwarp();  // the warp's reads of the raw stage are done
-          if (lane == 0) mbar_arrive(&pp.raw_empty[stage]);
-          if (++stage == S) { stage = 0; phase ^= 1; }
-        } else {
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const int k = ks * BK + kh * 16 + i;
-            v[i] = (k < tl.K && r < R) ? __ldg(Db + (int64_t)k * R + r) : 0.f;
-          }
+        for (int i = 0; i < 16; ++i) {
+          const int kl = kh * 16 + i;
+          const float x = *reinterpret_cast<const float*>(
+              box + kl * 128 + ((((lane >> 2) ^ (kl & 7))) << 4) + (lane & 3) * 4);
+          v[i] = ks * BK + kl < tl.K ? x : 0.f;  // rows past K belong to the next problem
         }
+        __syncwarp();  // the warp's reads of the raw stage are done
+        if (lane == 0) mbar_arrive(&pp.raw_empty[stage]);
+        if (++stage == S) { stage = 0; phase ^= 1; }
         // The TMEM slot's previous MMAs are done.
         ok = wait_bar(&pp.a_empty[aslot], aphase ^ 1, pp, a.err, 7);
         if (!ok) break;
@@ -872,35 +861,10 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
       if (tl.kst == 0) continue;
       const TcGroup& G = a.g[tl.group];
       const int64_t R = G.R;
-      const float* Db = G.data + tl.d_row * R;
       const int64_t rbase = tl.r0 + mg * 8;
       float sc[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) sc[i] = rbase + i < R ? row_scale(G, rbase + i) : 1.f;
-      const bool full_rows = rbase + 8 <= R && (R % 4) == 0;
-      // Stage ks + 1 is loaded while stage ks waits for its slot and is
-      // converted (two register buffers, swapped by a 2x unrolled loop).
-      auto load_stage = [&](int ks, float (&v)[BK / 16][8]) {
-#pragma unroll
-        for (int j = 0; j < BK / 16; ++j) {
-          const int k = ks * BK + (kgs + 2 * j) * 8 + kk;
-          if (k < tl.K) {
-            const float* p = Db + (int64_t)k * R + rbase;
-            if (full_rows) {
-              const float4 u0 = __ldg(reinterpret_cast<const float4*>(p));
-              const float4 u1 = __ldg(reinterpret_cast<const float4*>(p + 4));
-              v[j][0] = u0.x; v[j][1] = u0.y; v[j][2] = u0.z; v[j][3] = u0.w;
-              v[j][4] = u1.x; v[j][5] = u1.y; v[j][6] = u1.z; v[j][7] = u1.w;
-            } else {
-#pragma unroll
-              for (int i = 0; i < 8; ++i) v[j][i] = (rbase + i < R) ? __ldg(p + i) : 0.f;
-            }
-          } else {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) v[j][i] = 0.f;
-          }
-        }
-      };
       // The stage's data from the TMA-filled shared tile: boxes of 32 rows
       // x 32 k with the 16-byte chunks of each 128-byte k row XOR-swizzled
       // by (k mod 8), which makes this warp's reads (8 consecutive k of one
@@ -921,8 +885,8 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
           v[j][6] = live ? u1.z : 0.f; v[j][7] = live ? u1.w : 0.f;
         }
       };
-      auto convert_stage = [&](const float (&v)[BK / 16][8], bool wait_slot) -> bool {
-        if (wait_slot && !wait_bar(&pp.empty[stage], phase ^ 1, pp, a.err, 7)) return false;
+      auto convert_stage = [&](const float (&v)[BK / 16][8]) -> bool {
+        if (!wait_bar(&pp.empty[stage], phase ^ 1, pp, a.err, 7)) return false;
         unsigned char* dst = sA + stage * NPARTS * kAPart;
 #pragma unroll
         for (int j = 0; j < BK / 16; ++j) {
@@ -946,28 +910,17 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
         return true;
       };
       bool ok = true;
-      float va[BK / 16][8], vb[BK / 16][8];
-      if (G.use_tma) {
-        // Read the raw stage into registers and hand it back at once, then
-        // wait for the converted-operand slot.
-        for (int ks = 0; ks < tl.kst && ok; ++ks) {
-          ok = wait_bar(&pp.full_raw[rstage], rphase, pp, a.err, 8);
-          if (!ok) break;
-          fetch_raw(ks, va);
-          __syncwarp();  // the warp's reads of the raw stage are done
-          if ((threadIdx.x & 31) == 0) mbar_arrive(&pp.raw_empty[rstage]);
-          if (++rstage == S) { rstage = 0; rphase ^= 1; }
-          ok = convert_stage(va, true);
-        }
-      } else {
-        load_stage(0, va);
-        for (int ks = 0; ks < tl.kst && ok; ks += 2) {
-          if (ks + 1 < tl.kst) load_stage(ks + 1, vb);
-          ok = convert_stage(va, true);
-          if (!ok || ks + 1 >= tl.kst) break;
-          if (ks + 2 < tl.kst) load_stage(ks + 2, va);
-          ok = convert_stage(vb, true);
-        }
+      float va[BK / 16][8];
+      // Read the raw stage into registers and hand it back at once, then wait
+      // for the converted-operand slot.
+      for (int ks = 0; ks < tl.kst && ok; ++ks) {
+        ok = wait_bar(&pp.full_raw[rstage], rphase, pp, a.err, 8);
+        if (!ok) break;
+        fetch_raw(ks, va);
+        __syncwarp();  // the warp's reads of the raw stage are done
+        if ((threadIdx.x & 31) == 0) mbar_arrive(&pp.raw_empty[rstage]);
+        if (++rstage == S) { rstage = 0; rphase ^= 1; }
+        ok = convert_stage(va);
       }
       if (!ok) break;
     }
@@ -1345,15 +1298,13 @@ void launch_gemm_tc_groups(const TcGroupSpec* g, int ngroups, TcTileCache* cache
   }
   if (list.n == 0) return;
   TcArgs a{};
-  // All groups of a launch take the data by TMA, or none does (the loader
-  // and the converters then agree on which barriers a stage completes).
-  bool tma = true;
   {
     std::lock_guard<std::mutex> lock(cache->mu);
-    for (int gi = 0; gi < ngroups && tma; ++gi) {
+    for (int gi = 0; gi < ngroups; ++gi) {
       const sht_plan* p = g[gi].plan;
       const int64_t rows = g[gi].direction == 0 ? p->cf_rows : (int64_t)(p->T + 1) * 2 * p->H;
-      tma = data_map(cache, g[gi].data, g[gi].R, rows, &a.g[gi].data_map);
+      if (!data_map(cache, g[gi].data, g[gi].R, rows, &a.g[gi].data_map))
+        throw Error{SHT_ERR_STATE, "tensor-core launch: the data operand has no tensor map"};
     }
   }
   int rs_off = 0;
@@ -1361,10 +1312,8 @@ void launch_gemm_tc_groups(const TcGroupSpec* g, int ngroups, TcTileCache* cache
     const sht_plan* p = g[gi].plan;
     const ShtTc16* tc = p->tc;
     TcGroup& G = a.g[gi];
-    G.use_tma = tma ? 1 : 0;
     G.img = (const unsigned char*)tc->img[g[gi].table_kind];
     G.colscale = tc->colscale[g[gi].table_kind];
-    G.data = g[gi].data;
     G.rowmax = g[gi].rowmax;
     G.out = g[gi].out;
     G.R = g[gi].R;

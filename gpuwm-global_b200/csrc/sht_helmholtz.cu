@@ -135,7 +135,7 @@ __device__ __forceinline__ void half_map_scalars(double omega, double dt, double
 struct SemiArgs {
   int Tn, nlev, mode;
   double radius, dt, alpha;
-  int64_t cf_planes;  // Cfold column count (the levels), when cfold is set
+  int64_t cf_planes;  // Cfold column stride, when cfold is set
 };
 
 // Shared-memory plan of one mode (element counts in T).
@@ -470,8 +470,8 @@ __global__ void __launch_bounds__(256) semi_implicit_kernel(
 template <typename T>
 void launch_semi_implicit(const sht_plan* p, int nlev, const T* mats, bool has_thermo, int mode,
                           double dt, double alpha, const T* div, const T* theta, const T* lnps,
-                          T* odiv, T* otheta, T* olnps, T* metric, T* cfold, float* rowmax,
-                          cudaStream_t s) {
+                          T* odiv, T* otheta, T* olnps, T* metric, T* cfold, int64_t ldc,
+                          float* rowmax, cudaStream_t s) {
   SHT_REQUIRE(nlev >= 1 && nlev <= kMaxLev, "nlev must be in [1, 96]");
   SHT_REQUIRE(mode == kSemiSolve || mode == kSemiApply || mode == kSemiHalf ||
                   mode == kSemiLinear,
@@ -490,7 +490,7 @@ void launch_semi_implicit(const sht_plan* p, int nlev, const T* mats, bool has_t
   SHT_CUDA_OR_THROW(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const int64_t items = div_up(p->T + 1, 32) * (int64_t)(p->T + 1);
   const int ctas = (int)std::min<int64_t>(items, (int64_t)per_sm * sms);
-  SemiArgs a{p->T, nlev, mode, p->radius, dt, alpha, (int64_t)nlev};
+  SemiArgs a{p->T, nlev, mode, p->radius, dt, alpha, ldc};
   semi_implicit_kernel<T><<<ctas, dim3(32, 8), sm, s>>>(
       a, mats, (const V2<T>*)div, (const V2<T>*)theta, (const V2<T>*)lnps, (V2<T>*)odiv,
       (V2<T>*)otheta, (V2<T>*)olnps, metric, (V2<T>*)cfold, rowmax);
@@ -502,13 +502,13 @@ void launch_helmholtz(const sht_plan* p, int nlev, const T* mats, double tau_w, 
                       const T* theta, const T* lnps, T* odiv, T* otheta, T* olnps,
                       cudaStream_t s) {
   launch_semi_implicit<T>(p, nlev, mats, false, kSemiSolve, tau_w, 1.0, div, theta, lnps, odiv,
-                          otheta, olnps, nullptr, nullptr, nullptr, s);
+                          otheta, olnps, nullptr, nullptr, 0, nullptr, s);
 }
 
 #define INST(T)                                                                               \
   template void launch_semi_implicit<T>(const sht_plan*, int, const T*, bool, int, double,   \
                                         double, const T*, const T*, const T*, T*, T*, T*, T*, \
-                                        T*, float*, cudaStream_t);                            \
+                                        T*, int64_t, float*, cudaStream_t);                            \
   template void launch_helmholtz<T>(const sht_plan*, int, const T*, double, const T*,        \
                                     const T*, const T*, T*, T*, T*, cudaStream_t);
 INST(float)

@@ -35,7 +35,7 @@ template <typename T, bool INVLAP>
 __global__ void __launch_bounds__(256) pack_kernel(int Tn, double radius,
                                                    const V2<T>* __restrict__ c0,
                                                    const V2<T>* __restrict__ c1, int64_t planes,
-                                                   int F, V2<T>* __restrict__ cf,
+                                                   int64_t Rc, int F, V2<T>* __restrict__ cf,
                                                    float* __restrict__ rowmax) {
   constexpr int NB = PackCfg<T>::NB;
   __shared__ V2<T> tile[NB][32][33];
@@ -67,7 +67,6 @@ __global__ void __launch_bounds__(256) pack_kernel(int Tn, double radius,
       for (int k = 0; k < 4; ++k) tile[nb][ty + 8 * k][tx] = v[nb][k];
   }
   __syncthreads();
-  const int64_t Rc = planes * F;
   const int64_t p = p0 + tx;
   float mre = 0.f, mim = 0.f;
   if (p < planes) {
@@ -124,7 +123,7 @@ template <typename T, int MODE> struct UnpackCfg {
 template <typename T, int MODE>
 __global__ void __launch_bounds__(256) unpack_kernel(int Tn, const V2<T>* __restrict__ cf0,
                                                      const V2<T>* __restrict__ cf1, int64_t planes,
-                                                     V2<T>* __restrict__ o0, V2<T>* __restrict__ o1) {
+                                                     int64_t Rc, V2<T>* __restrict__ o0, V2<T>* __restrict__ o1) {
   constexpr int NB = UnpackCfg<T, MODE>::NB, NO = UnpackCfg<T, MODE>::NO;
   __shared__ V2<T> tile[NO][NB][32][33];
   const int m0 = blockIdx.x * 32;
@@ -150,7 +149,6 @@ __global__ void __launch_bounds__(256) unpack_kernel(int Tn, const V2<T>* __rest
     }
     return;
   }
-  const int64_t Rc = planes * NO;
   const int64_t p = p0 + tx;
   {
     V2<T> va[NB][4], vb[NB][4];
@@ -241,7 +239,7 @@ __global__ void elementwise_kernel(int Tn, double radius, int mode, const V2<T>*
 }  // namespace
 
 template <typename T>
-void launch_pack(const sht_plan* p, const T* coeff0, const T* coeff1, int64_t planes, int mode,
+void launch_pack(const sht_plan* p, const T* coeff0, const T* coeff1, int64_t planes, int64_t ldc, int mode,
                  T* cfold, cudaStream_t s, float* rowmax) {
   if (planes == 0) return;
   int F = coeff1 ? 2 : 1;
@@ -250,36 +248,36 @@ void launch_pack(const sht_plan* p, const T* coeff0, const T* coeff1, int64_t pl
   SHT_REQUIRE(grid.z <= 65535, "too many planes for one pack launch");
   if (mode == kPackInvLap)
     pack_kernel<T, true><<<grid, dim3(32, 8), 0, s>>>(p->T, p->radius, (const V2<T>*)coeff0,
-                                                      (const V2<T>*)coeff1, planes, F,
+                                                      (const V2<T>*)coeff1, planes, ldc, F,
                                                       (V2<T>*)cfold, rowmax);
   else
     pack_kernel<T, false><<<grid, dim3(32, 8), 0, s>>>(p->T, p->radius, (const V2<T>*)coeff0,
-                                                       (const V2<T>*)coeff1, planes, F,
+                                                       (const V2<T>*)coeff1, planes, ldc, F,
                                                        (V2<T>*)cfold, rowmax);
   SHT_CUDA_OR_THROW(cudaGetLastError());
 }
 
 template <typename T, int MODE>
-void launch_unpack_mode(const sht_plan* p, const T* cf0, const T* cf1, int64_t planes, T* out0,
-                        T* out1, cudaStream_t s) {
+void launch_unpack_mode(const sht_plan* p, const T* cf0, const T* cf1, int64_t planes,
+                        int64_t ldc, T* out0, T* out1, cudaStream_t s) {
   dim3 grid((unsigned)div_up(p->T + 1, 32), (unsigned)div_up(p->T + 1, UnpackCfg<T, MODE>::NB),
             (unsigned)div_up(planes, 32));
   SHT_REQUIRE(grid.z <= 65535, "too many planes for one unpack launch");
   unpack_kernel<T, MODE><<<grid, dim3(32, 8), 0, s>>>(p->T, (const V2<T>*)cf0, (const V2<T>*)cf1,
-                                                      planes, (V2<T>*)out0, (V2<T>*)out1);
+                                                      planes, ldc, (V2<T>*)out0, (V2<T>*)out1);
   SHT_CUDA_OR_THROW(cudaGetLastError());
 }
 
 template <typename T>
 void launch_unpack(const sht_plan* p, int mode, const T* cf0, const T* cf1, int64_t planes,
-                   T* out0, T* out1, cudaStream_t s) {
+                   int64_t ldc, T* out0, T* out1, cudaStream_t s) {
   if (planes == 0) return;
   if (mode == kUnpackVorDiv)
-    launch_unpack_mode<T, kUnpackVorDiv>(p, cf0, cf1, planes, out0, out1, s);
+    launch_unpack_mode<T, kUnpackVorDiv>(p, cf0, cf1, planes, ldc, out0, out1, s);
   else if (mode == kUnpackDiv)
-    launch_unpack_mode<T, kUnpackDiv>(p, cf0, cf1, planes, out0, out1, s);
+    launch_unpack_mode<T, kUnpackDiv>(p, cf0, cf1, planes, ldc, out0, out1, s);
   else
-    launch_unpack_mode<T, kUnpackScalar>(p, cf0, cf1, planes, out0, out1, s);
+    launch_unpack_mode<T, kUnpackScalar>(p, cf0, cf1, planes, ldc, out0, out1, s);
 }
 
 template <typename T>
@@ -294,9 +292,9 @@ void launch_elementwise(const sht_plan* p, int mode, const T* in, int64_t planes
 }
 
 #define INST(T)                                                                                  \
-  template void launch_pack<T>(const sht_plan*, const T*, const T*, int64_t, int, T*,          \
+  template void launch_pack<T>(const sht_plan*, const T*, const T*, int64_t, int64_t, int, T*,          \
                                cudaStream_t, float*);                                           \
-  template void launch_unpack<T>(const sht_plan*, int, const T*, const T*, int64_t, T*, T*,    \
+  template void launch_unpack<T>(const sht_plan*, int, const T*, const T*, int64_t, int64_t, T*, T*,    \
                                  cudaStream_t);                                                 \
   template void launch_elementwise<T>(const sht_plan*, int, const T*, int64_t, T*, cudaStream_t);
 INST(float)

@@ -119,6 +119,15 @@ struct sht_plan {
 
 namespace sht {
 
+// The scratch operands (wfold, cfold) hold one complex column per (plane,
+// field), columns innermost; `ldc` is their column stride.  The plan's own
+// scratch pads an odd count by one column (which nothing reads as a result),
+// so every row starts on a 16-byte boundary and every kernel takes its aligned
+// path: at T255 x 161 planes in FP32 the inverse FFT took 154 us on the odd
+// stride, with a kernel of its own, and takes 100 us; the FP32 contractions 413
+// us with 8-byte copies and 351 us; the tensor-core one could not use TMA.
+inline int64_t padded_cols(int64_t cols) { return (cols + 1) & ~int64_t(1); }
+
 // Geometry and tables (sht_geometry.cu).
 void build_geometry_and_tables(sht_plan* p, cudaStream_t s);
 
@@ -129,22 +138,22 @@ void build_fft(sht_plan* p, cudaStream_t s);
 // float bits (the row scales of the split-precision contraction).
 template <typename T>
 void launch_forward_fold(const sht_plan* p, const T* g0, const T* g1, int64_t planes,
-                         T* wfold, cudaStream_t s, float* rowmax = nullptr);
+                         int64_t ldc, T* wfold, cudaStream_t s, float* rowmax = nullptr);
 // Inverse modes.
 enum UnfoldMode { kUnfoldScalar = 0, kUnfoldZonal = 1, kUnfoldGradient = 2, kUnfoldWind = 3,
                   kUnfoldMeridional = 4 };
 template <typename T>
 void launch_inverse_unfold(const sht_plan* p, int mode, const T* wP, const T* wD,
-                           int64_t planes, T* out0, T* out1, cudaStream_t s);
+                           int64_t planes, int64_t ldc, T* out0, T* out1, cudaStream_t s);
 
 // Register-resident FP32 FFTs for nlon = 64 F, F in {2,3,4,6,8,12,16,24}
 // (sht_fft_fast.cu).
 bool fast_fft_supported(const sht_plan* p);
 void fast_fft_init_constants(cudaStream_t s);
 void fast_forward_fold(const sht_plan* p, const float* g0, const float* g1, int64_t planes,
-                       float* wfold, cudaStream_t s, float* rowmax = nullptr);
+                       int64_t ldc, float* wfold, cudaStream_t s, float* rowmax = nullptr);
 void fast_inverse_unfold(const sht_plan* p, int mode, const float* wP, const float* wD,
-                         int64_t planes, float* out0, float* out1, cudaStream_t s);
+                         int64_t planes, int64_t ldc, float* out0, float* out1, cudaStream_t s);
 
 // SIMT Legendre GEMM (sht_gemm_simt.cu).
 void build_gemm_items(sht_plan* p);
@@ -161,7 +170,7 @@ void launch_gemm_simt_groups(const sht_plan* p, int direction, int ngroups, cons
 enum PackMode { kPackPlain = 0, kPackInvLap = 1 };
 template <typename T>
 void launch_pack(const sht_plan* p, const T* coeff0, const T* coeff1, int64_t planes,
-                 int mode, T* cfold, cudaStream_t s, float* rowmax = nullptr);
+                 int64_t ldc, int mode, T* cfold, cudaStream_t s, float* rowmax = nullptr);
 
 // Warp-level merge of per-thread row maxima: lanes with equal lane % nper
 // hold the same column (complex index col); lanes < nper publish.
@@ -182,7 +191,7 @@ __device__ __forceinline__ void rowmax_merge(float* rowmax, int64_t col, bool va
 enum UnpackMode { kUnpackScalar = 0, kUnpackVorDiv = 1, kUnpackDiv = 2 };
 template <typename T>
 void launch_unpack(const sht_plan* p, int mode, const T* cf0, const T* cf1, int64_t planes,
-                   T* out0, T* out1, cudaStream_t s);
+                   int64_t ldc, T* out0, T* out1, cudaStream_t s);
 enum ElemMode { kElemProject = 0, kElemLaplacian = 1, kElemInvLaplacian = 2 };
 template <typename T>
 void launch_elementwise(const sht_plan* p, int mode, const T* in, int64_t planes, T* out,
@@ -194,8 +203,8 @@ enum SemiMode { kSemiSolve = 0, kSemiApply = 1, kSemiHalf = 2, kSemiLinear = 3 }
 template <typename T>
 void launch_semi_implicit(const sht_plan* p, int nlev, const T* mats, bool has_thermo, int mode,
                           double dt, double alpha, const T* div, const T* theta, const T* lnps,
-                          T* odiv, T* otheta, T* olnps, T* metric, T* cfold, float* rowmax,
-                          cudaStream_t s);
+                          T* odiv, T* otheta, T* olnps, T* metric, T* cfold, int64_t ldc,
+                          float* rowmax, cudaStream_t s);
 template <typename T>
 void launch_helmholtz(const sht_plan* p, int nlev, const T* mats, double tau_w,
                       const T* div, const T* theta, const T* lnps, T* odiv, T* otheta,
@@ -203,10 +212,10 @@ void launch_helmholtz(const sht_plan* p, int nlev, const T* mats, double tau_w,
 
 // Reference-layout Fourier waist <-> folded waist (sht_waist.cu).
 template <typename T>
-void launch_waist_export(const sht_plan* p, const T* wfold, int64_t planes, double c, int zonal,
+void launch_waist_export(const sht_plan* p, const T* wfold, int64_t planes, int64_t ldc, double c, int zonal,
                          T* waist, cudaStream_t s);
 template <typename T>
-void launch_waist_import(const sht_plan* p, const T* waist, int64_t planes, double c, T* wfold,
+void launch_waist_import(const sht_plan* p, const T* waist, int64_t planes, int64_t ldc, double c, T* wfold,
                          float* rowmax, cudaStream_t s, int fields = 1);
 
 // Split-precision tensor-core path (sht_gemm_tc.cu).

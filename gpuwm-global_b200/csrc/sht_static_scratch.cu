@@ -53,9 +53,9 @@ void forward_static(sht_plan* p, const T* grid, int64_t planes, T* coeff, void* 
   T* w = static_cast<T*>(base);
   const int64_t w_bytes = sht::round_up((int64_t)sizeof(T) * p->wfold_elems(R), 256);
   T* c = reinterpret_cast<T*>(static_cast<unsigned char*>(base) + w_bytes);
-  sht::launch_forward_fold<T>(p, grid, nullptr, planes, w, s);
+  sht::launch_forward_fold<T>(p, grid, nullptr, planes, planes, w, s);
   sht::launch_gemm_simt<T>(p, 1, 0, static_cast<const T*>(p->analysis), w, c, R, s);
-  sht::launch_unpack<T>(p, sht::kUnpackScalar, c, nullptr, planes, coeff, nullptr, s);
+  sht::launch_unpack<T>(p, sht::kUnpackScalar, c, nullptr, planes, planes, coeff, nullptr, s);
 }
 
 }  // namespace

@@ -29,7 +29,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) waist_export_kernel(int Tn, int H, int nlat, int nlat_odd,
                                                            double c, int zonal,
                                                            const V2<T>* __restrict__ wf,
-                                                           int64_t planes, V2<T>* __restrict__ out) {
+                                                           int64_t planes, int64_t ldc, V2<T>* __restrict__ out) {
   __shared__ V2<T> tile[2][32][33];  // [side][plane][order]
   const int m0 = blockIdx.x * 32;
   const int h = blockIdx.y;
@@ -43,8 +43,8 @@ __global__ void __launch_bounds__(256) waist_export_kernel(int Tn, int H, int nl
     const int64_t p = p0 + tx;
     V2<T> a = mk2<T>(T(0), T(0)), b = a;
     if (m < t1 && p < planes) {
-      const V2<T> S = wf[((int64_t)(m * 2 + 0) * H + h) * planes + p];
-      const V2<T> D = wf[((int64_t)(m * 2 + 1) * H + h) * planes + p];
+      const V2<T> S = wf[((int64_t)(m * 2 + 0) * H + h) * ldc + p];
+      const V2<T> D = wf[((int64_t)(m * 2 + 1) * H + h) * ldc + p];
       if (eq) {
         a = S;
       } else {
@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(256) waist_export_kernel(int Tn, int H, int nl
 template <typename T>
 __global__ void __launch_bounds__(256) waist_import_kernel(int Tn, int H, int nlat, int nlat_odd,
                                                            double c, const V2<T>* __restrict__ in,
-                                                           int64_t planes, int fields,
+                                                           int64_t planes, int64_t ldc, int fields,
                                                            V2<T>* __restrict__ wf,
                                                            float* __restrict__ rowmax) {
   __shared__ V2<T> tile[2][32][33];  // [S/D][plane][order]
@@ -115,8 +115,8 @@ __global__ void __launch_bounds__(256) waist_import_kernel(int Tn, int H, int nl
     const int m = m0 + mm;
     if (m >= t1 || p >= planes) continue;
     const V2<T> S = tile[0][tx][mm], D = tile[1][tx][mm];
-    wf[((int64_t)(m * 2 + 0) * H + h) * planes + col] = S;
-    wf[((int64_t)(m * 2 + 1) * H + h) * planes + col] = D;
+    wf[((int64_t)(m * 2 + 0) * H + h) * ldc + col] = S;
+    wf[((int64_t)(m * 2 + 1) * H + h) * ldc + col] = D;
     mre = fmaxf(mre, fmaxf((float)fabs(S.x), (float)fabs(D.x)));
     mim = fmaxf(mim, fmaxf((float)fabs(S.y), (float)fabs(D.y)));
   }
@@ -139,34 +139,34 @@ __global__ void __launch_bounds__(256) waist_import_kernel(int Tn, int H, int nl
 }  // namespace
 
 template <typename T>
-void launch_waist_export(const sht_plan* p, const T* wfold, int64_t planes, double c, int zonal,
+void launch_waist_export(const sht_plan* p, const T* wfold, int64_t planes, int64_t ldc, double c, int zonal,
                          T* waist, cudaStream_t s) {
   if (planes == 0) return;
   dim3 grid((unsigned)div_up(p->T + 1, 32), (unsigned)p->H, (unsigned)div_up(planes, 32));
   SHT_REQUIRE(grid.z <= 65535, "too many planes for one waist launch");
   waist_export_kernel<T><<<grid, dim3(32, 8), 0, s>>>(p->T, p->H, p->nlat, p->nlat_odd ? 1 : 0, c,
-                                                      zonal, (const V2<T>*)wfold, planes,
+                                                      zonal, (const V2<T>*)wfold, planes, ldc,
                                                       (V2<T>*)waist);
   SHT_CUDA_OR_THROW(cudaGetLastError());
 }
 
 template <typename T>
-void launch_waist_import(const sht_plan* p, const T* waist, int64_t planes, double c, T* wfold,
+void launch_waist_import(const sht_plan* p, const T* waist, int64_t planes, int64_t ldc, double c, T* wfold,
                          float* rowmax, cudaStream_t s, int fields) {
   if (planes == 0) return;
   SHT_REQUIRE(fields >= 1 && planes % fields == 0, "waist import: planes not a multiple of fields");
   dim3 grid((unsigned)div_up(p->T + 1, 32), (unsigned)p->H, (unsigned)div_up(planes, 32));
   SHT_REQUIRE(grid.z <= 65535, "too many planes for one waist launch");
   waist_import_kernel<T><<<grid, dim3(32, 8), 0, s>>>(p->T, p->H, p->nlat, p->nlat_odd ? 1 : 0, c,
-                                                      (const V2<T>*)waist, planes, fields,
+                                                      (const V2<T>*)waist, planes, ldc, fields,
                                                       (V2<T>*)wfold, rowmax);
   SHT_CUDA_OR_THROW(cudaGetLastError());
 }
 
 #define INST(T)                                                                                  \
-  template void launch_waist_export<T>(const sht_plan*, const T*, int64_t, double, int, T*,     \
+  template void launch_waist_export<T>(const sht_plan*, const T*, int64_t, int64_t, double, int, T*,     \
                                        cudaStream_t);                                           \
-  template void launch_waist_import<T>(const sht_plan*, const T*, int64_t, double, T*, float*,  \
+  template void launch_waist_import<T>(const sht_plan*, const T*, int64_t, int64_t, double, T*, float*,  \
                                        cudaStream_t, int);
 INST(float)
 INST(double)
