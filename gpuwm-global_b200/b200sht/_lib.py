@@ -113,6 +113,9 @@ SIGNATURES = {
                                           ctypes.POINTER(ctypes.c_int), _DP]),
     "sht_sl_gather": (ctypes.c_int, [_P, ctypes.c_int, ctypes.c_int, ctypes.c_int, _P, _I64,
                                      ctypes.c_int, _P, _P, _P, _P, _P, _P]),
+    "sht_sl_gather_fields": (ctypes.c_int, [_P, _P, ctypes.c_int, ctypes.c_int, ctypes.c_int,
+                                            ctypes.POINTER(_P), _I64, _P, ctypes.c_int, _P, _P,
+                                            _P, _P, _P, _P]),
     "sht_sl_gather_linear": (ctypes.c_int, [_P, _P, _I64, ctypes.c_int, _P, _P, _P, _P, _P]),
     "sht_sl_departure": (ctypes.c_int, [_P, ctypes.c_int, _P, _P, _P, _P, _P, _P, _P, _P,
                                         ctypes.c_int, _D, _D, _P, _P, _P, _P, _P, _P]),

@@ -354,17 +354,20 @@ def gather_batch(fields: Sequence[torch.Tensor], stencil: Stencil, *, monotone: 
         window.clear_escape()
     out: list = []
     for start in range(0, len(fields), int(batch)):
-        chunk = fields[start:start + int(batch)]
-        src = _source_block(chunk)
+        chunk = [f.contiguous() for f in fields[start:start + int(batch)]]
         count = len(chunk)
-        dst = torch.empty((count, *stencil.shape), dtype=src.dtype, device=src.device)
+        dst = torch.empty((count, *stencil.shape), dtype=chunk[0].dtype, device=chunk[0].device)
         cut = torch.empty_like(dst) if deficit else None
-        name, handle = (("sht_sl_gather", stencil.tables._handle) if window is None
-                        else ("sht_sl_gather_band", window._handle))
-        _lib.call(name, handle, order, lim, 1 if deficit else 0,
-                  _ptr(src), count, nlev, _ptr(stencil.xi), _ptr(stencil.phi),
-                  _ptr(stencil.level), _ptr(dst), _ptr(cut) if cut is not None else None,
-                  _stream())
+        # room for the fields interleaved (a single one is read in place)
+        packed = (torch.empty((count, *stencil.source_shape), dtype=dst.dtype, device=dst.device)
+                  if count > 1 else None)
+        ptrs = (ctypes.c_void_p * count)(*[f.data_ptr() for f in chunk])
+        tables = stencil.tables if window is None else window.tables
+        _lib.call("sht_sl_gather_fields", tables._handle,
+                  None if window is None else window._handle, order, lim, 1 if deficit else 0,
+                  ptrs, count, _ptr(packed) if packed is not None else None, nlev,
+                  _ptr(stencil.xi), _ptr(stencil.phi), _ptr(stencil.level), _ptr(dst),
+                  _ptr(cut) if cut is not None else None, _stream())
         if deficit:
             out.extend((dst[i], cut[i]) for i in range(count))
         else:

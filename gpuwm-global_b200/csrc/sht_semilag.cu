@@ -199,20 +199,108 @@ __device__ __forceinline__ int held_row(const int32_t* __restrict__ rowoff, int 
 }
 
 // --------------------------------------------------------------- gather
-template <typename T, int NH, bool QM, bool DEF>
-__global__ void __launch_bounds__(256, (sizeof(T) == 4 && NH == 4) ? 3 : 2) sl_gather_kernel(const SlArgs<T> a) {
+// VEC fields of one point side by side (16 bytes for four floats or two
+// doubles), so one tap load brings VEC fields.
+template <typename T, int VEC> struct alignas(sizeof(T) * VEC) Pack { T v[VEC]; };
+template <typename T, int VEC>
+__device__ __forceinline__ Pack<T, VEC> load_pack(const Pack<T, VEC>* p) {
+  Pack<T, VEC> r;
+  if constexpr (sizeof(r) == 16) {
+    const int4 q = __ldg(reinterpret_cast<const int4*>(p));
+    *reinterpret_cast<int4*>(&r) = q;
+  } else if constexpr (sizeof(r) == 8) {
+    const int2 q = __ldg(reinterpret_cast<const int2*>(p));
+    *reinterpret_cast<int2*>(&r) = q;
+  } else {
+    r.v[0] = __ldg(&p->v[0]);
+  }
+  return r;
+}
+// a - b, w a and c + w a (fused); floats in packed pairs.
+template <typename T, int VEC>
+__device__ __forceinline__ Pack<T, VEC> pk_sub(const Pack<T, VEC>& a, const Pack<T, VEC>& b) {
+  Pack<T, VEC> r;
+  if constexpr (sizeof(T) == 4 && VEC % 2 == 0) {
+#pragma unroll
+    for (int e = 0; e < VEC; e += 2) {
+      const float2 d = __fadd2_rn(make_float2(a.v[e], a.v[e + 1]), make_float2(-b.v[e], -b.v[e + 1]));
+      r.v[e] = d.x;
+      r.v[e + 1] = d.y;
+    }
+  } else {
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) r.v[e] = a.v[e] - b.v[e];
+  }
+  return r;
+}
+template <typename T, int VEC>
+__device__ __forceinline__ Pack<T, VEC> pk_mul(T w, const Pack<T, VEC>& a) {
+  Pack<T, VEC> r;
+  if constexpr (sizeof(T) == 4 && VEC % 2 == 0) {
+#pragma unroll
+    for (int e = 0; e < VEC; e += 2) {
+      const float2 d = __fmul2_rn(make_float2(w, w), make_float2(a.v[e], a.v[e + 1]));
+      r.v[e] = d.x;
+      r.v[e + 1] = d.y;
+    }
+  } else {
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) r.v[e] = w * a.v[e];
+  }
+  return r;
+}
+template <typename T, int VEC>
+__device__ __forceinline__ void pk_fma(T w, const Pack<T, VEC>& a, Pack<T, VEC>& c) {
+  if constexpr (sizeof(T) == 4 && VEC % 2 == 0) {
+#pragma unroll
+    for (int e = 0; e < VEC; e += 2) {
+      const float2 d = __ffma2_rn(make_float2(w, w), make_float2(a.v[e], a.v[e + 1]),
+                                  make_float2(c.v[e], c.v[e + 1]));
+      c.v[e] = d.x;
+      c.v[e + 1] = d.y;
+    }
+  } else {
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) c.v[e] = fma(w, a.v[e], c.v[e]);
+  }
+}
+
+// Interleaves fields into groups of VEC: out[g][point] = (f[g VEC], ...).
+constexpr int kPackFields = 16;
+struct PackArgs { const void* f[kPackFields]; };
+template <typename T, int VEC>
+__global__ void __launch_bounds__(256) sl_pack_kernel(const __grid_constant__ PackArgs a, int64_t n,
+                                                      Pack<T, VEC>* __restrict__ out) {
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  Pack<T, VEC> r;
+#pragma unroll
+  for (int e = 0; e < VEC; ++e) r.v[e] = __ldcs(static_cast<const T*>(a.f[blockIdx.y * VEC + e]) + t);
+  out[blockIdx.y * n + t] = r;
+}
+
+// A CTA takes 32 columns x 4 levels x 2 rows of arrival points: the taps of
+// its 256 points fall in about 36 x 7 x 6 source points, which stay in L1 (a
+// CTA of 256 columns of one level reads 260 x 4 x 4).  Four floats per tap
+// load (fields interleaved by sl_pack_kernel, which takes the place of the
+// copy that put the batch's fields in one block) cut the load instructions by
+// four and the half-used lines of misaligned 128-byte warp loads; the
+// interpolation arithmetic runs on packed pairs.  Sixteen FP32 fields with the
+// limiter at T511 L40: 16.2 ms one float per load, 9.9 ms four (19.6 TB/s of
+// taps; the bound is the L1's 128 bytes a clock, 5.4 ms), and 0.98 ms to
+// interleave against 0.89 ms for the copy.
+template <typename T, int NH, int VEC, bool QM, bool DEF>
+__global__ void __launch_bounds__(256, (sizeof(T) == 4 && VEC <= 2 && NH == 4) ? 3 : 2)
+    sl_gather_kernel(const SlArgs<T> a) {
+  using P = Pack<T, VEC>;
   constexpr int G = NH / 2 - 1;  // zonal lead and meridional start offset
   constexpr int MID = NH / 2 - 1;
   const int plane = a.njs * a.ni;              // a held source level
   const int64_t n = (int64_t)a.nk * a.nja * a.ni;  // arrival points
-  // Threads walk the points row by row with the levels of a row together:
-  // a source level plane is read by the stencils of four arrival levels,
-  // which then run at the same time and find it in L2 (level-major order
-  // brought every plane in from DRAM about four times).
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  const int64_t gid = point_index(t, a.nk, a.nja, a.ni);
-
+  const int ia = blockIdx.x * 32 + threadIdx.x;
+  const int ka = blockIdx.y * 4 + threadIdx.y, ja = blockIdx.z * 2 + threadIdx.z;
+  if (ia >= a.ni || ka >= a.nk || ja >= a.nja) return;
+  const int64_t gid = ((int64_t)ka * a.nja + ja) * a.ni + ia;
   const T p = min(max(a.phi[gid], T(-kHalfPi)), T(kHalfPi));
   const T xk = min(max(a.lev[gid], T(-0.5)), T(a.nk) - T(0.5));
   const bool below = xk < T(0);
@@ -286,21 +374,23 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 && NH == 4) ? 3 : 2) sl_g
       if (m == cy && q == cx) centre = adr[m][q];
 
   const int64_t fstride = n;                          // output field stride
-  const int64_t sstride = (int64_t)a.nk * plane;       // source field stride
+  const int64_t sstride = (int64_t)a.nk * plane;       // source field (or group) stride
   const int64_t cofs = (int64_t)kn * plane + centre;
-  // NB fields per pass share every address; their taps are in flight
+  // NB groups per pass share every address; their taps are in flight
   // together, two levels at a time (a fully unrolled level loop holds every
   // level's loads and weights at once, 180+ registers; one level at a time
   // measured 4-14 % slower).
   auto fields = [&](auto nb_tag, int f0) {
     constexpr int NB = decltype(nb_tag)::value;
-    const T* s[NB];
-    T base[NB], acc[NB], lo[NB], hi[NB], f_edge[NB], f_next[NB];
+    const P* s[NB];
+    P base[NB], acc[NB], lo[NB], hi[NB], f_edge[NB], f_next[NB];
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
-      s[b] = a.src + (f0 + b) * sstride;
-      base[b] = __ldg(s[b] + cofs);
-      acc[b] = lo[b] = hi[b] = f_edge[b] = f_next[b] = T(0);
+      s[b] = reinterpret_cast<const P*>(a.src) + (f0 + b) * sstride;
+      base[b] = load_pack<T, VEC>(s[b] + cofs);
+#pragma unroll
+      for (int e = 0; e < VEC; ++e)
+        acc[b].v[e] = lo[b].v[e] = hi[b].v[e] = f_edge[b].v[e] = f_next[b].v[e] = T(0);
     }
     bool boxed = false;
 #pragma unroll 2
@@ -308,56 +398,68 @@ __global__ void __launch_bounds__(256, (sizeof(T) == 4 && NH == 4) ? 3 : 2) sl_g
       const int64_t lofs = (int64_t)(k0 + c) * plane;
       const T wzc = c == 0 ? wz[0] : (c == 1 ? wz[1] : (c == 2 ? wz[2] : wz[3]));
       const bool inbox = QM && (c == kbox || c == kbox + 1);
-      T rowsum[NB];
+      P rowsum[NB];
 #pragma unroll
-      for (int b = 0; b < NB; ++b) rowsum[b] = T(0);
+      for (int b = 0; b < NB; ++b)
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) rowsum[b].v[e] = T(0);
 #pragma unroll
       for (int m = 0; m < NH; ++m) {
-        T v[NB][NH];
+        P v[NB][NH];
 #pragma unroll
         for (int b = 0; b < NB; ++b)
 #pragma unroll
-          for (int q = 0; q < NH; ++q) v[b][q] = __ldg(s[b] + lofs + adr[m][q]);
+          for (int q = 0; q < NH; ++q) v[b][q] = load_pack<T, VEC>(s[b] + lofs + adr[m][q]);
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
           if (inbox && (m == MID || m == MID + 1)) {
-            const T vmin = min(v[b][MID], v[b][MID + 1]), vmax = max(v[b][MID], v[b][MID + 1]);
-            lo[b] = boxed ? min(lo[b], vmin) : vmin;
-            hi[b] = boxed ? max(hi[b], vmax) : vmax;
-          }
-          T colsum = wx[0] * (v[b][0] - base[b]);
 #pragma unroll
-          for (int q = 1; q < NH; ++q) colsum += wx[q] * (v[b][q] - base[b]);
-          rowsum[b] += wy[m] * colsum;
+            for (int e = 0; e < VEC; ++e) {
+              const T x = v[b][MID].v[e], y = v[b][MID + 1].v[e];
+              const T vmin = min(x, y), vmax = max(x, y);
+              lo[b].v[e] = boxed ? min(lo[b].v[e], vmin) : vmin;
+              hi[b].v[e] = boxed ? max(hi[b].v[e], vmax) : vmax;
+            }
+          }
+          P colsum = pk_mul<T, VEC>(wx[0], pk_sub<T, VEC>(v[b][0], base[b]));
+#pragma unroll
+          for (int q = 1; q < NH; ++q) pk_fma<T, VEC>(wx[q], pk_sub<T, VEC>(v[b][q], base[b]), colsum);
+          pk_fma<T, VEC>(wy[m], colsum, rowsum[b]);
         }
         if (inbox && (m == MID || m == MID + 1)) boxed = true;
       }
 #pragma unroll
       for (int b = 0; b < NB; ++b) {
-        acc[b] += wzc * rowsum[b];
+        pk_fma<T, VEC>(wzc, rowsum[b], acc[b]);
         if (c == c_edge) f_edge[b] = rowsum[b];
         if (c == c_next) f_next[b] = rowsum[b];
       }
     }
 #pragma unroll
-    for (int b = 0; b < NB; ++b) {
-      T r = acc[b];
-      if (!QM && outside) {
-        const T f_face = f_edge[b] + T(0.5) * (f_edge[b] - f_next[b]);
-        r = min(max(r, min(f_edge[b], f_face)), max(f_edge[b], f_face));
+    for (int b = 0; b < NB; ++b)
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) {
+        T r = acc[b].v[e];
+        if (!QM && outside) {
+          const T fe = f_edge[b].v[e];
+          const T f_face = fe + T(0.5) * (fe - f_next[b].v[e]);
+          r = min(max(r, min(fe, f_face)), max(fe, f_face));
+        }
+        r += base[b].v[e];
+        const T kept = QM ? min(max(r, lo[b].v[e]), hi[b].v[e]) : r;
+        const int64_t o = ((f0 + b) * (int64_t)VEC + e) * fstride + gid;
+        a.out[o] = kept;
+        if (DEF) a.cut[o] = r - kept;
       }
-      r += base[b];
-      const T kept = QM ? min(max(r, lo[b]), hi[b]) : r;
-      a.out[(f0 + b) * fstride + gid] = kept;
-      if (DEF) a.cut[(f0 + b) * fstride + gid] = r - kept;
-    }
   };
-  // Two fields per pass on the four-point stencil; the six-point one
-  // takes one (two would hold 190+ registers).
-  constexpr int NB = NH == 4 ? 2 : 1;
+  // Two single fields per pass on the four-point stencil; a group of VEC, or
+  // a field on the six-point stencil, by itself (two would hold 190+
+  // registers).
+  constexpr int NB = NH == 4 && VEC == 1 ? 2 : 1;
   int f = 0;
   for (; f + NB <= a.F; f += NB) fields(std::integral_constant<int, NB>{}, f);
-  if (f < a.F) fields(std::integral_constant<int, 1>{}, f);
+  if constexpr (NB > 1)
+    if (f < a.F) fields(std::integral_constant<int, 1>{}, f);
 }
 
 // ------------------------------------------------------------ trilinear
@@ -947,17 +1049,74 @@ SlArgs<T> make_args(const sht_sl_tables* t, const SlWidth& w, const void* src, i
   return a;
 }
 
-template <typename T, int NH>
+template <typename T, int NH, int VEC>
 void launch_gather(const SlArgs<T>& a, bool qm, bool def, cudaStream_t s) {
-  const int64_t n = (int64_t)a.nk * a.nja * a.ni;
-  const unsigned blocks = (unsigned)div_up(n, 256);
-  if (qm && def)
-    sl_gather_kernel<T, NH, true, true><<<blocks, 256, 0, s>>>(a);
-  else if (qm)
-    sl_gather_kernel<T, NH, true, false><<<blocks, 256, 0, s>>>(a);
-  else
-    sl_gather_kernel<T, NH, false, false><<<blocks, 256, 0, s>>>(a);
+  const dim3 block(32, 4, 2);
+  const dim3 grid((unsigned)div_up(a.ni, 32), (unsigned)div_up(a.nk, 4), (unsigned)div_up(a.nja, 2));
+  SHT_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "too many levels or rows for one gather launch");
+  if constexpr (NH == 6) {
+    if (qm) sl_gather_kernel<T, 6, VEC, true, false><<<grid, block, 0, s>>>(a);
+    else sl_gather_kernel<T, 6, VEC, false, false><<<grid, block, 0, s>>>(a);
+  } else {
+    if (def) sl_gather_kernel<T, 4, VEC, true, true><<<grid, block, 0, s>>>(a);
+    else if (qm) sl_gather_kernel<T, 4, VEC, true, false><<<grid, block, 0, s>>>(a);
+    else sl_gather_kernel<T, 4, VEC, false, false><<<grid, block, 0, s>>>(a);
+  }
   SHT_CUDA_OR_THROW(cudaGetLastError());
+}
+template <typename T, int VEC>
+void launch_gather_order(const SlArgs<T>& a, int order, bool qm, bool def, cudaStream_t s) {
+  if (order == 6) launch_gather<T, 6, VEC>(a, qm, def, s);
+  else launch_gather<T, 4, VEC>(a, qm, def, s);
+}
+
+// Interleaves `groups` groups of VEC fields into `packed` and gathers them
+// (field f's output at a.out + f * points).
+template <typename T, int VEC>
+void gather_groups(SlArgs<T> a, const void* const* fields, int groups, T* packed, int order,
+                   bool qm, bool def, cudaStream_t s) {
+  if (groups == 0) return;
+  const int64_t n = (int64_t)a.nk * a.njs * a.ni;
+  constexpr int kGroups = kPackFields / VEC;
+  for (int g0 = 0; g0 < groups; g0 += kGroups) {
+    const int ng = std::min(kGroups, groups - g0);
+    PackArgs pa{};
+    for (int e = 0; e < ng * VEC; ++e) pa.f[e] = fields[g0 * VEC + e];
+    sl_pack_kernel<T, VEC><<<dim3((unsigned)div_up(n, 256), (unsigned)ng), 256, 0, s>>>(
+        pa, n, reinterpret_cast<Pack<T, VEC>*>(packed) + g0 * n);
+    SHT_CUDA_OR_THROW(cudaGetLastError());
+  }
+  a.src = packed;
+  a.F = groups;
+  launch_gather_order<T, VEC>(a, order, qm, def, s);
+}
+
+// All fields of a call: groups of 16 bytes, then (FP32) one group of two, then
+// a single field read in place.
+template <typename T>
+void gather_fields(SlArgs<T> a, const void* const* fields, int count, T* packed, int order,
+                   bool qm, bool def, cudaStream_t s) {
+  constexpr int V = 16 / (int)sizeof(T);
+  const int64_t n_src = (int64_t)a.nk * a.njs * a.ni, n_out = (int64_t)a.nk * a.nja * a.ni;
+  T* const out = a.out;
+  T* const cut = a.cut;
+  int f = count / V * V;
+  gather_groups<T, V>(a, fields, count / V, packed, order, qm, def, s);
+  if constexpr (V == 4) {
+    if (count - f >= 2) {
+      a.out = out + f * n_out;
+      a.cut = cut ? cut + f * n_out : nullptr;
+      gather_groups<T, 2>(a, fields + f, 1, packed + f * n_src, order, qm, def, s);
+      f += 2;
+    }
+  }
+  if (f < count) {
+    a.out = out + f * n_out;
+    a.cut = cut ? cut + f * n_out : nullptr;
+    a.src = static_cast<const T*>(fields[f]);
+    a.F = 1;
+    launch_gather_order<T, 1>(a, order, qm, def, s);
+  }
 }
 
 void check_call(const sht_sl_tables* t, const void* src, int64_t fields, int nlev, const void* xi,
@@ -1068,11 +1227,16 @@ static int departure_entry(int solver, const sht_sl_window* win, const sht_sl_ta
                            void* move_m, void* move_k, void* stream);
 
 static int gather_entry(const sht_sl_window* win, const sht_sl_tables* tables, int order,
-                        int limiter, int deficit, const void* src, int64_t fields, int nlev,
+                        int limiter, int deficit, const void* src,
+                        const void* const* separate, void* packed, int64_t fields, int nlev,
                         const void* xi, const void* phi, const void* level, void* out, void* cut,
                         void* stream) {
   return guarded([&] {
-    check_call(tables, src, fields, nlev, xi, phi, level, out);
+    check_call(tables, separate ? separate[0] : src, fields, nlev, xi, phi, level, out);
+    if (separate) {
+      for (int64_t f = 0; f < fields; ++f) SHT_REQUIRE(separate[f] != nullptr, "null source field");
+      SHT_REQUIRE(fields == 1 || packed != nullptr, "null interleaving buffer");
+    }
     SHT_REQUIRE(limiter == SHT_SL_NONE || limiter == SHT_SL_QUASI_MONOTONE,
                 "the semi-Lagrangian gather's limiter must be one of 'quasi_monotone', 'none'");
     const SlWidth& w = width_of(tables, order);
@@ -1095,13 +1259,17 @@ static int gather_entry(const sht_sl_window* win, const sht_sl_tables* tables, i
     if (tables->prec == SHT_PREC_F64) {
       auto a = make_args<double>(tables, w, src, fields, nlev, xi, phi, level, out, cut);
       band(a);
-      if (order == 6) launch_gather<double, 6>(a, qm, false, s);
-      else launch_gather<double, 4>(a, qm, def, s);
+      if (separate)
+        gather_fields<double>(a, separate, (int)fields, static_cast<double*>(packed), order, qm, def, s);
+      else
+        launch_gather_order<double, 1>(a, order, qm, def, s);
     } else {
       auto a = make_args<float>(tables, w, src, fields, nlev, xi, phi, level, out, cut);
       band(a);
-      if (order == 6) launch_gather<float, 6>(a, qm, false, s);
-      else launch_gather<float, 4>(a, qm, def, s);
+      if (separate)
+        gather_fields<float>(a, separate, (int)fields, static_cast<float*>(packed), order, qm, def, s);
+      else
+        launch_gather_order<float, 1>(a, order, qm, def, s);
     }
   });
 }
@@ -1109,8 +1277,24 @@ static int gather_entry(const sht_sl_window* win, const sht_sl_tables* tables, i
 int sht_sl_gather(const sht_sl_tables* tables, int order, int limiter, int deficit,
                   const void* src, int64_t fields, int nlev, const void* xi, const void* phi,
                   const void* level, void* out, void* cut, void* stream) {
-  return gather_entry(nullptr, tables, order, limiter, deficit, src, fields, nlev, xi, phi, level,
+  return gather_entry(nullptr, tables, order, limiter, deficit, src, nullptr, nullptr, fields, nlev, xi, phi, level,
                       out, cut, stream);
+}
+
+int sht_sl_gather_fields(const sht_sl_tables* tables, const sht_sl_window* win, int order,
+                         int limiter, int deficit, const void* const* fields, int64_t count,
+                         void* packed, int nlev, const void* xi, const void* phi,
+                         const void* level, void* out, void* cut, void* stream) {
+  if (fields == nullptr || count < 1 || count > (1 << 20)) {
+    sht::set_error("fields must point to 1 to 2^20 source arrays");
+    return SHT_ERR_ARG;
+  }
+  if (win != nullptr && win->tables != tables) {
+    sht::set_error("the band window belongs to other tables");
+    return SHT_ERR_ARG;
+  }
+  return gather_entry(win, tables, order, limiter, deficit, nullptr, fields, packed, count, nlev,
+                      xi, phi, level, out, cut, stream);
 }
 
 int sht_sl_window_create(const sht_sl_tables* tables, int s0, int s1, int a0, int a1,
@@ -1193,7 +1377,7 @@ int sht_sl_gather_band(const sht_sl_window* win, int order, int limiter, int def
     sht::set_error("null band window");
     return SHT_ERR_ARG;
   }
-  return gather_entry(win, win->tables, order, limiter, deficit, src, fields, nlev, xi, phi,
+  return gather_entry(win, win->tables, order, limiter, deficit, src, nullptr, nullptr, fields, nlev, xi, phi,
                       level, out, cut, stream);
 }
 

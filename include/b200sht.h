@@ -416,6 +416,11 @@ int sht_batch_inverse(sht_batch* batch, const void* const* coeffs, void* const* 
  * the cubic vertical; limiter SHT_SL_QUASI_MONOTONE clips to the 2x2x2 cell
  * around the point; with deficit != 0 (cubic, limited) cut[f] receives raw
  * minus kept.  sht_sl_gather_linear is the trilinear value inside that cell.
+ * sht_sl_gather_fields is the same for `count` source volumes in arrays of
+ * their own (fields: host array of device pointers), on the whole grid or,
+ * with a window, on its band: the volumes are interleaved into `packed`
+ * (count source volumes of room, 16-byte aligned; not needed for count 1,
+ * whose volume is read in place) and gathered several to a load.
  * Stream-ordered; every pointer is device memory the caller owns. */
 typedef struct sht_sl_tables sht_sl_tables;
 #define SHT_SL_NONE 0
@@ -423,6 +428,11 @@ typedef struct sht_sl_tables sht_sl_tables;
 int sht_sl_tables_create(int nlat, int nlon, const double* lat_rad, const double* lon_rad,
                          int precision, sht_sl_tables** out);
 int sht_sl_tables_destroy(sht_sl_tables* tables);
+struct sht_sl_window;
+int sht_sl_gather_fields(const sht_sl_tables* tables, const struct sht_sl_window* window,
+                         int order, int limiter, int deficit, const void* const* fields,
+                         int64_t count, void* packed, int nlev, const void* xi, const void* phi,
+                         const void* level, void* out, void* cut, void* stream);
 /* Latitude-band windows (the reference's semilag/tables.py BandWindow):
  * arrival rows [a0, a1) of a step read from fields that hold only rows
  * [s0, s1), the band and a row halo.  sht_sl_gather_band and
