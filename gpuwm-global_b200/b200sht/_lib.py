@@ -124,6 +124,8 @@ SIGNATURES = {
     "sht_sl_departure_newton_ls": (ctypes.c_int, [_P, ctypes.c_int, _P, _P, _P, _P, _P, _P, _P,
                                                   _P, ctypes.c_int, _D, _D, _P, _P, _P, _P, _P,
                                                   _P]),
+    "sht_sl_departure_maxima": (ctypes.c_int, [_P, _P, ctypes.c_int, ctypes.c_int] + [_P] * 8
+                                + [ctypes.c_int, _D, _D, _P, _P, _P, _P, _P]),
     "sht_sl_lipschitz": (ctypes.c_int, [_P, ctypes.c_int, ctypes.c_int, ctypes.c_int, _P, _P, _P,
                                         _P, ctypes.c_int, ctypes.c_int, _P, _P, _P, _P,
                                         ctypes.c_int, ctypes.c_int, _D, _D, _D, _DP, _DP,

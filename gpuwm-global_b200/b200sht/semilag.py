@@ -500,28 +500,6 @@ def meridional_grid_length_m(tables: SphericalGridTables) -> np.ndarray:
     return tables.radius_m * 0.5 * (lat_ext[3:nlat + 3] - lat_ext[1:nlat + 1])
 
 
-def _diagnostics(stencil: Stencil, move_m, move_k, tables, dt_s, iterations):
-    nlev, nrows, nlon = stencil.shape
-    nlat = tables.nlat
-    rows = slice(0, nlat) if stencil.window is None else stencil.window.arrival
-    dt = tables.dtype
-    dev = tables.device
-    cell = torch.as_tensor(meridional_grid_length_m(tables)[rows], dtype=dt,
-                           device=dev)[None, :, None]
-    lat = torch.as_tensor(tables.host_tables(4)["lat_ext"][2:nlat + 2][rows], dtype=dt,
-                          device=dev)[None, :, None]
-    index = torch.arange(nlon, dtype=dt, device=dev)[None, None, :]
-    lev0 = torch.arange(nlev, dtype=dt, device=dev)[:, None, None]
-    # great-circle distance through the haversine (no floor from arccos)
-    dphi = 0.5 * (stencil.phi - lat)
-    dlon = 0.5 * (stencil.xi - index) * tables.dlam
-    hav = torch.sin(dphi) ** 2 + torch.cos(lat) * torch.cos(stencil.phi) * torch.sin(dlon) ** 2
-    dist = (2.0 * tables.radius_m) * torch.arcsin(torch.sqrt(torch.clamp(hav, 0.0, 1.0)))
-    maxima = torch.stack([move_m.max(), (move_m / cell).max(), move_k.max(), dist.max(),
-                          (dist / cell).max(), (stencil.level - lev0).abs().max()]).tolist()
-    return TrajectoryDiagnostics(int(iterations), float(dt_s), *[float(x) for x in maxima])
-
-
 _SOLVER_CALLS = {"fixed_point": "sht_sl_departure", "newton": "sht_sl_departure_newton",
                  "newton_ls": "sht_sl_departure_newton_ls"}
 
@@ -575,20 +553,20 @@ def departure_points(wind: CartesianWind, tables: SphericalGridTables, dt_s: flo
             if not field.is_cuda:
                 raise ValueError(f"{name} fields must be CUDA tensors")
     ins = [f.contiguous() for f in wind.arrays()] + [f.contiguous() for f in ex.arrays()]
-    outs = [torch.empty(out_shape, dtype=tables.dtype, device=ins[0].device) for _ in range(5)]
-    if window is None:
-        search_into(tables, ins, int(iterations), float(dt_s), outs, solver=solver)
-    else:
-        if not defer_escape:
-            window.clear_escape()
-        _lib.call("sht_sl_departure_band", window._handle, TRAJECTORY_SOLVERS.index(solver), nlev,
-                  *[_ptr(t) for t in ins], int(iterations), float(dt_s), float(tables.radius_m),
-                  *[_ptr(t) for t in outs], _stream())
-        if not defer_escape:
-            window.raise_if_escaped("departure-point search")
-    xi, phi, lev, move_m, move_k = outs
+    xi, phi, lev = (torch.empty(out_shape, dtype=tables.dtype, device=ins[0].device)
+                    for _ in range(3))
+    # the diagnostics' maxima, merged by the search kernel
+    maxima = torch.zeros(6, dtype=tables.dtype, device=ins[0].device)
+    if window is not None and not defer_escape:
+        window.clear_escape()
+    _lib.call("sht_sl_departure_maxima", (tables if window is None else window.tables)._handle,
+              None if window is None else window._handle, TRAJECTORY_SOLVERS.index(solver), nlev,
+              *[_ptr(t) for t in ins], int(iterations), float(dt_s), float(tables.radius_m),
+              _ptr(xi), _ptr(phi), _ptr(lev), _ptr(maxima), _stream())
+    if window is not None and not defer_escape:
+        window.raise_if_escaped("departure-point search")
     stencil = Stencil(xi=xi, phi=phi, level=lev, tables=tables, window=window)
-    return stencil, _diagnostics(stencil, move_m, move_k, tables, dt_s, iterations)
+    return stencil, TrajectoryDiagnostics(int(iterations), float(dt_s), *maxima.tolist())
 
 
 # ------------------------------------------------------- trajectory gate

@@ -1,7 +1,9 @@
 """Gathers of several separate fields (interleaved in groups of 16 bytes, the
-rest in a pair and a single) against the one-field call."""
+rest in a pair and a single) against the one-field call, and the departure
+search's diagnostics against its move arrays."""
 from __future__ import annotations
 
+import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -47,3 +49,40 @@ def test_grouped_fields_equal_single_fields(dtype, kw):
     for a, b in zip(gather_batch(held, st, **kw), single):
         assert all(torch.equal(x, y[:, 9:24]) for x, y in zip(flat(a), flat(b)))
 
+
+@pytest.mark.parametrize("dtype, tol", [("float64", 1e-11), ("float32", 2e-4)])
+@pytest.mark.parametrize("solver", ["fixed_point", "newton", "newton_ls"])
+def test_search_maxima_match_the_move_arrays(dtype, tol, solver):
+    """The maxima of the moves the arrays hold, and the displacement as a
+    great-circle distance in float64 (float32: a unit vector's rounding,
+    6e-8 rad, against displacements of a few 1e-3 rad)."""
+    import torch
+
+    from b200sht.semilag import (CartesianWind, departure_points, meridional_grid_length_m,
+                                 search_into)
+
+    dt = getattr(torch, dtype)
+    tables, _, field = _setup(dt)
+    wind = [30.0 * field() for _ in range(3)] + [1e-3 * field()]
+    ahead = [30.0 * field() for _ in range(3)] + [1e-3 * field()]
+    outs = [torch.empty_like(wind[0]) for _ in range(5)]
+    search_into(tables, wind + ahead, 3, 300.0, outs, solver=solver)
+    st, d = departure_points(CartesianWind(*wind), tables, 300.0, extrapolated=CartesianWind(*ahead),
+                             solver=solver)
+    assert all(torch.equal(a, b) for a, b in zip((st.xi, st.phi, st.level), outs))
+    xi, phi, lev, move_m, move_k = (x.double().cpu().numpy() for x in outs)
+    cell = meridional_grid_length_m(tables)[None, :, None]
+    lat = tables.host_tables(4)["lat_ext"][2:-2][None, :, None]
+    dlam = 2 * np.pi / tables.nlon
+    dl = (xi - np.arange(tables.nlon)) * dlam
+    hav = np.sin(0.5 * (phi - lat)) ** 2 + np.cos(lat) * np.cos(phi) * np.sin(0.5 * dl) ** 2
+    dist = 2 * tables.radius_m * np.arcsin(np.sqrt(hav))
+    want = [move_m.max(), (move_m / cell).max(), move_k.max(), dist.max(), (dist / cell).max(),
+            np.abs(lev - np.arange(lev.shape[0])[:, None, None]).max()]
+    got = [d.move_max_m, d.move_max_cells, d.move_max_levels, d.displacement_max_m,
+           d.displacement_max_cells, d.displacement_max_levels]
+    np.testing.assert_allclose(got, want, rtol=tol)
+    wind[3][2, 5, 6] = float("nan")  # a NaN level rate reaches the level maxima
+    _, d = departure_points(CartesianWind(*wind), tables, 300.0, solver=solver)
+    assert np.isnan(d.displacement_max_levels) == bool(torch.isnan(
+        departure_points(CartesianWind(*wind), tables, 300.0, solver=solver)[0].level).any())
