@@ -269,6 +269,7 @@ __device__ __forceinline__ void pk_fma(T w, const Pack<T, VEC>& a, Pack<T, VEC>&
   }
 }
 
+constexpr int kGatherX = 32, kGatherY = 2, kGatherZ = 2;  // points of a CTA: columns, levels, rows
 // Interleaves fields into groups of VEC: out[g][point] = (f[g VEC], ...).
 constexpr int kPackFields = 16;
 struct PackArgs { const void* f[kPackFields]; };
@@ -283,26 +284,28 @@ __global__ void __launch_bounds__(256) sl_pack_kernel(const __grid_constant__ Pa
   out[blockIdx.y * n + t] = r;
 }
 
-// A CTA takes 32 columns x 4 levels x 2 rows of arrival points: the taps of
-// its 256 points fall in about 36 x 7 x 6 source points, which stay in L1 (a
+// A CTA takes 32 columns x 2 levels x 2 rows of arrival points: the taps of
+// its 128 points fall in about 36 x 5 x 6 source points, which stay in L1 (a
 // CTA of 256 columns of one level reads 260 x 4 x 4).  Four floats per tap
 // load (fields interleaved by sl_pack_kernel, which takes the place of the
 // copy that put the batch's fields in one block) cut the load instructions by
 // four and the half-used lines of misaligned 128-byte warp loads; the
 // interpolation arithmetic runs on packed pairs.  Sixteen FP32 fields with the
-// limiter at T511 L40: 16.2 ms one float per load, 9.9 ms four (19.6 TB/s of
-// taps; the bound is the L1's 128 bytes a clock, 5.4 ms), and 0.98 ms to
-// interleave against 0.89 ms for the copy.
+// limiter at T511 L40: 16.2 ms one float per load, 9.9 ms four (the L1's 128
+// bytes a clock would take 5.4 ms: it waits for the taps at 16 warps an SM), 9.3
+// ms in CTAs of 128 points, five to an SM (FP64: four); and 0.98 ms to interleave
+// against 0.89 ms for the copy.
 template <typename T, int NH, int VEC, bool QM, bool DEF>
-__global__ void __launch_bounds__(256, (sizeof(T) == 4 && VEC <= 2 && NH == 4) ? 3 : 2)
+__global__ void __launch_bounds__(kGatherX * kGatherY * kGatherZ,
+                                  NH == 6 || sizeof(T) == 8 ? 4 : (VEC == 4 ? 5 : 6))
     sl_gather_kernel(const SlArgs<T> a) {
   using P = Pack<T, VEC>;
   constexpr int G = NH / 2 - 1;  // zonal lead and meridional start offset
   constexpr int MID = NH / 2 - 1;
   const int plane = a.njs * a.ni;              // a held source level
   const int64_t n = (int64_t)a.nk * a.nja * a.ni;  // arrival points
-  const int ia = blockIdx.x * 32 + threadIdx.x;
-  const int ka = blockIdx.y * 4 + threadIdx.y, ja = blockIdx.z * 2 + threadIdx.z;
+  const int ia = blockIdx.x * kGatherX + threadIdx.x;
+  const int ka = blockIdx.y * kGatherY + threadIdx.y, ja = blockIdx.z * kGatherZ + threadIdx.z;
   if (ia >= a.ni || ka >= a.nk || ja >= a.nja) return;
   const int64_t gid = ((int64_t)ka * a.nja + ja) * a.ni + ia;
   const T p = min(max(a.phi[gid], T(-kHalfPi)), T(kHalfPi));
@@ -1137,8 +1140,9 @@ SlArgs<T> make_args(const sht_sl_tables* t, const SlWidth& w, const void* src, i
 
 template <typename T, int NH, int VEC>
 void launch_gather(const SlArgs<T>& a, bool qm, bool def, cudaStream_t s) {
-  const dim3 block(32, 4, 2);
-  const dim3 grid((unsigned)div_up(a.ni, 32), (unsigned)div_up(a.nk, 4), (unsigned)div_up(a.nja, 2));
+  const dim3 block(kGatherX, kGatherY, kGatherZ);
+  const dim3 grid((unsigned)div_up(a.ni, kGatherX), (unsigned)div_up(a.nk, kGatherY),
+                  (unsigned)div_up(a.nja, kGatherZ));
   SHT_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "too many levels or rows for one gather launch");
   if constexpr (NH == 6) {
     if (qm) sl_gather_kernel<T, 6, VEC, true, false><<<grid, block, 0, s>>>(a);
