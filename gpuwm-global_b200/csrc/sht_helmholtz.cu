@@ -465,6 +465,332 @@ __global__ void __launch_bounds__(256) semi_implicit_kernel(
   }
 }
 
+// ------------------------------------------------------- the stage solve
+// kSemiSolve as four small matrix products per CTA over 64 coefficients (two
+// blocks of 32 orders, each of its own degree): forcing = D + tau k^2 B x, the
+// modal solve, D' and x'.  Bound by the shared loads that feed the multiply-
+// adds: a thread holds RT rows x 4 complex columns (8 x 4 in FP32, where the
+// real and imaginary parts are one packed pair), so a loaded matrix entry
+// serves 4 columns and a loaded coefficient RT rows; the general kernel above
+// holds 6 rows x 1 column and reads a 16-byte matrix piece per 8 multiply-adds.
+// The next item's x comes in by cp.async behind the products.  Blocks above the
+// triangle are zeroed by the same launch.  T255 x 40 levels FP32: 88 -> 64 us,
+// T511 288 -> 249 us; what is left waits for instructions and for the serial
+// products (6 warps an SM, 25 % of the FMA pipe).
+template <typename T> struct SolveCfg { static constexpr int RT = sizeof(T) == 4 ? 8 : 4; };
+constexpr int kSolveCols = 64;
+
+// Shared memory of one CTA (bytes) and its threads, for nlev levels.
+template <typename T>
+size_t solve_smem(int nlev, int* threads) {
+  constexpr int RT = SolveCfg<T>::RT;
+  const int L1 = nlev + 1, groups = (L1 + RT - 1) / RT, rpc = RT * groups;
+  const int rp = RT * ((nlev + RT - 1) / RT);
+  *threads = (16 * groups + 31) / 32 * 32;
+  return sizeof(T) * ((size_t)(L1 + 2 * nlev) * rp + (size_t)nlev * rpc + padded(nlev)) +
+         sizeof(V2<T>) * (size_t)kSolveCols * (2 * L1 + 2 * nlev);
+}
+
+// acc[r][c] += sum_j Mt[j][g RT + r] vec[j][c] for the thread's columns
+// 2 cg, 2 cg + 1, 32 + 2 cg, 33 + 2 cg.
+template <typename T>
+__device__ __forceinline__ void solve_product(const T* Mt, int rp, int K, const V2<T>* vec, int g,
+                                              int cg, V2<T> (&acc)[SolveCfg<T>::RT][4]) {
+  constexpr int RT = SolveCfg<T>::RT;
+  const T* m = Mt + g * RT;
+  const V2<T>* v = vec + 2 * cg;
+#pragma unroll
+  for (int r = 0; r < RT; ++r)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) acc[r][c] = mk2<T>(T(0), T(0));
+#pragma unroll 4
+  for (int j = 0; j < K; ++j) {
+    T a[RT];
+#pragma unroll
+    for (int r = 0; r < RT; r += 4) {
+      T q[4];
+      Quad<T>::load(m + j * rp + r, q);
+      a[r] = q[0]; a[r + 1] = q[1]; a[r + 2] = q[2]; a[r + 3] = q[3];
+    }
+    V2<T> x[4];
+    T q[4];
+    Quad<T>::load(reinterpret_cast<const T*>(v + j * kSolveCols), q);
+    x[0] = mk2<T>(q[0], q[1]);
+    x[1] = mk2<T>(q[2], q[3]);
+    Quad<T>::load(reinterpret_cast<const T*>(v + j * kSolveCols + 32), q);
+    x[2] = mk2<T>(q[0], q[1]);
+    x[3] = mk2<T>(q[2], q[3]);
+#pragma unroll
+    for (int r = 0; r < RT; ++r)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        if constexpr (sizeof(T) == 4) {
+          acc[r][c] = __ffma2_rn(make_float2(a[r], a[r]), x[c], acc[r][c]);
+        } else {
+          acc[r][c].x = fma(a[r], x[c].x, acc[r][c].x);
+          acc[r][c].y = fma(a[r], x[c].y, acc[r][c].y);
+        }
+      }
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(224) semi_solve_kernel(
+    SemiArgs a, const T* __restrict__ mats, const V2<T>* div, const V2<T>* theta,
+    const V2<T>* lnps, V2<T>* odiv, V2<T>* otheta, V2<T>* olnps, T* __restrict__ metric,
+    V2<T>* __restrict__ cfold, float* __restrict__ rowmax) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int RT = SolveCfg<T>::RT, NC = kSolveCols;
+  const int Tn = a.Tn, nlev = a.nlev, L1 = nlev + 1;
+  const int groups = (L1 + RT - 1) / RT, rpc = RT * groups, rp = RT * ((nlev + RT - 1) / RT);
+  // [column][row] copies of B, V^-1, V, C, rows padded with zeros to rp (C: rpc)
+  T* sB = reinterpret_cast<T*>(smem_raw);
+  T* sVi = sB + L1 * rp;
+  T* sV = sVi + nlev * rp;
+  T* sC = sV + nlev * rp;
+  T* sLam = sC + nlev * rpc;
+  V2<T>* xbuf = reinterpret_cast<V2<T>*>(sLam + padded(nlev));  // x of two items
+  V2<T>* fs = xbuf + 2 * L1 * NC;
+  V2<T>* gs = fs + nlev * NC;
+  __shared__ float s_rowmax[2 * kMaxLev];
+  __shared__ T s_metric;
+  const int tid = threadIdx.x, nt = blockDim.x;
+  const int g = tid >> 4, cg = tid & 15;
+  {
+    const T* B = mats;
+    const T* C = B + nlev * L1;
+    const T* V = C + L1 * nlev;
+    const T* Vi = V + nlev * nlev;
+    const T* lam = Vi + nlev * nlev;
+    auto transpose = [&](T* dst, const T* src, int rows, int cols, int ld) {
+#pragma unroll 8
+      for (int e = tid; e < cols * ld; e += nt) {
+        const int j = e / ld, i = e - j * ld;
+        dst[e] = i < rows ? src[i * cols + j] : T(0);
+      }
+    };
+    transpose(sB, B, nlev, L1, rp);
+    transpose(sVi, Vi, nlev, nlev, rp);
+    transpose(sV, V, nlev, nlev, rp);
+    transpose(sC, C, L1, nlev, rpc);
+    for (int e = tid; e < nlev; e += nt) sLam[e] = lam[e];
+    for (int e = tid; e < 2 * kMaxLev; e += nt) s_rowmax[e] = 0.f;
+    if (tid == 0) s_metric = T(0);
+  }
+  const int64_t t1 = Tn + 1, lev = t1 * t1;
+  const int nmb = (Tn + 32) / 32;
+  const T dt = T(a.dt);
+  T my_metric = T(0);
+  // Blocks inside the triangle in the order (order block, degree): block mb
+  // holds the degrees 32 mb .. T.
+  const int blocks = nmb * (Tn + 1) - 16 * nmb * (nmb - 1);
+  const int items = (blocks + 1) / 2;
+  auto locate = [&](int item, int (&n)[2], int (&m0)[2]) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      int b = 2 * item + h, mb = 0;
+      const bool have = b < blocks;
+      while (have && b >= Tn + 1 - 32 * mb) b -= Tn + 1 - 32 * mb++;
+      n[h] = have ? 32 * mb + b : -1;
+      m0[h] = 32 * mb;
+    }
+  };
+  // x of an item into one of the two buffers, copies in flight while the
+  // previous item is worked on; zero outside the triangle.
+  auto fetch_x = [&](int item, V2<T>* xs) {
+    int n[2], m0[2];
+    locate(item, n, m0);
+    for (int e = tid; e < L1 * NC; e += nt) {
+      const int i = e / NC, c = e % NC, h = c >> 5, m = m0[h] + (c & 31);
+      const bool in = m <= n[h];
+      const V2<T>* src = in ? (i < nlev ? theta + i * lev : lnps) + n[h] * t1 + m : lnps;
+      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(xs + e), bytes = in ? sizeof(V2<T>) : 0;
+      if constexpr (sizeof(V2<T>) == 8)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+      else
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+    }
+  };
+  int turn = 0;
+  fetch_x(blockIdx.x, xbuf);
+  for (int item = blockIdx.x; item < items; item += gridDim.x, turn ^= 1) {
+    int n[2], m0[2];
+    locate(item, n, m0);
+    V2<T>* xs = xbuf + turn * L1 * NC;
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();  // x and the operators are staged; the previous item's vectors are consumed
+    if (item + (int)gridDim.x < items) fetch_x(item + gridDim.x, xbuf + (turn ^ 1) * L1 * NC);
+    T k2[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      k2[h] = T((double)n[h] * ((double)n[h] + 1.0) / (a.radius * a.radius));
+    const bool rows_in = g < groups;
+    V2<T> acc[RT][4];
+    // column c of the thread: half h = c >> 1, order m0[h] + 2 cg + (c & 1)
+    auto order = [&](int c) { return m0[c >> 1] + 2 * cg + (c & 1); };
+    auto live = [&](int c) { return order(c) <= n[c >> 1]; };
+    auto at = [&](int c) { return (int64_t)n[c >> 1] * t1 + order(c); };
+    auto put = [&](V2<T>* vec, int i, int c, V2<T> v) { vec[i * NC + 32 * (c >> 1) + 2 * cg + (c & 1)] = v; };
+    const bool rows_n = g * RT < nlev;  // C has one row more than the others
+    // forcing = D + dt k2 (B x)
+    if (rows_n) {
+      V2<T> d[RT][4];
+#pragma unroll
+      for (int r = 0; r < RT; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          d[r][c] = g * RT + r < nlev && live(c) ? div[(g * RT + r) * lev + at(c)] : mk2<T>(T(0), T(0));
+      solve_product<T>(sB, rp, L1, xs, g, cg, acc);
+#pragma unroll
+      for (int r = 0; r < RT; ++r)
+        if (g * RT + r < nlev)
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            put(fs, g * RT + r, c, mk2<T>(d[r][c].x + dt * k2[c >> 1] * acc[r][c].x,
+                                          d[r][c].y + dt * k2[c >> 1] * acc[r][c].y));
+    }
+    __syncthreads();
+    // g = diag(1 / (1 + dt^2 k2 lambda)) V^-1 forcing
+    if (rows_n) {
+      solve_product<T>(sVi, rp, nlev, fs, g, cg, acc);
+#pragma unroll
+      for (int r = 0; r < RT; ++r)
+        if (g * RT + r < nlev) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const T modal = T(1) / (T(1) + (dt * dt * k2[c >> 1]) * sLam[g * RT + r]);
+            put(gs, g * RT + r, c, mk2<T>(acc[r][c].x * modal, acc[r][c].y * modal));
+          }
+        }
+    }
+    __syncthreads();
+    // D' = V g: degree zero passes through, the outputs are projected
+    if (rows_n) {
+      // D itself, for degree zero and the metric
+      V2<T> d[RT][4];
+#pragma unroll
+      for (int r = 0; r < RT; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          d[r][c] = g * RT + r < nlev && live(c) && (metric != nullptr || n[c >> 1] == 0)
+                        ? div[(g * RT + r) * lev + at(c)] : mk2<T>(T(0), T(0));
+      solve_product<T>(sV, rp, nlev, gs, g, cg, acc);
+#pragma unroll
+      for (int r = 0; r < RT; ++r) {
+        const int i = g * RT + r;
+        float mre = 0.f, mim = 0.f;
+        if (i < nlev) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            V2<T> dn = acc[r][c];
+            const int m = order(c), nn = n[c >> 1];
+            if (m > nn) {
+              dn = mk2<T>(T(0), T(0));
+            } else {
+              const V2<T> d0 = d[r][c];
+              if (nn == 0) dn = d0;
+              if (m == 0) dn.y = T(0);
+              const T ex = dn.x - d0.x, ey = dn.y - d0.y;
+              my_metric = fmax(my_metric, sqrt(ex * ex + ey * ey));
+            }
+            if (nn >= 0 && m <= Tn) odiv[i * lev + at(c)] = dn;
+            put(fs, i, c, dn);
+            acc[r][c] = dn;
+            mre = fmaxf(mre, (float)fabs(dn.x));
+            mim = fmaxf(mim, (float)fabs(dn.y));
+          }
+        }
+        if (rowmax != nullptr) {
+          // the 16 threads of a row group hold row i's columns
+          const unsigned mask = 0xffffu << (16 * (g & 1));
+          for (int off = 8; off > 0; off >>= 1) {
+            mre = fmaxf(mre, __shfl_xor_sync(mask, mre, off));
+            mim = fmaxf(mim, __shfl_xor_sync(mask, mim, off));
+          }
+          if (cg == 0 && i < nlev) {
+            atomicMax(reinterpret_cast<int*>(&s_rowmax[2 * i]), __float_as_int(mre));
+            atomicMax(reinterpret_cast<int*>(&s_rowmax[2 * i + 1]), __float_as_int(mim));
+          }
+        }
+      }
+      if (cfold != nullptr) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          if (!live(c)) continue;
+          const int m = order(c), q = (n[c >> 1] - m) & 1, ii = (n[c >> 1] - m) >> 1;
+          const int64_t row = (int64_t)m * (Tn + 1) - (int64_t)m * (m - 1) / 2 +
+                              (q ? parity_count(Tn, m, 0) : 0) + ii;
+          V2<T>* dst = cfold + row * a.cf_planes + g * RT;
+#pragma unroll
+          for (int r = 0; r < RT; ++r)
+            if (g * RT + r < nlev) dst[r] = acc[r][c];
+        }
+      }
+    }
+    __syncthreads();
+    // x' = x + dt C D'
+    if (rows_in) {
+      solve_product<T>(sC, rpc, nlev, fs, g, cg, acc);
+#pragma unroll
+      for (int r = 0; r < RT; ++r) {
+        const int i = g * RT + r;
+        if (i >= L1) continue;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const int m = order(c), nn = n[c >> 1];
+          if (nn < 0 || m > Tn) continue;
+          const V2<T> x = xs[i * NC + 32 * (c >> 1) + 2 * cg + (c & 1)];
+          V2<T> xn = mk2<T>(x.x + dt * acc[r][c].x, x.y + dt * acc[r][c].y);
+          if (nn == 0) xn = x;
+          if (m == 0) xn.y = T(0);
+          if (m > nn) xn = mk2<T>(T(0), T(0));
+          (i < nlev ? otheta[i * lev + at(c)] : olnps[at(c)]) = xn;
+        }
+      }
+    }
+  }
+  // Blocks above the triangle: zeros.
+  {
+    const int above = 16 * nmb * (nmb - 1), lane = tid & 31, warps = nt >> 5;
+    for (int b0 = blockIdx.x; b0 < above; b0 += gridDim.x) {
+      int b = b0, mb = 1;
+      while (b >= 32 * mb) b -= 32 * mb++;
+      const int m = 32 * mb + lane;
+      if (m > Tn) continue;
+      const int64_t cidx = (int64_t)b * t1 + m;
+      for (int i = tid >> 5; i < nlev; i += warps) {
+        odiv[i * lev + cidx] = mk2<T>(T(0), T(0));
+        otheta[i * lev + cidx] = mk2<T>(T(0), T(0));
+      }
+      if (tid < 32) olnps[cidx] = mk2<T>(T(0), T(0));
+    }
+  }
+  if (metric != nullptr || rowmax != nullptr) {
+    __syncthreads();
+    for (int off = 16; off > 0; off >>= 1)
+      my_metric = fmax(my_metric, __shfl_xor_sync(0xffffffffu, my_metric, off));
+    if (metric != nullptr && (tid & 31) == 0) {
+      if constexpr (sizeof(T) == 8) {
+        atomicMax(reinterpret_cast<unsigned long long*>(&s_metric),
+                  (unsigned long long)__double_as_longlong(my_metric));
+      } else {
+        atomicMax(reinterpret_cast<unsigned*>(&s_metric), __float_as_uint(my_metric));
+      }
+    }
+    __syncthreads();
+    if (metric != nullptr && tid == 0) {
+      if constexpr (sizeof(T) == 8)
+        atomicMax(reinterpret_cast<unsigned long long*>(metric),
+                  (unsigned long long)__double_as_longlong(s_metric));
+      else
+        atomicMax(reinterpret_cast<unsigned*>(metric), __float_as_uint(s_metric));
+    }
+    if (rowmax != nullptr)
+      for (int e = tid; e < 2 * nlev; e += nt)
+        atomicMax(reinterpret_cast<int*>(rowmax + e), __float_as_int(s_rowmax[e]));
+  }
+}
+
 }  // namespace
 
 template <typename T>
@@ -478,19 +804,41 @@ void launch_semi_implicit(const sht_plan* p, int nlev, const T* mats, bool has_t
               "unknown semi-implicit mode");
   SHT_REQUIRE(mode != kSemiHalf || has_thermo,
               "half_apply needs the thermodynamic block's modes (sht_vertical_create_modes)");
+  int dev = 0, sms = 0;
+  SHT_CUDA_OR_THROW(cudaGetDevice(&dev));
+  SHT_CUDA_OR_THROW(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const SemiArgs a{p->T, nlev, mode, p->radius, dt, alpha, ldc};
+  // The stage solve by its own kernel while its operators and three vectors fit
+  // an SM (FP32 to about 66 levels, FP64 to about 40); the general kernel keeps
+  // the other maps and more levels.
+  int threads = 0;
+  const size_t solve = solve_smem<T>(nlev, &threads);
+  if (mode == kSemiSolve && threads <= 224 && solve + 2048 <= 227 * 1024) {
+    SHT_CUDA_OR_THROW(cudaFuncSetAttribute(semi_solve_kernel<T>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)solve));
+    int per_sm = 0;
+    SHT_CUDA_OR_THROW(
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, semi_solve_kernel<T>, threads, solve));
+    SHT_REQUIRE(per_sm > 0, "semi-implicit solve does not fit on an SM at this nlev");
+    const int64_t nmb = div_up(p->T + 1, 32);
+    const int64_t items = div_up(nmb * (p->T + 1) - 16 * nmb * (nmb - 1), 2);
+    const int ctas = (int)std::min<int64_t>(items, (int64_t)per_sm * sms);
+    semi_solve_kernel<T><<<ctas, threads, solve, s>>>(
+        a, mats, (const V2<T>*)div, (const V2<T>*)theta, (const V2<T>*)lnps, (V2<T>*)odiv,
+        (V2<T>*)otheta, (V2<T>*)olnps, metric, (V2<T>*)cfold, rowmax);
+    SHT_CUDA_OR_THROW(cudaGetLastError());
+    return;
+  }
   const SmemPlan sp = smem_plan(nlev, mode);
   const size_t sm = sizeof(T) * (size_t)sp.nmat + sizeof(V2<T>) * 32 * (size_t)(sp.nvec * sp.vp);
   SHT_CUDA_OR_THROW(cudaFuncSetAttribute(semi_implicit_kernel<T>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  int per_sm = 0, dev = 0, sms = 0;
+  int per_sm = 0;
   SHT_CUDA_OR_THROW(
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, semi_implicit_kernel<T>, 256, sm));
   SHT_REQUIRE(per_sm > 0, "semi-implicit kernel does not fit on an SM at this nlev");
-  SHT_CUDA_OR_THROW(cudaGetDevice(&dev));
-  SHT_CUDA_OR_THROW(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const int64_t items = div_up(p->T + 1, 32) * (int64_t)(p->T + 1);
   const int ctas = (int)std::min<int64_t>(items, (int64_t)per_sm * sms);
-  SemiArgs a{p->T, nlev, mode, p->radius, dt, alpha, ldc};
   semi_implicit_kernel<T><<<ctas, dim3(32, 8), sm, s>>>(
       a, mats, (const V2<T>*)div, (const V2<T>*)theta, (const V2<T>*)lnps, (V2<T>*)odiv,
       (V2<T>*)otheta, (V2<T>*)olnps, metric, (V2<T>*)cfold, rowmax);
