@@ -217,6 +217,61 @@ __global__ void __launch_bounds__(32 * WX, 16 / WX) gemm_simt_kernel(const __gri
     simt_tile<T, WX, G, DB>(grp, d, it.x0, r0, a.R, smem);
 }
 
+// At most 8 data rows (one to four planes): bound by reading the table once and,
+// below T511, by the latency of the chain over k, so every lane takes one
+// column (the most warps in flight) with U table rows on their way; the data
+// values are one address for the whole warp.  The same chain of fused multiply-
+// adds per output as the tiles.  Against a half-empty 32-row tile: T241 x 3
+// planes FP32 (8 rows), both contractions, 45 us less of a 136 us pair (four
+// columns to a lane: 22 us more); the P and dP/dphi syntheses of one T255 plane
+// 44 -> 28 us; T21 x 1 plane 7.4 -> 6.0 us.
+template <typename T, int RR>
+__global__ void __launch_bounds__(128) gemm_skinny_kernel(const __grid_constant__ SimtArgs<T> a) {
+  constexpr int U = 16 * 4 / (RR * (int)sizeof(T) / 4);
+  unsigned b = blockIdx.x;
+  const SimtGroup<T>& grp = a.g[a.ng == 2 ? (b & 1) : 0];
+  if (a.ng == 2) b >>= 1;
+  const ShtGemmItem it = a.items[b];
+  const ShtGemmDesc d = grp.descs[it.problem];
+  const int R = (int)a.R;
+  const int x = it.x0 + (int)threadIdx.x;
+  if (x >= d.X) return;
+  using Q = std::conditional_t<sizeof(T) == 4, float2, double2>;  // two rows
+  const T* tab = grp.table + d.t_off + x;
+  const T* dat = grp.data + d.d_row * a.R;
+  T acc[RR];
+#pragma unroll
+  for (int r = 0; r < RR; ++r) acc[r] = T(0);
+  auto step = [&](int k, T t) {
+    const Q* p = reinterpret_cast<const Q*>(dat + (int64_t)k * R);
+#pragma unroll
+    for (int r = 0; r < RR; r += 2)
+      if (r < R) {
+        const Q q = __ldg(p + r / 2);
+        acc[r] = fma(t, q.x, acc[r]);
+        acc[r + 1] = fma(t, q.y, acc[r + 1]);
+      }
+  };
+  int k = 0;
+  for (; k + U <= d.K; k += U) {
+    T t[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) t[u] = __ldg(tab + (int64_t)(k + u) * d.ldt);
+#pragma unroll
+    for (int u = 0; u < U; ++u) step(k + u, t[u]);
+  }
+  for (; k < d.K; ++k) step(k, __ldg(tab + (int64_t)k * d.ldt));
+  T* o = grp.out + (d.c_row + x) * a.R;
+#pragma unroll
+  for (int r = 0; r < RR; r += 2)
+    if (r < R) {
+      Q q;
+      q.x = acc[r];
+      q.y = acc[r + 1];
+      *reinterpret_cast<Q*>(o + r) = q;
+    }
+}
+
 }  // namespace
 
 void build_gemm_items(sht_plan* p) {
@@ -315,17 +370,27 @@ void launch_gemm_simt_groups(const sht_plan* p, int direction, int ngroups, cons
   // data reloads make up for it (T511 x 200 planes 1921 against 1955 us; T255 x
   // 161 planes 292 against 264, T126 x 200 planes 76 against 70).
   const bool narrow = std::is_same<T, float>::value && (p->tune_simt_tile == 1 || p->H < 256);
-  const int n_items = narrow ? p->n_items_narrow[direction] : p->n_items[direction];
+  const bool skinny = R <= 8;
+  const int n_items = narrow && !skinny ? p->n_items_narrow[direction] : p->n_items[direction];
   if (n_items == 0 || R == 0) return;
   SHT_REQUIRE(ngroups == 1 || ngroups == 2, "one or two tables per SIMT launch");
   SHT_REQUIRE(p->gemm_bx == tile_x<T>(4), "SIMT work list built for another tile width");
   SimtArgs<T> a{};
   for (int g = 0; g < ngroups; ++g)
     a.g[g] = {p->d_desc[direction][flip[g]], table[g], data[g], out[g]};
-  a.items = narrow ? p->d_items_narrow[direction] : p->d_items[direction];
+  a.items = narrow && !skinny ? p->d_items_narrow[direction] : p->d_items[direction];
   SHT_REQUIRE(a.items != nullptr, "SIMT work list not built");
   a.ng = ngroups;
   a.R = R;
+  if (skinny) {
+    const unsigned blocks = (unsigned)n_items * (unsigned)ngroups, threads = tile_x<T>(4);
+    if (R <= 4)
+      gemm_skinny_kernel<T, 4><<<blocks, threads, 0, s>>>(a);
+    else
+      gemm_skinny_kernel<T, 8><<<blocks, threads, 0, s>>>(a);
+    SHT_CUDA_OR_THROW(cudaGetLastError());
+    return;
+  }
   const int whole = tile_r<T>(SimtCfg<T>::G);
   a.nrb = (int)div_up(R, whole);
   a.half = R % whole != 0 && R % whole <= whole / 2;
