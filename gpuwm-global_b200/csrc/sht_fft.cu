@@ -646,8 +646,12 @@ FftShape make_shape(const sht_plan* p, int64_t cols, int no, size_t* smem, int* 
   f.rs = stride(lc);
   f.tw_shared = bytes(lc) + table <= kMost ? 1 : 0;
   *smem = bytes(lc) + (f.tw_shared ? table : 0);
-  const int work = ((2 * no) << lc) * p->L;  // elements; about eight per thread and pass
-  *threads = std::max(work >= 1536 ? 256 : (work >= 768 ? 128 : 64), 4 * ((2 * no) << lc));
+  // About eight elements per thread and pass; in FP64 (128 registers a thread:
+  // 16 warps an SM) 256 threads only where shared memory leaves two CTAs (T62,
+  // forward: 256 threads 25 us, 128 threads 20; T159 x 39 planes: 41 against 49).
+  const int work = ((2 * no) << lc) * p->L;
+  const int wide = sizeof(T) == 8 && 3 * (*smem + 1024) <= kMost ? 3072 : 1536;
+  *threads = std::max(work >= wide ? 256 : (work >= 768 ? 128 : 64), 4 * ((2 * no) << lc));
   return f;
 }
 
