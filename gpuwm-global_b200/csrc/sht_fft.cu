@@ -580,6 +580,15 @@ __global__ void twiddle_cast_kernel(const double2* in, float2* out, int n) {
   if (k < n) out[k] = make_float2((float)in[k].x, (float)in[k].y);
 }
 
+// [k1][lane] twiddles of the register kernels: exp(-2 pi i lane k1 / L), L = 32 F.
+__global__ void lane_twiddle_kernel(const double2* tl, float2* out, int F) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e < 32 * F) {
+    const double2 w = tl[(e & 31) * (e >> 5) % (32 * F)];
+    out[e] = make_float2((float)w.x, (float)w.y);
+  }
+}
+
 // The radix sequence of length L: the fewest passes of radices 2 .. 16 (13
 // and below the prime ones), and among those the smallest sum of radices
 // (the widest passes); other primes by the direct pass.
@@ -684,6 +693,13 @@ void build_fft(sht_plan* p, cudaStream_t s) {
     SHT_CUDA_OR_THROW(cudaMalloc(&fn, sizeof(float2) * (L + 1)));
     twiddle_cast_kernel<<<(L + 255) / 256, 256, 0, s>>>(tl, fl, L);
     twiddle_cast_kernel<<<(L + 256) / 256, 256, 0, s>>>(tn, fn, L + 1);
+    if (fast_fft_supported(p)) {
+      float2* lanes = nullptr;
+      SHT_CUDA_OR_THROW(cudaMalloc(&lanes, sizeof(float2) * L));
+      p->tw_lane = lanes;
+      lane_twiddle_kernel<<<(L + 255) / 256, 256, 0, s>>>(tl, lanes, L / 32);
+      SHT_CUDA_OR_THROW(cudaGetLastError());
+    }
     SHT_CUDA_OR_THROW(cudaStreamSynchronize(s));
     cudaFree(tl);
     cudaFree(tn);

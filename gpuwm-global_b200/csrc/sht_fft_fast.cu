@@ -169,14 +169,12 @@ template <int F> struct WarpSmem {
 // The four-step twiddles exp(-2 pi i l k1 / L) of every lane l, as a shared
 // table [k1][32]: a warp's read of one k1 is 32 consecutive entries (two
 // wavefronts), where reading them from the length-L table in global memory
-// touched up to F * 8 different cache lines per instruction.
+// touched up to F * 8 different cache lines per instruction.  The plan holds
+// the table in this order (sht_plan::tw_lane), so a CTA's copy is in order too
+// (T511 x 200 planes forward: 408 us gathering it, 396).
 template <int F>
-__device__ __forceinline__ void load_lane_twiddles(float2* tws, const float2* __restrict__ twL) {
-  constexpr int L = 32 * F;
-  for (int e = threadIdx.x; e < F * 32; e += blockDim.x) {
-    const int k1 = e >> 5, l = e & 31;
-    tws[e] = twL[(l * k1) % L];
-  }
+__device__ __forceinline__ void load_lane_twiddles(float2* tws, const float2* __restrict__ tw_lane) {
+  for (int e = threadIdx.x; e < F * 32; e += blockDim.x) tws[e] = tw_lane[e];
 }
 
 // R rows per warp: for small F one row leaves most lanes idle in the
@@ -271,7 +269,7 @@ template <int FF, int W, int TC>
 __global__ void __launch_bounds__(W * 32, 24 / W) fast_forward_fold(FastFoldArgs a,
                                                                     const float* __restrict__ g0,
                                                                     const float* __restrict__ g1,
-                                                                    const float2* __restrict__ twL,
+                                                                    const float2* __restrict__ tw_lane,
                                                                     const float2* __restrict__ twN,
                                                                     float2* __restrict__ wfold,
                                                                     float* __restrict__ rowmax) {
@@ -304,7 +302,7 @@ __global__ void __launch_bounds__(W * 32, 24 / W) fast_forward_fold(FastFoldArgs
                   (uint32_t)(a.nlon * sizeof(float)));
     }
   }
-  load_lane_twiddles<FF>(tws, twL);
+  load_lane_twiddles<FF>(tws, tw_lane);
   for (int m = threadIdx.x; m <= a.T; m += blockDim.x) twn[m] = twN[m];
   __syncthreads();
   {
@@ -432,7 +430,7 @@ template <int FF, int NF, int TC>
 __global__ void __launch_bounds__(InvCfg<NF>::W * 32, 16 / InvCfg<NF>::W)
     fast_inverse_pair(FastUnfoldArgs a, const float2* __restrict__ wP,
                       const float2* __restrict__ wD, const double* __restrict__ coslat,
-                      const float2* __restrict__ twL, const float2* __restrict__ twN,
+                      const float2* __restrict__ tw_lane, const float2* __restrict__ twN,
                       float* __restrict__ out0, float* __restrict__ out1, int n_pb) {
   constexpr int NO = InvCfg<NF>::NO, NB = InvCfg<NF>::NB, kW = InvCfg<NF>::W;
   constexpr int R = RowsPerWarp<FF>::R;     // rows per warp
@@ -470,7 +468,7 @@ __global__ void __launch_bounds__(InvCfg<NF>::W * 32, 16 / InvCfg<NF>::W)
   };
   int64_t item = blockIdx.x;
   if (item < n_items) prefetch(item);
-  load_lane_twiddles<FF>(tws, twL);
+  load_lane_twiddles<FF>(tws, tw_lane);
   for (int k = threadIdx.x; k < 32 * FF; k += blockDim.x) twn[k] = twN[k];
   // warp w: slots w, w + kW, ...; slot s = (gg * NO + o) * 2 + side
   const int side = warp & 1, o = (warp >> 1) % NO, gp = (warp >> 1) / NO;
@@ -634,7 +632,7 @@ void launch_inv_pair_t(const sht_plan* p, int mode, const float* wP, const float
   const int64_t ctas = std::min<int64_t>(
       n_items, (int64_t)resident_ctas(fast_inverse_pair<FF, NF, TC>, kW * 32, sm) * sm_count());
   fast_inverse_pair<FF, NF, TC><<<(unsigned)ctas, kW * 32, sm, s>>>(
-      a, (const float2*)wP, (const float2*)(wD ? wD : wP), p->d_coslat, (const float2*)p->tw_l,
+      a, (const float2*)wP, (const float2*)(wD ? wD : wP), p->d_coslat, (const float2*)p->tw_lane,
       (const float2*)p->tw_n, out0, out1 ? out1 : out0, n_pb);
   SHT_CUDA_OR_THROW(cudaGetLastError());
 }
@@ -669,7 +667,7 @@ void launch_fwd_t(const sht_plan* p, const float* g0, const float* g1, int64_t p
   const int64_t wave = (int64_t)resident_ctas(fast_forward_fold<FF, W, TC>, W * 32, sm) * sm_count();
   a.pf_dist = kFwdPrefetch ? (int)div_up(wave, (int64_t)grid.x) : 0;
   fast_forward_fold<FF, W, TC><<<grid, W * 32, sm, s>>>(a, g0, g1 ? g1 : g0,
-                                                        (const float2*)p->tw_l,
+                                                        (const float2*)p->tw_lane,
                                                         (const float2*)p->tw_n, (float2*)wfold,
                                                         rowmax);
   SHT_CUDA_OR_THROW(cudaGetLastError());

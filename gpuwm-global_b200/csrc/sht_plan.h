@@ -58,6 +58,7 @@ struct sht_plan {
   // FFT: twiddles exp(-2 pi i k / L), k < L, and exp(-2 pi i k / N), k <= L.
   void* tw_l = nullptr;
   void* tw_n = nullptr;
+  void* tw_lane = nullptr;         // [k1][lane] table of the register kernels
   std::vector<int> radices;
   int* d_radices = nullptr;
   bool fast_fft = false;           // register-resident kernels (sht_fft_fast.cu)
