@@ -159,12 +159,13 @@ class LegendreTable(str):
         return (str, (str(self),))
 
 
-def _ptr(t: torch.Tensor):
-    return ctypes.c_void_p(t.data_ptr())
+def _ptr(t: torch.Tensor) -> int:
+    return t.data_ptr()
 
 
-def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+def _stream() -> int:
+    """The current stream of the current device, as the library takes it."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 class _FusedJob:
@@ -389,16 +390,16 @@ class SphericalHarmonicTransform:
     def _grid_in(self, field):
         f = self.backend.asarray(field, dtype=self.backend.float_dtype)
         self._validate_grid(f)
-        return f.contiguous()
+        return f if f.is_contiguous() else f.contiguous()
 
     def _spec_in(self, coeff):
         c = self.backend.asarray(coeff, dtype=self.backend.complex_dtype)
         self._validate_spectral(c)
-        return c.contiguous()
+        return c if c.is_contiguous() else c.contiguous()
 
     @staticmethod
     def _planes(t: torch.Tensor) -> int:
-        return int(np.prod(t.shape[:-2], dtype=np.int64)) if t.dim() > 2 else 1
+        return math.prod(t.shape[:-2])
 
     def _empty_grid(self, lead):
         return torch.empty((*lead, *self.grid.shape), dtype=self.backend.float_dtype,

@@ -4,7 +4,9 @@
 // failure leaves a thread-local message (sht_last_error).
 #include <cstdio>
 #include <exception>
+#include <map>
 #include <mutex>
+#include <tuple>
 
 #include "sht_plan.h"
 
@@ -33,6 +35,53 @@ namespace sht {
 static thread_local std::string g_error;
 void set_error(const std::string& msg) { g_error = msg; }
 void clear_error() { g_error.clear(); }
+
+namespace {
+
+// What the driver said, per process: entries are few (a kernel at the shared-
+// memory sizes of the plans in use) and the table is emptied if they are not.
+struct LaunchLimits {
+  std::mutex mu;
+  std::map<std::pair<const void*, int>, size_t> shared;                      // (kernel, device)
+  std::map<std::tuple<const void*, int, int, size_t>, int> resident;         // + threads, bytes
+};
+LaunchLimits& launch_limits() {
+  static LaunchLimits* l = new LaunchLimits;  // outlives every static destructor
+  return *l;
+}
+void raise_shared(LaunchLimits& l, const void* kernel, int dev, size_t bytes) {
+  size_t& have = l.shared[{kernel, dev}];
+  if (bytes <= have) return;
+  SHT_CUDA_OR_THROW(
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  have = bytes;
+}
+
+}  // namespace
+
+void allow_shared(const void* kernel, size_t bytes) {
+  int dev = 0;
+  SHT_CUDA_OR_THROW(cudaGetDevice(&dev));
+  LaunchLimits& l = launch_limits();
+  std::lock_guard<std::mutex> lock(l.mu);
+  raise_shared(l, kernel, dev, bytes);
+}
+
+int resident_ctas(const void* kernel, int threads, size_t bytes) {
+  int dev = 0;
+  SHT_CUDA_OR_THROW(cudaGetDevice(&dev));
+  LaunchLimits& l = launch_limits();
+  std::lock_guard<std::mutex> lock(l.mu);
+  const auto key = std::make_tuple(kernel, dev, threads, bytes);
+  const auto found = l.resident.find(key);
+  if (found != l.resident.end()) return found->second;
+  raise_shared(l, kernel, dev, bytes);
+  int per_sm = 0, sms = 0;
+  SHT_CUDA_OR_THROW(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, bytes));
+  SHT_CUDA_OR_THROW(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  if (l.resident.size() >= 4096) l.resident.clear();
+  return l.resident[key] = per_sm * sms;
+}
 
 namespace {
 

@@ -664,12 +664,6 @@ FftShape make_shape(const sht_plan* p, int64_t cols, int no, size_t* smem, int* 
   return f;
 }
 
-template <typename K>
-void allow_smem(K kernel, size_t bytes) {
-  SHT_CUDA_OR_THROW(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)std::max<size_t>(bytes, 48 * 1024)));
-}
-
 }  // namespace
 
 void build_fft(sht_plan* p, cudaStream_t s) {
@@ -723,7 +717,7 @@ void launch_forward_fold(const sht_plan* p, const T* g0, const T* g1, int64_t pl
   int threads = 0;
   const FftShape f = make_shape<T>(p, planes * fields, 1, &sm, &threads);
   const FoldArgs a{f, p->nlat, p->nlon, p->T, p->H, p->nlat_odd ? 1 : 0, fields, planes * fields, ldc};
-  allow_smem(forward_fold_kernel<T>, sm);
+  allow_shared((const void*)forward_fold_kernel<T>, sm);
   const dim3 grid((unsigned)div_up(a.cols, (int64_t)1 << f.lc), (unsigned)p->H);
   forward_fold_kernel<T><<<grid, threads, sm, s>>>(a, g0, g1 ? g1 : g0, (const V2<T>*)p->tw_l,
                                                    (const V2<T>*)p->tw_n, wfold, rowmax);
@@ -738,7 +732,7 @@ void launch_unfold(const sht_plan* p, int mode, const T* wP, const T* wD, int64_
   const FftShape f = make_shape<T>(p, planes, NF == 1 ? 1 : 2, &sm, &threads);
   const UnfoldArgs a{f, p->nlat, p->nlon, p->T, p->H, p->nlat_odd ? 1 : 0,
                      mode == kUnfoldZonal ? 1 : 0, planes, ldc, p->radius};
-  allow_smem(inverse_unfold_kernel<T, NF>, sm);
+  allow_shared((const void*)inverse_unfold_kernel<T, NF>, sm);
   const dim3 grid((unsigned)div_up(planes, (int64_t)1 << f.lc), (unsigned)p->H);
   inverse_unfold_kernel<T, NF><<<grid, threads, sm, s>>>(
       a, wP, wD ? wD : wP, p->d_coslat, (const V2<T>*)p->tw_l, (const V2<T>*)p->tw_n, out0,

@@ -597,22 +597,12 @@ __global__ void __launch_bounds__(InvCfg<NF>::W * 32, 16 / InvCfg<NF>::W)
   }
 }
 
-// SMs of the current device, and resident CTAs per SM of a kernel with the
-// given block and dynamic shared memory (the latter also raised to `sm`).
-int sm_count() {
-  int dev = 0, sms = 0;
-  SHT_CUDA_OR_THROW(cudaGetDevice(&dev));
-  SHT_CUDA_OR_THROW(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  return sms;
-}
+// resident_ctas of a kernel that has to fit.
 template <typename K>
-int resident_ctas(K kernel, int threads, size_t sm) {
-  SHT_CUDA_OR_THROW(
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  int per_sm = 0;
-  SHT_CUDA_OR_THROW(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, sm));
-  SHT_REQUIRE(per_sm > 0, "FFT kernel does not fit on an SM");
-  return per_sm;
+int64_t resident(K kernel, int threads, size_t sm) {
+  const int ctas = resident_ctas((const void*)kernel, threads, sm);
+  SHT_REQUIRE(ctas > 0, "FFT kernel does not fit on an SM");
+  return ctas;
 }
 
 // The waist rows must be 16-byte aligned for cp.async: an even column stride.
@@ -630,7 +620,7 @@ void launch_inv_pair_t(const sht_plan* p, int mode, const float* wP, const float
   const int64_t n_items = (int64_t)n_pb * p->H;
   if (n_items == 0) return;
   const int64_t ctas = std::min<int64_t>(
-      n_items, (int64_t)resident_ctas(fast_inverse_pair<FF, NF, TC>, kW * 32, sm) * sm_count());
+      n_items, resident(fast_inverse_pair<FF, NF, TC>, kW * 32, sm));
   fast_inverse_pair<FF, NF, TC><<<(unsigned)ctas, kW * 32, sm, s>>>(
       a, (const float2*)wP, (const float2*)(wD ? wD : wP), p->d_coslat, (const float2*)p->tw_lane,
       (const float2*)p->tw_n, out0, out1 ? out1 : out0, n_pb);
@@ -663,8 +653,8 @@ void launch_fwd_t(const sht_plan* p, const float* g0, const float* g1, int64_t p
   dim3 grid((unsigned)div_up(planes, a.G), (unsigned)p->H);
   const size_t sm = sizeof(float2) * (W * R * WarpSmem<FF>::kFloats2 + FF * 32 + p->T + 1);
   // One resident wave of CTAs, in latitude pairs (grid.x CTAs per pair);
-  // resident_ctas also raises the kernel's shared-memory limit to `sm`.
-  const int64_t wave = (int64_t)resident_ctas(fast_forward_fold<FF, W, TC>, W * 32, sm) * sm_count();
+  // resident() also raises the kernel's shared-memory limit to `sm`.
+  const int64_t wave = resident(fast_forward_fold<FF, W, TC>, W * 32, sm);
   a.pf_dist = kFwdPrefetch ? (int)div_up(wave, (int64_t)grid.x) : 0;
   fast_forward_fold<FF, W, TC><<<grid, W * 32, sm, s>>>(a, g0, g1 ? g1 : g0,
                                                         (const float2*)p->tw_lane,

@@ -353,8 +353,7 @@ void launch_simt(const SimtArgs<T>& a, int n_items, cudaStream_t s) {
   const size_t sm = sizeof(T) * C::S * C::BK * (tile_x<T>(WX) + tile_r<T>(C::G));
   const int64_t blocks = (int64_t)n_items * a.nrb * a.ng;
   SHT_REQUIRE(blocks < ((int64_t)1 << 31), "too many planes for one launch");
-  SHT_CUDA_OR_THROW(cudaFuncSetAttribute(gemm_simt_kernel<T, WX, DB>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  allow_shared((const void*)gemm_simt_kernel<T, WX, DB>, sm);
   gemm_simt_kernel<T, WX, DB><<<(unsigned)blocks, 32 * WX, sm, s>>>(a);
   SHT_CUDA_OR_THROW(cudaGetLastError());
 }

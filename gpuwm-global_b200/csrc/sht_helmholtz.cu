@@ -804,9 +804,6 @@ void launch_semi_implicit(const sht_plan* p, int nlev, const T* mats, bool has_t
               "unknown semi-implicit mode");
   SHT_REQUIRE(mode != kSemiHalf || has_thermo,
               "half_apply needs the thermodynamic block's modes (sht_vertical_create_modes)");
-  int dev = 0, sms = 0;
-  SHT_CUDA_OR_THROW(cudaGetDevice(&dev));
-  SHT_CUDA_OR_THROW(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const SemiArgs a{p->T, nlev, mode, p->radius, dt, alpha, ldc};
   // The stage solve by its own kernel while its operators and three vectors fit
   // an SM (FP32 to about 66 levels, FP64 to about 40); the general kernel keeps
@@ -814,15 +811,11 @@ void launch_semi_implicit(const sht_plan* p, int nlev, const T* mats, bool has_t
   int threads = 0;
   const size_t solve = solve_smem<T>(nlev, &threads);
   if (mode == kSemiSolve && threads <= 224 && solve + 2048 <= 227 * 1024) {
-    SHT_CUDA_OR_THROW(cudaFuncSetAttribute(semi_solve_kernel<T>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)solve));
-    int per_sm = 0;
-    SHT_CUDA_OR_THROW(
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, semi_solve_kernel<T>, threads, solve));
-    SHT_REQUIRE(per_sm > 0, "semi-implicit solve does not fit on an SM at this nlev");
+    const int fit = resident_ctas((const void*)semi_solve_kernel<T>, threads, solve);
+    SHT_REQUIRE(fit > 0, "semi-implicit solve does not fit on an SM at this nlev");
     const int64_t nmb = div_up(p->T + 1, 32);
     const int64_t items = div_up(nmb * (p->T + 1) - 16 * nmb * (nmb - 1), 2);
-    const int ctas = (int)std::min<int64_t>(items, (int64_t)per_sm * sms);
+    const int ctas = (int)std::min<int64_t>(items, fit);
     semi_solve_kernel<T><<<ctas, threads, solve, s>>>(
         a, mats, (const V2<T>*)div, (const V2<T>*)theta, (const V2<T>*)lnps, (V2<T>*)odiv,
         (V2<T>*)otheta, (V2<T>*)olnps, metric, (V2<T>*)cfold, rowmax);
@@ -831,14 +824,10 @@ void launch_semi_implicit(const sht_plan* p, int nlev, const T* mats, bool has_t
   }
   const SmemPlan sp = smem_plan(nlev, mode);
   const size_t sm = sizeof(T) * (size_t)sp.nmat + sizeof(V2<T>) * 32 * (size_t)(sp.nvec * sp.vp);
-  SHT_CUDA_OR_THROW(cudaFuncSetAttribute(semi_implicit_kernel<T>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  int per_sm = 0;
-  SHT_CUDA_OR_THROW(
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, semi_implicit_kernel<T>, 256, sm));
-  SHT_REQUIRE(per_sm > 0, "semi-implicit kernel does not fit on an SM at this nlev");
+  const int fit = resident_ctas((const void*)semi_implicit_kernel<T>, 256, sm);
+  SHT_REQUIRE(fit > 0, "semi-implicit kernel does not fit on an SM at this nlev");
   const int64_t items = div_up(p->T + 1, 32) * (int64_t)(p->T + 1);
-  const int ctas = (int)std::min<int64_t>(items, (int64_t)per_sm * sms);
+  const int ctas = (int)std::min<int64_t>(items, fit);
   semi_implicit_kernel<T><<<ctas, dim3(32, 8), sm, s>>>(
       a, mats, (const V2<T>*)div, (const V2<T>*)theta, (const V2<T>*)lnps, (V2<T>*)odiv,
       (V2<T>*)otheta, (V2<T>*)olnps, metric, (V2<T>*)cfold, rowmax);

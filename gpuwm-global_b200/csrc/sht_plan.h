@@ -120,6 +120,15 @@ struct sht_plan {
 
 namespace sht {
 
+// Raises a kernel's dynamic shared-memory limit on the current device to at
+// least `bytes`; the driver is asked only when the limit grows.
+void allow_shared(const void* kernel, size_t bytes);
+// CTAs of the kernel resident on the whole current device (SMs x CTAs per SM)
+// at the given block and dynamic shared memory, its limit raised to `bytes`;
+// 0 if it does not fit.  Asked of the driver once per set of arguments (the two
+// queries and the limit cost about 3 us a launch, T21's transforms take 20).
+int resident_ctas(const void* kernel, int threads, size_t bytes);
+
 // The scratch operands (wfold, cfold) hold one complex column per (plane,
 // field), columns innermost; `ldc` is their column stride.  The plan's own
 // scratch pads an odd count by one column (which nothing reads as a result),
