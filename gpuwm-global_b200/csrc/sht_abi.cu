@@ -276,6 +276,11 @@ void do_forward(sht_plan* p, const T* grid, int64_t planes, T* coeff, cudaStream
     KernelScope k(p, SHT_KIND_FFT_FORWARD, s);
     launch_forward_fold<T>(p, grid, nullptr, planes, ldc, w, s, rm);
   }
+  if (!uses_tc(p) && simt_takes_coefficients(p, R)) {
+    KernelScope k(p, SHT_KIND_LEGENDRE_ANALYSIS, s);
+    launch_simt_to_coefficients<T>(p, static_cast<const T*>(p->analysis), w, coeff, planes, R, s);
+    return;
+  }
   contract<T>(p, kAnalysis, w, c, R, s);
   {
     KernelScope k(p, SHT_KIND_UNPACK, s);
@@ -283,43 +288,57 @@ void do_forward(sht_plan* p, const T* grid, int64_t planes, T* coeff, cudaStream
   }
 }
 
+// The contractions of one or two tables (kind1 < 0: one) from coefficients:
+// packed first, or read in place at few rows.
 template <typename T>
-void do_synthesis(sht_plan* p, int kind, int mode, const T* coeff, int64_t planes, T* grid,
-                  cudaStream_t s) {
-  const int64_t ldc = padded_cols(planes), R = 2 * ldc;
-  ensure_scratch(p, R);
-  T* w = static_cast<T*>(p->wfold[0]);
+void synthesize(sht_plan* p, int kind0, int kind1, const T* coeff, int64_t planes, int64_t ldc,
+                cudaStream_t s) {
+  const int64_t R = 2 * ldc;
   T* c = static_cast<T*>(p->cfold[0]);
+  T* w[2] = {static_cast<T*>(p->wfold[0]), static_cast<T*>(p->wfold[1])};
+  if (!uses_tc(p) && simt_takes_coefficients(p, R)) {
+    KernelScope k(p, SHT_KIND_LEGENDRE_SYNTHESIS, s);
+    const int n = kind1 < 0 ? 1 : 2, kinds[2] = {kind0, kind1};
+    int flip[2] = {};
+    const T* table[2] = {};
+    for (int g = 0; g < n; ++g) {
+      flip[g] = table_flip(kinds[g]);
+      table[g] = static_cast<const T*>(table_ptr(p, kinds[g]));
+    }
+    launch_simt_from_coefficients<T>(p, n, flip, table, coeff, planes, w, R, s);
+    return;
+  }
   {
     float* rm = rowmax_for(p, R, s);
     KernelScope k(p, SHT_KIND_PACK, s);
     launch_pack<T>(p, coeff, nullptr, planes, ldc, kPackPlain, c, s, rm);
   }
-  contract<T>(p, kind, c, w, R, s);
-  {
-    KernelScope k(p, SHT_KIND_FFT_INVERSE, s);
-    launch_inverse_unfold<T>(p, mode, w, nullptr, planes, ldc, grid, nullptr, s);
-  }
+  if (kind1 < 0)
+    contract<T>(p, kind0, c, w[0], R, s);
+  else
+    contract2<T>(p, kind0, w[0], kind1, w[1], c, R, s);
+}
+
+template <typename T>
+void do_synthesis(sht_plan* p, int kind, int mode, const T* coeff, int64_t planes, T* grid,
+                  cudaStream_t s) {
+  const int64_t ldc = padded_cols(planes);
+  ensure_scratch(p, 2 * ldc);
+  synthesize<T>(p, kind, -1, coeff, planes, ldc, s);
+  KernelScope k(p, SHT_KIND_FFT_INVERSE, s);
+  launch_inverse_unfold<T>(p, mode, static_cast<const T*>(p->wfold[0]), nullptr, planes, ldc, grid,
+                           nullptr, s);
 }
 
 template <typename T>
 void do_gradient(sht_plan* p, const T* coeff, int64_t planes, T* east, T* north,
                  cudaStream_t s) {
-  const int64_t ldc = padded_cols(planes), R = 2 * ldc;
-  ensure_scratch(p, R);
-  T* c = static_cast<T*>(p->cfold[0]);
-  T* w0 = static_cast<T*>(p->wfold[0]);
-  T* w1 = static_cast<T*>(p->wfold[1]);
-  {
-    float* rm = rowmax_for(p, R, s);
-    KernelScope k(p, SHT_KIND_PACK, s);
-    launch_pack<T>(p, coeff, nullptr, planes, ldc, kPackPlain, c, s, rm);
-  }
-  contract2<T>(p, kBasis, w0, kDBasis, w1, c, R, s);
-  {
-    KernelScope k(p, SHT_KIND_FFT_INVERSE, s);
-    launch_inverse_unfold<T>(p, kUnfoldGradient, w0, w1, planes, ldc, east, north, s);
-  }
+  const int64_t ldc = padded_cols(planes);
+  ensure_scratch(p, 2 * ldc);
+  synthesize<T>(p, kBasis, kDBasis, coeff, planes, ldc, s);
+  KernelScope k(p, SHT_KIND_FFT_INVERSE, s);
+  launch_inverse_unfold<T>(p, kUnfoldGradient, static_cast<const T*>(p->wfold[0]),
+                           static_cast<const T*>(p->wfold[1]), planes, ldc, east, north, s);
 }
 
 template <typename T>

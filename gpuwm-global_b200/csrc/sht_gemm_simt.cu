@@ -56,6 +56,8 @@ template <typename T> struct SimtArgs {
   int nrb;     // row blocks of tile_r(G)
   bool half;   // the last one holds at most tile_r(1) rows
   int64_t R;
+  int Tn;          // truncation and planes of a spectral side taken in place
+  int64_t planes;
 };
 
 template <int BYTES>
@@ -225,7 +227,19 @@ __global__ void __launch_bounds__(32 * WX, 16 / WX) gemm_simt_kernel(const __gri
 // planes FP32 (8 rows), both contractions, 45 us less of a 136 us pair (four
 // columns to a lane: 22 us more); the P and dP/dphi syntheses of one T255 plane
 // 44 -> 28 us; T21 x 1 plane 7.4 -> 6.0 us.
-template <typename T, int RR>
+//
+// The transforms' own calls take the spectral side in place, too: with CPACK the
+// data rows are read from the coefficients [plane][n][m] (the pack pass's
+// layout change is nothing for values that a whole warp shares), with CUNPACK
+// the outputs go to them, real at m = 0, and the block of parity 0 zeroes its
+// order above the triangle.  T21 x 1 plane FP32, the pair: 36.3 us with the two
+// layout passes, 32.2 us without; forward, inverse and gradient of one to four
+// planes at T62 FP32: 78-82 us and 67-75.  Below T128 and R * T of 512: past it
+// the strided reads cost more than the passes (T106 x 4 planes 93 and 95 us,
+// T126 x 4 97 and 105, T170 x 1 or 2 the same both ways, T255's gradient of
+// one plane 4 us more).
+enum SkinnySpectral { kFolded = 0, kCPack = 1, kCUnpack = 2 };
+template <typename T, int RR, int SPEC>
 __global__ void __launch_bounds__(128) gemm_skinny_kernel(const __grid_constant__ SimtArgs<T> a) {
   constexpr int U = 16 * 4 / (RR * (int)sizeof(T) / 4);
   unsigned b = blockIdx.x;
@@ -235,19 +249,30 @@ __global__ void __launch_bounds__(128) gemm_skinny_kernel(const __grid_constant_
   const ShtGemmDesc d = grp.descs[it.problem];
   const int R = (int)a.R;
   const int x = it.x0 + (int)threadIdx.x;
-  if (x >= d.X) return;
   using Q = std::conditional_t<sizeof(T) == 4, float2, double2>;  // two rows
+  const int64_t t1 = a.Tn + 1;
+  const int n0 = d.m + (it.problem & 1);  // degree of the problem's first coefficient
+  if constexpr (SPEC == kCUnpack) {
+    if ((it.problem & 1) == 0 && it.x0 == 0)
+      for (int64_t p = 0; p < a.planes; ++p)
+        for (int n = threadIdx.x; n < d.m; n += blockDim.x)
+          reinterpret_cast<Q*>(grp.out)[(p * t1 + n) * t1 + d.m] = Q{};
+  }
+  if (x >= d.X) return;
   const T* tab = grp.table + d.t_off + x;
   const T* dat = grp.data + d.d_row * a.R;
   T acc[RR];
 #pragma unroll
   for (int r = 0; r < RR; ++r) acc[r] = T(0);
   auto step = [&](int k, T t) {
-    const Q* p = reinterpret_cast<const Q*>(dat + (int64_t)k * R);
+    const Q* p = SPEC == kCPack
+                     ? reinterpret_cast<const Q*>(grp.data) + (n0 + 2 * k) * t1 + d.m
+                     : reinterpret_cast<const Q*>(dat + (int64_t)k * R);
+    const int64_t ld = SPEC == kCPack ? t1 * t1 : 1;
 #pragma unroll
     for (int r = 0; r < RR; r += 2)
-      if (r < R) {
-        const Q q = __ldg(p + r / 2);
+      if (SPEC == kCPack ? r < 2 * a.planes : r < R) {
+        const Q q = __ldg(p + r / 2 * ld);
         acc[r] = fma(t, q.x, acc[r]);
         acc[r + 1] = fma(t, q.y, acc[r + 1]);
       }
@@ -261,15 +286,19 @@ __global__ void __launch_bounds__(128) gemm_skinny_kernel(const __grid_constant_
     for (int u = 0; u < U; ++u) step(k + u, t[u]);
   }
   for (; k < d.K; ++k) step(k, __ldg(tab + (int64_t)k * d.ldt));
-  T* o = grp.out + (d.c_row + x) * a.R;
 #pragma unroll
-  for (int r = 0; r < RR; r += 2)
-    if (r < R) {
-      Q q;
-      q.x = acc[r];
-      q.y = acc[r + 1];
-      *reinterpret_cast<Q*>(o + r) = q;
+  for (int r = 0; r < RR; r += 2) {
+    Q q;
+    q.x = acc[r];
+    q.y = acc[r + 1];
+    if constexpr (SPEC == kCUnpack) {
+      if (d.m == 0) q.y = T(0);
+      if (r < 2 * a.planes)
+        reinterpret_cast<Q*>(grp.out)[(r / 2 * t1 + n0 + 2 * x) * t1 + d.m] = q;
+    } else if (r < R) {
+      *reinterpret_cast<Q*>(grp.out + (d.c_row + x) * a.R + r) = q;
     }
+  }
 }
 
 }  // namespace
@@ -360,6 +389,51 @@ void launch_simt(const SimtArgs<T>& a, int n_items, cudaStream_t s) {
 
 }  // namespace
 
+namespace {
+
+template <typename T, int SPEC>
+void launch_skinny(const SimtArgs<T>& a, int n_items, cudaStream_t s) {
+  const unsigned blocks = (unsigned)n_items * (unsigned)a.ng, threads = tile_x<T>(4);
+  if (a.R <= 4)
+    gemm_skinny_kernel<T, 4, SPEC><<<blocks, threads, 0, s>>>(a);
+  else
+    gemm_skinny_kernel<T, 8, SPEC><<<blocks, threads, 0, s>>>(a);
+  SHT_CUDA_OR_THROW(cudaGetLastError());
+}
+
+}  // namespace
+
+bool simt_takes_coefficients(const sht_plan* p, int64_t R) {
+  return R <= 8 && p->T < 128 && R * p->T <= 512;
+}
+
+template <typename T>
+void launch_simt_from_coefficients(const sht_plan* p, int ngroups, const int* flip,
+                                   const T* const* table, const T* coeff, int64_t planes,
+                                   T* const* wfold, int64_t R, cudaStream_t s) {
+  SimtArgs<T> a{};
+  for (int g = 0; g < ngroups; ++g) a.g[g] = {p->d_desc[0][flip[g]], table[g], coeff, wfold[g]};
+  a.items = p->d_items[0];
+  a.ng = ngroups;
+  a.R = R;
+  a.Tn = p->T;
+  a.planes = planes;
+  launch_skinny<T, kCPack>(a, p->n_items[0], s);
+}
+
+template <typename T>
+void launch_simt_to_coefficients(const sht_plan* p, const T* table, const T* wfold, T* coeff,
+                                 int64_t planes, int64_t R, cudaStream_t s) {
+  SimtArgs<T> a{};
+  a.g[0] = {p->d_desc[1][0], table, wfold, coeff};
+  a.items = p->d_items[1];
+  a.ng = 1;
+  a.R = R;
+  a.Tn = p->T;
+  a.planes = planes;
+  launch_skinny<T, kCUnpack>(a, p->n_items[1], s);
+}
+
 template <typename T>
 void launch_gemm_simt_groups(const sht_plan* p, int direction, int ngroups, const int* flip,
                              const T* const* table, const T* const* data, T* const* out,
@@ -382,12 +456,7 @@ void launch_gemm_simt_groups(const sht_plan* p, int direction, int ngroups, cons
   a.ng = ngroups;
   a.R = R;
   if (skinny) {
-    const unsigned blocks = (unsigned)n_items * (unsigned)ngroups, threads = tile_x<T>(4);
-    if (R <= 4)
-      gemm_skinny_kernel<T, 4><<<blocks, threads, 0, s>>>(a);
-    else
-      gemm_skinny_kernel<T, 8><<<blocks, threads, 0, s>>>(a);
-    SHT_CUDA_OR_THROW(cudaGetLastError());
+    launch_skinny<T, kFolded>(a, n_items, s);
     return;
   }
   const int whole = tile_r<T>(SimtCfg<T>::G);
@@ -414,6 +483,15 @@ template void launch_gemm_simt<float>(const sht_plan*, int, int, const float*, c
                                       float*, int64_t, cudaStream_t);
 template void launch_gemm_simt<double>(const sht_plan*, int, int, const double*, const double*,
                                        double*, int64_t, cudaStream_t);
+#define INST(T)                                                                                  \
+  template void launch_simt_from_coefficients<T>(const sht_plan*, int, const int*,              \
+                                                 const T* const*, const T*, int64_t, T* const*, \
+                                                 int64_t, cudaStream_t);                        \
+  template void launch_simt_to_coefficients<T>(const sht_plan*, const T*, const T*, T*, int64_t, \
+                                               int64_t, cudaStream_t);
+INST(float)
+INST(double)
+#undef INST
 template void launch_gemm_simt_groups<float>(const sht_plan*, int, int, const int*,
                                              const float* const*, const float* const*,
                                              float* const*, int64_t, cudaStream_t);
