@@ -25,11 +25,11 @@
 // their row scales come from the row maxima the producing kernel (the
 // longitude FFT or the pack kernel) merged while writing the operand.
 //
-// Roles (576 threads, one CTA per SM, persistent over a cost-sorted tile list
+// Roles (608 threads, one CTA per SM, persistent over a cost-sorted tile list
 // that may merge several contractions: the P and dP/dphi tables of a
 // gradient or wind synthesis, or the plans of a batch):
 //   warp 0      bulk-copy loader for the table stages; owns TMEM alloc/free
-//   warp 1      MMA issuer (one thread)
+//   warp 1      MMA issuer (one elected lane)
 //   warps 2-9   epilogue: tcgen05.ld of the accumulators, unscale, release
 //               the accumulators, store the tile to global memory
 //   warps 10-17 converters for the data operand (into shared memory, or into
@@ -212,6 +212,11 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
       " [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)),
       "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar))
       : "memory");
+}
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+  return one != 0;
 }
 __device__ __forceinline__ void fence_proxy_async() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -419,7 +424,7 @@ __device__ bool wait_bar(uint64_t* bar, uint32_t parity, const Pipe& pp, unsigne
   return true;
 }
 
-// 576 threads = 18 warps, 5 on the busiest of the four SM sub-partitions,
+// 608 threads = 19 warps, 5 on the busiest of the four SM sub-partitions,
 // whose 16 384 registers cap a thread at 96.
 template <typename Acc>
 __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_constant__ TcArgs a) {
@@ -445,7 +450,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
           bars + 2 * NA + 3 * S + 2 * kMaxNBuf + 1,
           abort_flag};
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < NA; ++s) {
       mbar_init(&pp.full_a[s], kConvThreads);
@@ -502,31 +507,35 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
 
   if (warp == 0) {
     // ------------------------------------------------------------ loader
-    if (lane == 0) {
+    // The whole warp walks the loop and one elected lane issues, as in the
+    // MMA warp: the copy's operands are warp-uniform values.
+    {
+      const bool leader = elect_one();
       int stage = 0;
       uint32_t phase = 0;
-      int armed[S];
-#pragma unroll
-      for (int s = 0; s < S; ++s) armed[s] = -1;
-      for (int k = 0; k < my_tiles && !*abort_flag; ++k) {
+      uint32_t armed = 0, armed_phase = 0;  // bit per stage: copied to; parity of the last copy
+      for (int k = 0; k < my_tiles; ++k) {
         const ShtTcTile tl = tile_k(k);
-        if (reject_tile(tl, abort_flag, a.err)) break;
+        if (__any_sync(0xffffffffu, *abort_flag || reject_tile(tl, abort_flag, a.err))) break;
         const TcGroup& G = a.g[tl.group];
-        const int part = tl.nsize * BK * 2;  // bytes of one FP16 part of one stage
-        const unsigned char* src = G.img + tl.img;
+        const int kst = __shfl_sync(0xffffffffu, tl.kst, 0);
+        // bytes of one stage: both FP16 parts
+        const int part = __shfl_sync(0xffffffffu, NPARTS * tl.nsize * BK * 2, 0);
+        const unsigned char* src = reinterpret_cast<const unsigned char*>(
+            __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(G.img + tl.img), 0));
         bool ok = true;
-        for (int ks = 0; ks < tl.kst; ++ks) {
-          if (!wait_bar(&pp.empty[stage], phase ^ 1, pp, a.err, 1)) {
+        for (int ks = 0; ks < kst; ++ks) {
+          if (!__all_sync(0xffffffffu, wait_fast(&pp.empty[stage], phase ^ 1, pp, a.err, 1))) {
             ok = false;
             break;
           }
-          mbar_arrive_expect_tx(&pp.full_b[stage], NPARTS * part);
-          unsigned char* dst = sB + stage * NPARTS * kBPart;
-#pragma unroll
-          for (int pt = 0; pt < NPARTS; ++pt)
-            bulk_g2s(dst + pt * kBPart, src + ((int64_t)ks * NPARTS + pt) * part, part,
-                     &pp.full_b[stage]);
-          armed[stage] = (int)phase;
+          if (leader) {
+            mbar_arrive_expect_tx(&pp.full_b[stage], part);
+            bulk_g2s(sB + stage * NPARTS * kBPart, src, part, &pp.full_b[stage]);
+          }
+          src += part;
+          armed |= 1u << stage;
+          armed_phase = (armed_phase & ~(1u << stage)) | phase << stage;
           if (++stage == S) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
@@ -536,10 +545,11 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
       // this wait is what keeps a late copy from writing freed shared memory).
       for (int s = 0; s < S; ++s) {
         long long t0 = clock64();
-        if (armed[s] >= 0)
-          while (!mbar_try_wait(&pp.full_b[s], (uint32_t)armed[s]) && clock64() - t0 < kWaitBudget) {
+        if (armed >> s & 1)
+          while (!mbar_try_wait(&pp.full_b[s], armed_phase >> s & 1) && clock64() - t0 < kWaitBudget) {
           }
       }
+      __syncwarp();
     }
   } else if (warp == kRawWarp) {
     // ---------------------------------------------------- data-tile loader
@@ -548,31 +558,34 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
     // its stage finish): the data runs up to S stages ahead of the converted
     // operand ring, which is what keeps the tensor pipe fed across the
     // memory latency.
-    if (lane == 0) {
+    {
+      const bool leader = elect_one();
       int stage = 0;
       uint32_t phase = 0;
-      int armed[S];
-#pragma unroll
-      for (int s = 0; s < S; ++s) armed[s] = -1;
-      for (int k = 0; k < my_tiles && !*abort_flag; ++k) {
+      uint32_t armed = 0, armed_phase = 0;  // bit per stage: copied to; parity of the last copy
+      for (int k = 0; k < my_tiles; ++k) {
         const ShtTcTile tl = tile_k(k);
-        if (reject_tile(tl, abort_flag, a.err)) break;
-        const TcGroup& G = a.g[tl.group];
+        if (__any_sync(0xffffffffu, *abort_flag || reject_tile(tl, abort_flag, a.err))) break;
+        const TcGroup& G = a.g[__shfl_sync(0xffffffffu, tl.group, 0)];
+        const int kst = __shfl_sync(0xffffffffu, tl.kst, 0), r0 = __shfl_sync(0xffffffffu, tl.r0, 0);
+        int row = __shfl_sync(0xffffffffu, (int)tl.d_row, 0);
         bool ok = true;
-        for (int ks = 0; ks < tl.kst; ++ks) {
-          if (!wait_bar(&pp.raw_empty[stage], phase ^ 1, pp, a.err, 9)) {
+        for (int ks = 0; ks < kst; ++ks, row += BK) {
+          if (!__all_sync(0xffffffffu, wait_fast(&pp.raw_empty[stage], phase ^ 1, pp, a.err, 9))) {
             ok = false;
             break;
           }
           // Rows r0 .. r0+127 as four 32-row boxes, contraction rows
           // d_row + ks*BK .. +BK-1.
-          mbar_arrive_expect_tx(&pp.full_raw[stage], kRawStage);
-          unsigned char* raw = sRaw + stage * kRawStage;
+          if (leader) {
+            mbar_arrive_expect_tx(&pp.full_raw[stage], kRawStage);
+            unsigned char* raw = sRaw + stage * kRawStage;
 #pragma unroll
-          for (int q = 0; q < BM / 32; ++q)
-            tma_load_2d(raw + q * kRawBox, &G.data_map, tl.r0 + 32 * q,
-                        (int)(tl.d_row + (int64_t)ks * BK), &pp.full_raw[stage]);
-          armed[stage] = (int)phase;
+            for (int q = 0; q < BM / 32; ++q)
+              tma_load_2d(raw + q * kRawBox, &G.data_map, r0 + 32 * q, row, &pp.full_raw[stage]);
+          }
+          armed |= 1u << stage;
+          armed_phase = (armed_phase & ~(1u << stage)) | phase << stage;
           if (++stage == S) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
@@ -581,96 +594,109 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
       // this wait keeps a late copy from writing freed shared memory).
       for (int s = 0; s < S; ++s) {
         long long t0 = clock64();
-        if (armed[s] >= 0)
-          while (!mbar_try_wait(&pp.full_raw[s], (uint32_t)armed[s]) && clock64() - t0 < kWaitBudget) {
+        if (armed >> s & 1)
+          while (!mbar_try_wait(&pp.full_raw[s], armed_phase >> s & 1) && clock64() - t0 < kWaitBudget) {
           }
       }
+      __syncwarp();
     }
   } else if (warp == 1) {
     // --------------------------------------------------------------- MMA
-    if (lane == 0) {
-      int stage = 0;  // shared stage (table; data when !A_TMEM)
-      uint32_t phase = 0;
-      int aslot = 0;  // TMEM data slot (A_TMEM)
-      uint32_t aphase = 0;
-      uint32_t acc_it = 0;  // accumulator set = acc_it % NBUF, parity = (acc_it / NBUF) & 1
-      bool issued = false;
-      for (int k = 0; k < my_tiles && !*abort_flag; ++k) {
-        const ShtTcTile tl = tile_k(k);
-        if (reject_tile(tl, abort_flag, a.err)) break;
-        if (tl.kst == 0) continue;
-        const uint32_t buf = acc_it % NBUF, acc_phase = (acc_it / NBUF) & 1;
-        if (!wait_bar(&pp.acc_empty[buf], acc_phase ^ 1, pp, a.err, 2)) break;
-        const uint32_t d_set = tmem_base + buf * kAccCols;
-        const uint32_t d_corr = d_set + NMAIN * NMAX;
+    // The whole warp walks the loop and one elected lane issues: descriptors,
+    // flags and addresses are then warp-uniform values, where a single-lane
+    // loop moved every operand of every MMA from vector registers and spent
+    // about 700 cycles a stage on it, more than its MMAs (384) or any other
+    // role (with the copies, the conversion and the stores all taken out a
+    // launch still took two thirds of its time).  T511 x 200 planes: analysis
+    // 325 -> 271 us, synthesis 356 -> 334, 268 and 330 with both loaders alike.
+    const bool leader = elect_one();
+    int stage = 0;  // shared stage (table; data when !A_TMEM)
+    uint32_t phase = 0;
+    int aslot = 0;  // TMEM data slot (A_TMEM)
+    uint32_t aphase = 0;
+    uint32_t acc_it = 0;  // accumulator set = acc_it % NBUF, parity = (acc_it / NBUF) & 1
+    bool issued = false;
+    const uint64_t da_base = smem_desc(smem_u32(sA), kALbo, 128);
+    // Every exit is a vote, so the warp stays together.
+    for (int k = 0; k < my_tiles; ++k) {
+      const ShtTcTile tl = tile_k(k);
+      if (__any_sync(0xffffffffu, *abort_flag || reject_tile(tl, abort_flag, a.err))) break;
+      const int kst = __shfl_sync(0xffffffffu, tl.kst, 0), nsize = __shfl_sync(0xffffffffu, tl.nsize, 0);
+      if (kst == 0) continue;
+      const uint32_t buf = acc_it % NBUF, acc_phase = (acc_it / NBUF) & 1;
+      if (!__all_sync(0xffffffffu, wait_fast(&pp.acc_empty[buf], acc_phase ^ 1, pp, a.err, 2))) break;
+      const uint32_t d_set = tmem_base + buf * kAccCols;
+      const uint32_t d_corr = d_set + NMAIN * NMAX;
+      tc_fence_after();
+      // A from TMEM is K-major (no transpose bit).
+      const uint32_t idesc = Acc::A_TMEM ? instr_desc(nsize) & ~(1u << 15) : instr_desc(nsize);
+      const uint32_t lbo_b = (uint32_t)nsize * 16;
+      const uint64_t db_base = smem_desc(smem_u32(sB), lbo_b, 128);
+      const uint32_t part_b = (uint32_t)nsize * (BK * 2 / 16);  // the lo part follows the hi part
+      const int nsteps = kst * (BK / 16);  // K steps of 16 in the tile
+      // Main segment of step k: floor(k * NMAIN / nsteps), so the segments
+      // start at steps 0, b1 and b2.
+      const int b1 = NMAIN > 1 ? (nsteps + NMAIN - 1) / NMAIN : nsteps;
+      const int b2 = NMAIN > 2 ? (2 * nsteps + NMAIN - 1) / NMAIN : nsteps;
+      uint32_t d_main = d_set;
+      bool ok = true;
+      for (int ks = 0; ks < kst; ++ks) {
+        const bool landed = wait_fast(Acc::A_TMEM ? &pp.full_a[aslot] : &pp.full_a[stage],
+                                      Acc::A_TMEM ? aphase : phase, pp, a.err, 3) &&
+                            wait_fast(&pp.full_b[stage], phase, pp, a.err, 4);
+        if (!__all_sync(0xffffffffu, landed)) {
+          ok = false;
+          break;
+        }
         tc_fence_after();
-        // A from TMEM is K-major (no transpose bit).
-        const uint32_t idesc = Acc::A_TMEM ? instr_desc(tl.nsize) & ~(1u << 15) : instr_desc(tl.nsize);
-        const uint32_t lbo_b = (uint32_t)tl.nsize * 16;
-        const int nsteps = tl.kst * (BK / 16);  // K steps of 16 in the tile
-        // Segment of step k: floor(k * NMAIN / nsteps), advanced at the
-        // boundaries ceil(s * nsteps / NMAIN) instead of divided per step.
-        int seg = 0, seg_prev = -1;
-        int next_b = NMAIN > 1 ? (nsteps + NMAIN - 1) / NMAIN : nsteps;
-        bool ok = true;
-        for (int ks = 0; ks < tl.kst; ++ks) {
-          if (!wait_fast(Acc::A_TMEM ? &pp.full_a[aslot] : &pp.full_a[stage],
-                         Acc::A_TMEM ? aphase : phase, pp, a.err, 3) ||
-              !wait_fast(&pp.full_b[stage], phase, pp, a.err, 4)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          // Descriptors of the stage's operands; a K step of 16 (two K groups
-          // of 8) advances the start-address field by 2 LBO / 16.
-          const uint64_t da0 = smem_desc(smem_u32(sA + stage * NPARTS * kAPart), kALbo, 128);
-          const uint64_t db0 = smem_desc(smem_u32(sB + stage * NPARTS * kBPart), lbo_b, 128);
+        // Descriptors of the stage's operands; a K step of 16 (two K groups
+        // of 8) advances the start-address field by 2 LBO / 16.
+        const uint64_t da0 = da_base + (uint32_t)(stage * (NPARTS * kAPart / 16));
+        const uint64_t db0 = db_base + (uint32_t)(stage * (NPARTS * kBPart / 16));
 #pragma unroll
-          for (int j = 0; j < BK / 16; ++j) {
-            const uint64_t da1 = da0 + (uint64_t)(j * 2 * kALbo / 16);
-            const uint64_t da2 = da1 + (uint64_t)(kAPart / 16);
-            const uint64_t db1 = db0 + (uint64_t)(j * 2 * lbo_b / 16);
-            const uint64_t db2 = db1 + (uint64_t)(kBPart / 16);
-            const int step = ks * (BK / 16) + j;
-            if (step >= next_b && seg < NMAIN - 1) {  // contiguous thirds of the K steps
-              ++seg;
-              next_b = ((seg + 1) * nsteps + NMAIN - 1) / NMAIN;
-            }
-            const uint32_t accum_main = seg == seg_prev ? 1u : 0u;
-            seg_prev = seg;
-            const uint32_t accum_corr = step > 0 ? 1u : 0u;
+        for (int j = 0; j < BK / 16; ++j) {
+          const int step = ks * (BK / 16) + j;
+          const bool first = step == 0 || step == b1 || step == b2;  // of its segment
+          if (first && step > 0) d_main += NMAX;
+          const uint32_t accum_main = first ? 0u : 1u, accum_corr = step > 0 ? 1u : 0u;
+          const uint64_t da1 = da0 + (uint64_t)(j * 2 * kALbo / 16);
+          const uint64_t da2 = da1 + (uint64_t)(kAPart / 16);
+          const uint64_t db1 = db0 + (uint64_t)(j * 2 * lbo_b / 16);
+          const uint64_t db2 = db1 + (uint64_t)part_b;
+          if (leader) {
             if constexpr (Acc::A_TMEM) {
               const uint32_t ta1 = tmem_base + (uint32_t)(Acc::kATmem + aslot * 32 + j * 8);
               const uint32_t ta2 = ta1 + 16;
-              mma_f16_ts(d_set + (uint32_t)(seg * NMAX), ta1, db1, idesc, accum_main);  // a1 b1
-              mma_f16_ts(d_corr, ta1, db2, idesc, accum_corr);                              // a1 b2
-              mma_f16_ts(d_corr, ta2, db1, idesc, 1u);                                      // a2 b1
+              mma_f16_ts(d_main, ta1, db1, idesc, accum_main);  // a1 b1
+              mma_f16_ts(d_corr, ta1, db2, idesc, accum_corr);  // a1 b2
+              mma_f16_ts(d_corr, ta2, db1, idesc, 1u);          // a2 b1
             } else {
-              mma_f16(d_set + (uint32_t)(seg * NMAX), da1, db1, idesc, accum_main);  // a1 b1
-              mma_f16(d_corr, da1, db2, idesc, accum_corr);                              // a1 b2
-              mma_f16(d_corr, da2, db1, idesc, 1u);                                      // a2 b1
+              mma_f16(d_main, da1, db1, idesc, accum_main);  // a1 b1
+              mma_f16(d_corr, da1, db2, idesc, accum_corr);  // a1 b2
+              mma_f16(d_corr, da2, db1, idesc, 1u);          // a2 b1
             }
           }
-          issued = true;
-          mma_commit(&pp.empty[stage]);  // frees the stage when these MMAs finish
-          if (++stage == S) { stage = 0; phase ^= 1; }
-          if constexpr (Acc::A_TMEM) {
-            mma_commit(&pp.a_empty[aslot]);  // and the TMEM data slot
-            if (++aslot == NA) { aslot = 0; aphase ^= 1; }
-          }
         }
-        if (!ok) break;
-        mma_commit(&pp.acc_full[buf]);
-        ++acc_it;
+        issued = true;
+        if (leader) mma_commit(&pp.empty[stage]);  // frees the stage when these MMAs finish
+        if (++stage == S) { stage = 0; phase ^= 1; }
+        if constexpr (Acc::A_TMEM) {
+          if (leader) mma_commit(&pp.a_empty[aslot]);  // and the TMEM data slot
+          if (++aslot == NA) { aslot = 0; aphase ^= 1; }
+        }
       }
-      if (issued) {
-        // All issued MMAs complete before TMEM is released.
-        mma_commit(pp.done);
-        long long t0 = clock64();
-        while (!mbar_try_wait(pp.done, 0) && clock64() - t0 < kWaitBudget) {
-        }
+      if (!ok) break;
+      if (leader) mma_commit(&pp.acc_full[buf]);
+      ++acc_it;
+    }
+    if (issued && leader) {
+      // All issued MMAs complete before TMEM is released.
+      mma_commit(pp.done);
+      long long t0 = clock64();
+      while (!mbar_try_wait(pp.done, 0) && clock64() - t0 < kWaitBudget) {
       }
     }
+    __syncwarp();
   } else if (warp < kConvWarp0) {
     // ----------------------------------------------------------- epilogue
     // Per tile: TMEM -> registers -> scaled values stored straight to global
@@ -886,7 +912,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
         }
       };
       auto convert_stage = [&](const float (&v)[BK / 16][8]) -> bool {
-        if (!wait_bar(&pp.empty[stage], phase ^ 1, pp, a.err, 7)) return false;
+        if (!wait_fast(&pp.empty[stage], phase ^ 1, pp, a.err, 7)) return false;
         unsigned char* dst = sA + stage * NPARTS * kAPart;
 #pragma unroll
         for (int j = 0; j < BK / 16; ++j) {
@@ -914,7 +940,7 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_kernel(const __grid_const
       // Read the raw stage into registers and hand it back at once, then wait
       // for the converted-operand slot.
       for (int ks = 0; ks < tl.kst && ok; ++ks) {
-        ok = wait_bar(&pp.full_raw[rstage], rphase, pp, a.err, 8);
+        ok = wait_fast(&pp.full_raw[rstage], rphase, pp, a.err, 8);
         if (!ok) break;
         fetch_raw(ks, va);
         __syncwarp();  // the warp's reads of the raw stage are done
