@@ -623,8 +623,13 @@ __device__ __forceinline__ void trilinear4(const SlDepArgs<T>& a, T lam, T phid,
   const T x = lam * a.inv_dlam;
   const T fi = floor(x);
   const T ax = x - fi;
-  int c0 = (int)fi;  // in [-ni / 2 - 1, ni / 2]: lambda is an atan2
+  // lambda is an atan2: a column in [-ni / 2 - 1, ni / 2], or anything at all
+  // where a wind that is not finite made it NaN (a double NaN converts to the
+  // lowest integer): the clamp keeps the taps in the row and costs less than
+  // the remainder.
+  int c0 = (int)fi;
   if (c0 < 0) c0 += a.ni;
+  c0 = min(max(c0, 0), a.ni - 1);
   const int c1 = c0 + 1 == a.ni ? 0 : c0 + 1;
   const int half = a.ni >> 1;
   const int h0 = c0 >= a.ni - half ? c0 + half - a.ni : c0 + half;

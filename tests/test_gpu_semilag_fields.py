@@ -86,3 +86,41 @@ def test_search_maxima_match_the_move_arrays(dtype, tol, solver):
     _, d = departure_points(CartesianWind(*wind), tables, 300.0, solver=solver)
     assert np.isnan(d.displacement_max_levels) == bool(torch.isnan(
         departure_points(CartesianWind(*wind), tables, 300.0, solver=solver)[0].level).any())
+
+
+@pytest.mark.parametrize("dtype", ["float64", "float32"])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), -float("inf")])
+@pytest.mark.parametrize("ahead", [False, True])
+def test_a_wind_that_is_not_finite_stays_at_its_points(dtype, bad, ahead):
+    """One horizontal component of the advecting or the extrapolated wind not
+    finite at one point: NaN where its value is read (the point itself, and
+    the points whose taps hold it), every other point as without it, on the
+    whole grid and on a band that holds every row (a NaN latitude counts as
+    the south pole's, so a smaller one escapes)."""
+    import torch
+
+    from b200sht.semilag import CartesianWind, departure_points
+
+    tables, _, field = _setup(getattr(torch, dtype))
+    wind, ex = ([30.0 * field() for _ in range(3)] + [1e-3 * field()] for _ in range(2))
+    search = lambda **kw: departure_points(CartesianWind(*wind), tables, 300.0,  # noqa: E731
+                                           extrapolated=CartesianWind(*ex), **kw)
+    clean, _ = search()
+    at = (3, 20, 70)
+    part = (ex if ahead else wind)[1]
+    keep, part[at] = part[at].clone(), 60.0
+    other, _ = search()  # another finite value: what moves reads the point
+    part[at] = bad
+    band = tables.window(slice(0, tables.nlat), slice(0, tables.nlat))
+    for kw in (dict(), dict(window=band, defer_escape=True)):
+        got, d = search(**kw)
+        lost = torch.isnan(got.xi)
+        assert lost[at] and int(lost.sum()) <= (1 if ahead else 64)
+        assert torch.equal(lost, torch.isnan(got.phi))
+        moved = (other.xi != clean.xi) | (other.phi != clean.phi)
+        assert bool((lost | ~moved).all())
+        for name in ("xi", "phi", "level"):
+            assert torch.equal(getattr(got, name)[~lost], getattr(clean, name)[~lost])
+        assert np.isnan(d.displacement_max_m) and np.isnan(d.displacement_max_cells)
+        assert np.isfinite([d.move_max_m, d.move_max_levels, d.displacement_max_levels]).all()
+    part[at] = keep
