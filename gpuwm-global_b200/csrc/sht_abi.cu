@@ -40,9 +40,17 @@ namespace {
 
 // What the driver said, per process: entries are few (a kernel at the shared-
 // memory sizes of the plans in use) and the table is emptied if they are not.
+// A device reset takes the raised limits with it and leaves no plan usable, so
+// making a plan marks them as not raised and the next launch of each kernel
+// raises its own again, to the largest size asked for so far (never below what
+// another thread is about to launch with).
 struct LaunchLimits {
+  struct Limit {
+    size_t most = 0;
+    bool raised = false;
+  };
   std::mutex mu;
-  std::map<std::pair<const void*, int>, size_t> shared;                      // (kernel, device)
+  std::map<std::pair<const void*, int>, Limit> shared;                       // (kernel, device)
   std::map<std::tuple<const void*, int, int, size_t>, int> resident;         // + threads, bytes
 };
 LaunchLimits& launch_limits() {
@@ -50,11 +58,18 @@ LaunchLimits& launch_limits() {
   return *l;
 }
 void raise_shared(LaunchLimits& l, const void* kernel, int dev, size_t bytes) {
-  size_t& have = l.shared[{kernel, dev}];
-  if (bytes <= have) return;
+  LaunchLimits::Limit& have = l.shared[{kernel, dev}];
+  if (have.raised && bytes <= have.most) return;
+  const size_t most = std::max(have.most, bytes);
   SHT_CUDA_OR_THROW(
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  have = bytes;
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+  have = {most, true};
+}
+void forget_raised(int dev) {
+  LaunchLimits& l = launch_limits();
+  std::lock_guard<std::mutex> lock(l.mu);
+  for (auto& e : l.shared)
+    if (e.first.second == dev) e.second.raised = false;
 }
 
 }  // namespace
@@ -72,10 +87,10 @@ int resident_ctas(const void* kernel, int threads, size_t bytes) {
   SHT_CUDA_OR_THROW(cudaGetDevice(&dev));
   LaunchLimits& l = launch_limits();
   std::lock_guard<std::mutex> lock(l.mu);
+  raise_shared(l, kernel, dev, bytes);
   const auto key = std::make_tuple(kernel, dev, threads, bytes);
   const auto found = l.resident.find(key);
   if (found != l.resident.end()) return found->second;
-  raise_shared(l, kernel, dev, bytes);
   int per_sm = 0, sms = 0;
   SHT_CUDA_OR_THROW(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, bytes));
   SHT_CUDA_OR_THROW(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -846,6 +861,7 @@ int sht_plan_create(int truncation, int nlat, int nlon, double radius_m, int pre
     cudaStream_t s = nullptr;
     try {
       SHT_CUDA_OR_THROW(cudaGetDevice(&p->device));
+      forget_raised(p->device);
       SHT_CUDA_OR_THROW(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
       SHT_CUDA_OR_THROW(cudaMalloc(&p->d_err, sizeof(unsigned) * 4));
       SHT_CUDA_OR_THROW(cudaMemsetAsync(p->d_err, 0, sizeof(unsigned) * 4, s));

@@ -121,7 +121,8 @@ struct sht_plan {
 namespace sht {
 
 // Raises a kernel's dynamic shared-memory limit on the current device to at
-// least `bytes`; the driver is asked only when the limit grows.
+// least `bytes`; the driver is asked only when the limit grows or a plan has
+// been made since (which may have been after a device reset).
 void allow_shared(const void* kernel, size_t bytes);
 // CTAs of the kernel resident on the whole current device (SMs x CTAs per SM)
 // at the given block and dynamic shared memory, its limit raised to `bytes`;
