@@ -188,6 +188,7 @@ struct SlArgs {
   // the whole grid njs = nja = nj and esc is null.
   int njs, nja;
   int* esc;
+  int k0, j0;  // first level and row of this launch
 };
 
 // The in-plane offset of extended row r: an offset of -1 (a row outside a
@@ -305,7 +306,8 @@ __global__ void __launch_bounds__(kGatherX * kGatherY * kGatherZ,
   const int plane = a.njs * a.ni;              // a held source level
   const int64_t n = (int64_t)a.nk * a.nja * a.ni;  // arrival points
   const int ia = blockIdx.x * kGatherX + threadIdx.x;
-  const int ka = blockIdx.y * kGatherY + threadIdx.y, ja = blockIdx.z * kGatherZ + threadIdx.z;
+  const int ka = a.k0 + blockIdx.y * kGatherY + threadIdx.y;
+  const int ja = a.j0 + blockIdx.z * kGatherZ + threadIdx.z;
   if (ia >= a.ni || ka >= a.nk || ja >= a.nja) return;
   const int64_t gid = ((int64_t)ka * a.nja + ja) * a.ni + ia;
   const T p = min(max(a.phi[gid], T(-kHalfPi)), T(kHalfPi));
@@ -552,6 +554,7 @@ struct SlDepArgs {
   // ja0 = lead = 0, esc null.
   int njs, nja, ja0, lead;
   int* esc;
+  int k0, j0;  // first level and row of this launch
 };
 
 constexpr int kDepX = 64, kDepY = 2, kDepZ = 1;  // arrival points of a CTA: columns, levels, rows
@@ -559,8 +562,8 @@ constexpr int kDepX = 64, kDepY = 2, kDepZ = 1;  // arrival points of a CTA: col
 struct Arrival { int k, j, i; bool live; };
 template <typename T>
 __device__ __forceinline__ Arrival arrival_point(const SlDepArgs<T>& a) {
-  const int i = blockIdx.x * kDepX + threadIdx.x, k = blockIdx.y * kDepY + threadIdx.y;
-  const int j = blockIdx.z * kDepZ + threadIdx.z;
+  const int i = blockIdx.x * kDepX + threadIdx.x, k = a.k0 + blockIdx.y * kDepY + threadIdx.y;
+  const int j = a.j0 + blockIdx.z * kDepZ + threadIdx.z;
   return {k, j, i, i < a.ni && k < a.nk && j < a.nja};
 }
 
@@ -1143,21 +1146,36 @@ SlArgs<T> make_args(const sht_sl_tables* t, const SlWidth& w, const void* src, i
   return a;
 }
 
+// launch(grid, k0, j0) over all arrival points: one launch, or several where
+// the levels or the rows pass the 65535 blocks of a grid's second and third
+// dimensions (which hold them so that no thread divides).
+template <class F>
+void over_points(int ni, int nk, int nj, dim3 block, F&& launch) {
+  constexpr int kMost = 65535;
+  for (int64_t j0 = 0; j0 < nj; j0 += (int64_t)kMost * block.z)
+    for (int64_t k0 = 0; k0 < nk; k0 += (int64_t)kMost * block.y)
+      launch(dim3((unsigned)div_up(ni, block.x),
+                  (unsigned)std::min<int64_t>(kMost, div_up(nk - k0, block.y)),
+                  (unsigned)std::min<int64_t>(kMost, div_up(nj - j0, block.z))),
+             (int)k0, (int)j0);
+}
+
 template <typename T, int NH, int VEC>
-void launch_gather(const SlArgs<T>& a, bool qm, bool def, cudaStream_t s) {
+void launch_gather(SlArgs<T> a, bool qm, bool def, cudaStream_t s) {
   const dim3 block(kGatherX, kGatherY, kGatherZ);
-  const dim3 grid((unsigned)div_up(a.ni, kGatherX), (unsigned)div_up(a.nk, kGatherY),
-                  (unsigned)div_up(a.nja, kGatherZ));
-  SHT_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "too many levels or rows for one gather launch");
-  if constexpr (NH == 6) {
-    if (qm) sl_gather_kernel<T, 6, VEC, true, false><<<grid, block, 0, s>>>(a);
-    else sl_gather_kernel<T, 6, VEC, false, false><<<grid, block, 0, s>>>(a);
-  } else {
-    if (def) sl_gather_kernel<T, 4, VEC, true, true><<<grid, block, 0, s>>>(a);
-    else if (qm) sl_gather_kernel<T, 4, VEC, true, false><<<grid, block, 0, s>>>(a);
-    else sl_gather_kernel<T, 4, VEC, false, false><<<grid, block, 0, s>>>(a);
-  }
-  SHT_CUDA_OR_THROW(cudaGetLastError());
+  over_points(a.ni, a.nk, a.nja, block, [&](dim3 grid, int k0, int j0) {
+    a.k0 = k0;
+    a.j0 = j0;
+    if constexpr (NH == 6) {
+      if (qm) sl_gather_kernel<T, 6, VEC, true, false><<<grid, block, 0, s>>>(a);
+      else sl_gather_kernel<T, 6, VEC, false, false><<<grid, block, 0, s>>>(a);
+    } else {
+      if (def) sl_gather_kernel<T, 4, VEC, true, true><<<grid, block, 0, s>>>(a);
+      else if (qm) sl_gather_kernel<T, 4, VEC, true, false><<<grid, block, 0, s>>>(a);
+      else sl_gather_kernel<T, 4, VEC, false, false><<<grid, block, 0, s>>>(a);
+    }
+    SHT_CUDA_OR_THROW(cudaGetLastError());
+  });
 }
 template <typename T, int VEC>
 void launch_gather_order(const SlArgs<T>& a, int order, bool qm, bool def, cudaStream_t s) {
@@ -1535,9 +1553,6 @@ static int departure_entry(int solver, const sht_sl_window* win, const sht_sl_ta
     const SlWidth& w = tables->w4;
     const int rows_out = win ? win->a1 - win->a0 : tables->nlat;
     const dim3 block(kDepX, kDepY, kDepZ);
-    const dim3 grid((unsigned)div_up(tables->nlon, kDepX), (unsigned)div_up(nlev, kDepY),
-                    (unsigned)div_up(rows_out, kDepZ));
-    SHT_REQUIRE(grid.y <= 65535 && grid.z <= 65535, "too many levels or rows for one search");
     cudaStream_t s = (cudaStream_t)stream;
     auto fill = [&](auto* a) {
       using T = std::remove_cv_t<std::remove_pointer_t<decltype(a->vx)>>;
@@ -1569,20 +1584,20 @@ static int departure_entry(int solver, const sht_sl_window* win, const sht_sl_ta
     };
     SHT_REQUIRE(solver >= kSolverFixedPoint && solver <= kSolverNewtonLs,
                 "departure solver is 0 (fixed point), 1 (Newton) or 2 (line-search Newton)");
-    if (tables->prec == SHT_PREC_F64) {
-      SlDepArgs<double> a;
+    auto search = [&](auto a) {
+      using T = std::remove_cv_t<std::remove_pointer_t<decltype(a.vx)>>;
       fill(&a);
-      if (solver == kSolverNewton) sl_departure_newton_kernel<double><<<grid, block, 0, s>>>(a);
-      else if (solver == kSolverNewtonLs) sl_departure_newton_ls_kernel<double><<<grid, block, 0, s>>>(a);
-      else sl_departure_kernel<double><<<grid, block, 0, s>>>(a);
-    } else {
-      SlDepArgs<float> a;
-      fill(&a);
-      if (solver == kSolverNewton) sl_departure_newton_kernel<float><<<grid, block, 0, s>>>(a);
-      else if (solver == kSolverNewtonLs) sl_departure_newton_ls_kernel<float><<<grid, block, 0, s>>>(a);
-      else sl_departure_kernel<float><<<grid, block, 0, s>>>(a);
-    }
-    SHT_CUDA_OR_THROW(cudaGetLastError());
+      over_points(tables->nlon, nlev, rows_out, block, [&](dim3 grid, int k0, int j0) {
+        a.k0 = k0;
+        a.j0 = j0;
+        if (solver == kSolverNewton) sl_departure_newton_kernel<T><<<grid, block, 0, s>>>(a);
+        else if (solver == kSolverNewtonLs) sl_departure_newton_ls_kernel<T><<<grid, block, 0, s>>>(a);
+        else sl_departure_kernel<T><<<grid, block, 0, s>>>(a);
+        SHT_CUDA_OR_THROW(cudaGetLastError());
+      });
+    };
+    if (tables->prec == SHT_PREC_F64) search(SlDepArgs<double>{});
+    else search(SlDepArgs<float>{});
   });
 }
 

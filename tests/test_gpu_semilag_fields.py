@@ -124,3 +124,33 @@ def test_a_wind_that_is_not_finite_stays_at_its_points(dtype, bad, ahead):
         assert np.isnan(d.displacement_max_m) and np.isnan(d.displacement_max_cells)
         assert np.isfinite([d.move_max_m, d.move_max_levels, d.displacement_max_levels]).all()
     part[at] = keep
+
+
+@pytest.mark.parametrize("shape", [(131074, 4, 6), (4, 131074, 6)])
+def test_more_levels_or_rows_than_a_grid_dimension(shape):
+    """Levels and rows past 65535 blocks, where a call takes several launches:
+    a resting wind departs from its arrival points, and the gather there
+    returns the field bit for bit."""
+    import types
+
+    import torch
+
+    from b200sht.semilag import (CartesianWind, SphericalGridTables, departure_points,
+                                 gather_batch, zero_stencil)
+
+    nlev, nlat, nlon = shape
+    lat = (np.arange(nlat) + 0.5) * np.pi / nlat - 0.5 * np.pi
+    tables = SphericalGridTables.create(types.SimpleNamespace(
+        nlat=nlat, nlon=nlon, lat_rad=lat, lon_rad=np.arange(nlon) * 2 * np.pi / nlon,
+        radius_m=6371220.0), dtype=torch.float64)
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    fields = [torch.randn(shape, generator=gen, device="cuda", dtype=torch.float64)
+              for _ in range(3)]
+    for got, want in zip(gather_batch(fields, zero_stencil(tables, nlev)), fields):
+        assert torch.equal(got, want)
+    rest = torch.zeros(shape, dtype=torch.float64, device="cuda")
+    st, d = departure_points(CartesianWind(rest, rest, rest, rest), tables, 300.0)
+    assert torch.equal(st.level, torch.arange(nlev, dtype=torch.float64, device="cuda")
+                       [:, None, None].expand(shape))
+    assert float((st.phi - torch.as_tensor(lat, device="cuda")[None, :, None]).abs().max()) < 1e-12
+    assert d.displacement_max_levels == 0.0 and d.displacement_max_m < 1e-6
