@@ -291,7 +291,7 @@ void do_forward(sht_plan* p, const T* grid, int64_t planes, T* coeff, cudaStream
     KernelScope k(p, SHT_KIND_FFT_FORWARD, s);
     launch_forward_fold<T>(p, grid, nullptr, planes, ldc, w, s, rm);
   }
-  if (!uses_tc(p) && simt_takes_coefficients(p, R)) {
+  if (!uses_tc(p) && simt_takes_coefficients(p, R, 1)) {
     KernelScope k(p, SHT_KIND_LEGENDRE_ANALYSIS, s);
     launch_simt_to_coefficients<T>(p, static_cast<const T*>(p->analysis), w, coeff, planes, R, s);
     return;
@@ -311,9 +311,10 @@ void synthesize(sht_plan* p, int kind0, int kind1, const T* coeff, int64_t plane
   const int64_t R = 2 * ldc;
   T* c = static_cast<T*>(p->cfold[0]);
   T* w[2] = {static_cast<T*>(p->wfold[0]), static_cast<T*>(p->wfold[1])};
-  if (!uses_tc(p) && simt_takes_coefficients(p, R)) {
+  const int n = kind1 < 0 ? 1 : 2;
+  if (!uses_tc(p) && simt_takes_coefficients(p, R, n)) {
     KernelScope k(p, SHT_KIND_LEGENDRE_SYNTHESIS, s);
-    const int n = kind1 < 0 ? 1 : 2, kinds[2] = {kind0, kind1};
+    const int kinds[2] = {kind0, kind1};
     int flip[2] = {};
     const T* table[2] = {};
     for (int g = 0; g < n; ++g) {

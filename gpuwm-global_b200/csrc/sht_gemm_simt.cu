@@ -219,25 +219,19 @@ __global__ void __launch_bounds__(32 * WX, 16 / WX) gemm_simt_kernel(const __gri
     simt_tile<T, WX, G, DB>(grp, d, it.x0, r0, a.R, smem);
 }
 
-// At most 8 data rows (one to four planes): bound by reading the table once and,
-// below T511, by the latency of the chain over k, so every lane takes one
-// column (the most warps in flight) with U table rows on their way; the data
-// values are one address for the whole warp.  The same chain of fused multiply-
-// adds per output as the tiles.  Against a half-empty 32-row tile: T241 x 3
-// planes FP32 (8 rows), both contractions, 45 us less of a 136 us pair (four
-// columns to a lane: 22 us more); the P and dP/dphi syntheses of one T255 plane
-// 44 -> 28 us; T21 x 1 plane 7.4 -> 6.0 us.
+// At most 8 data rows (one to four planes): bound by reading the table once and
+// by the latency of the chain over k, so every lane takes one column (the most
+// warps in flight) with U table rows on their way; the data values are one
+// address for the whole warp.  The same chain of fused multiply-adds per output
+// as the tiles, which keep more table rows in flight once a lane holds more than
+// four FP32 sums; skinny_folded and simt_takes_coefficients draw the lines.
 //
 // The transforms' own calls take the spectral side in place, too: with CPACK the
 // data rows are read from the coefficients [plane][n][m] (the pack pass's
 // layout change is nothing for values that a whole warp shares), with CUNPACK
 // the outputs go to them, real at m = 0, and the block of parity 0 zeroes its
 // order above the triangle.  T21 x 1 plane FP32, the pair: 36.3 us with the two
-// layout passes, 32.2 us without; forward, inverse and gradient of one to four
-// planes at T62 FP32: 78-82 us and 67-75.  Below T128 and R * T of 512: past it
-// the strided reads cost more than the passes (T106 x 4 planes 93 and 95 us,
-// T126 x 4 97 and 105, T170 x 1 or 2 the same both ways, T255's gradient of
-// one plane 4 us more).
+// layout passes, 32.2 us without.
 enum SkinnySpectral { kFolded = 0, kCPack = 1, kCUnpack = 2 };
 template <typename T, int RR, int SPEC>
 __global__ void __launch_bounds__(128) gemm_skinny_kernel(const __grid_constant__ SimtArgs<T> a) {
@@ -391,20 +385,39 @@ void launch_simt(const SimtArgs<T>& a, int n_items, cudaStream_t s) {
 
 namespace {
 
+// Folded operands by the streaming kernel: four FP32 rows (one or two planes;
+// one of a wind).  Forward and gradient of two planes, streaming and in tiles:
+// T170 24.9 / 22.8 and 24.8 / 26.4 us, T255 34.9 / 37.1 and 35.9 / 45.5, T511
+// 97 / 136 and 132 / 197.  Eight rows: T255 46 / 38 and 45 / 46, T511 215 / 138
+// and 213 / 207; FP64 four rows: T126 (wind of one plane) 29.7 / 24.7, T255
+// (forward of two planes) 58.8 / 42.5.
+template <typename T>
+constexpr bool skinny_folded(int64_t R) { return sizeof(T) == 4 && R <= 4; }
+
 template <typename T, int SPEC>
 void launch_skinny(const SimtArgs<T>& a, int n_items, cudaStream_t s) {
   const unsigned blocks = (unsigned)n_items * (unsigned)a.ng, threads = tile_x<T>(4);
-  if (a.R <= 4)
+  if (SPEC == kFolded || a.R <= 4)
     gemm_skinny_kernel<T, 4, SPEC><<<blocks, threads, 0, s>>>(a);
-  else
+  else if constexpr (SPEC != kFolded)
     gemm_skinny_kernel<T, 8, SPEC><<<blocks, threads, 0, s>>>(a);
   SHT_CUDA_OR_THROW(cudaGetLastError());
 }
 
 }  // namespace
 
-bool simt_takes_coefficients(const sht_plan* p, int64_t R) {
-  return R <= 8 && p->T < 128 && R * p->T <= 512;
+// In place while the chain is short: past these truncations the tiles with their
+// layout passes are faster, for the two tables of a gradient a little later.
+// Microseconds in place and in tiles, forward, inverse and gradient: FP32 two
+// planes T126 19.6 / 19.6, 18.5 / 20.6 and 19.4 / 22.8; four planes T53 17.5 /
+// 18.7, 16.4 / 17.7 and 18.6 / 21.9, T75 22.7 / 18.6, 18.5 / 17.6 and 21.4 / 21.7;
+// FP64 two planes T75 18.5 / 18.4, 16.5 / 17.6 and 18.7 / 21.9, T106 21.6 / 18.6,
+// 19.6 / 18.5 and 22.3 / 21.9; four planes T30 15.7 / 18.6, 16.4 / 17.7 and 18.8 /
+// 21.9, T53 20.6 / 18.8, 20.6 / 17.9 and 20.6 / 22.0, T62 gradient 22.7 / 22.0.
+bool simt_takes_coefficients(const sht_plan* p, int64_t R, int tables) {
+  const bool f64 = p->prec == SHT_PREC_F64, two = tables == 2;
+  if (R <= 4) return p->T < (f64 ? (two ? 100 : 80) : 128);
+  return R <= 8 && p->T < (f64 ? (two ? 60 : 43) : (two ? 76 : 56));
 }
 
 template <typename T>
@@ -443,7 +456,7 @@ void launch_gemm_simt_groups(const sht_plan* p, int direction, int ngroups, cons
   // data reloads make up for it (T511 x 200 planes 1921 against 1955 us; T255 x
   // 161 planes 292 against 264, T126 x 200 planes 76 against 70).
   const bool narrow = std::is_same<T, float>::value && (p->tune_simt_tile == 1 || p->H < 256);
-  const bool skinny = R <= 8;
+  const bool skinny = skinny_folded<T>(R);
   const int n_items = narrow && !skinny ? p->n_items_narrow[direction] : p->n_items[direction];
   if (n_items == 0 || R == 0) return;
   SHT_REQUIRE(ngroups == 1 || ngroups == 2, "one or two tables per SIMT launch");
@@ -455,9 +468,11 @@ void launch_gemm_simt_groups(const sht_plan* p, int direction, int ngroups, cons
   SHT_REQUIRE(a.items != nullptr, "SIMT work list not built");
   a.ng = ngroups;
   a.R = R;
-  if (skinny) {
-    launch_skinny<T, kFolded>(a, n_items, s);
-    return;
+  if constexpr (sizeof(T) == 4) {
+    if (skinny) {
+      launch_skinny<T, kFolded>(a, n_items, s);
+      return;
+    }
   }
   const int whole = tile_r<T>(SimtCfg<T>::G);
   a.nrb = (int)div_up(R, whole);

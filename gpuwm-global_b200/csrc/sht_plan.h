@@ -177,10 +177,10 @@ void launch_gemm_simt_groups(const sht_plan* p, int direction, int ngroups, cons
                              const T* const* table, const T* const* data, T* const* out,
                              int64_t R, cudaStream_t s);
 
-// At few rows (and below T128) the SIMT contraction takes the spectral side of a scalar
+// At few rows of a small truncation the SIMT contraction takes the spectral side of a scalar
 // transform in place: a synthesis of one or two tables from the coefficients
 // [plane][n][m], an analysis into them (real at m = 0, zero above the triangle).
-bool simt_takes_coefficients(const sht_plan* p, int64_t R);
+bool simt_takes_coefficients(const sht_plan* p, int64_t R, int tables);
 template <typename T>
 void launch_simt_from_coefficients(const sht_plan* p, int ngroups, const int* flip,
                                    const T* const* table, const T* coeff, int64_t planes,
