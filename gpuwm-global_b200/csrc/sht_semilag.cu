@@ -188,7 +188,7 @@ struct SlArgs {
   // the whole grid njs = nja = nj and esc is null.
   int njs, nja;
   int* esc;
-  int k0, j0;  // first level and row of this launch
+  int nkl, njl;  // levels and rows of this launch, from the first of its pointers on
 };
 
 // The in-plane offset of extended row r: an offset of -1 (a row outside a
@@ -306,9 +306,8 @@ __global__ void __launch_bounds__(kGatherX * kGatherY * kGatherZ,
   const int plane = a.njs * a.ni;              // a held source level
   const int64_t n = (int64_t)a.nk * a.nja * a.ni;  // arrival points
   const int ia = blockIdx.x * kGatherX + threadIdx.x;
-  const int ka = a.k0 + blockIdx.y * kGatherY + threadIdx.y;
-  const int ja = a.j0 + blockIdx.z * kGatherZ + threadIdx.z;
-  if (ia >= a.ni || ka >= a.nk || ja >= a.nja) return;
+  const int ka = blockIdx.y * kGatherY + threadIdx.y, ja = blockIdx.z * kGatherZ + threadIdx.z;
+  if (ia >= a.ni || ka >= a.nkl || ja >= a.njl) return;
   const int64_t gid = ((int64_t)ka * a.nja + ja) * a.ni + ia;
   const T p = min(max(a.phi[gid], T(-kHalfPi)), T(kHalfPi));
   const T xk = min(max(a.lev[gid], T(-0.5)), T(a.nk) - T(0.5));
@@ -1163,9 +1162,16 @@ void over_points(int ni, int nk, int nj, dim3 block, F&& launch) {
 template <typename T, int NH, int VEC>
 void launch_gather(SlArgs<T> a, bool qm, bool def, cudaStream_t s) {
   const dim3 block(kGatherX, kGatherY, kGatherZ);
+  const SlArgs<T> all = a;
   over_points(a.ni, a.nk, a.nja, block, [&](dim3 grid, int k0, int j0) {
-    a.k0 = k0;
-    a.j0 = j0;
+    const int64_t first = ((int64_t)k0 * a.nja + j0) * a.ni;
+    a.nkl = a.nk - k0;
+    a.njl = a.nja - j0;
+    a.xi = all.xi + first;
+    a.phi = all.phi + first;
+    a.lev = all.lev + first;
+    a.out = all.out + first;
+    a.cut = all.cut ? all.cut + first : nullptr;
     if constexpr (NH == 6) {
       if (qm) sl_gather_kernel<T, 6, VEC, true, false><<<grid, block, 0, s>>>(a);
       else sl_gather_kernel<T, 6, VEC, false, false><<<grid, block, 0, s>>>(a);
