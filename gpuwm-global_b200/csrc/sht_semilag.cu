@@ -188,7 +188,6 @@ struct SlArgs {
   // the whole grid njs = nja = nj and esc is null.
   int njs, nja;
   int* esc;
-  int nkl, njl;  // levels and rows of this launch, from the first of its pointers on
 };
 
 // The in-plane offset of extended row r: an offset of -1 (a row outside a
@@ -307,7 +306,7 @@ __global__ void __launch_bounds__(kGatherX * kGatherY * kGatherZ,
   const int64_t n = (int64_t)a.nk * a.nja * a.ni;  // arrival points
   const int ia = blockIdx.x * kGatherX + threadIdx.x;
   const int ka = blockIdx.y * kGatherY + threadIdx.y, ja = blockIdx.z * kGatherZ + threadIdx.z;
-  if (ia >= a.ni || ka >= a.nkl || ja >= a.njl) return;
+  if (ia >= a.ni || ka >= a.nk || ja >= a.nja) return;
   const int64_t gid = ((int64_t)ka * a.nja + ja) * a.ni + ia;
   const T p = min(max(a.phi[gid], T(-kHalfPi)), T(kHalfPi));
   const T xk = min(max(a.lev[gid], T(-0.5)), T(a.nk) - T(0.5));
@@ -1145,18 +1144,20 @@ SlArgs<T> make_args(const sht_sl_tables* t, const SlWidth& w, const void* src, i
   return a;
 }
 
-// launch(grid, k0, j0) over all arrival points: one launch, or several where
-// the levels or the rows pass the 65535 blocks of a grid's second and third
-// dimensions (which hold them so that no thread divides).
+// launch(grid, k0, j0) over all arrival points: one launch, or slabs from level
+// k0 and row j0 on where the levels or the rows pass the 65535 blocks of a
+// grid's second and third dimensions (which hold them so that no thread
+// divides).  A slab is whole blocks and the last one ends with the points,
+// writing some of the slab before it again: no slab reaches past the end.
 template <class F>
 void over_points(int ni, int nk, int nj, dim3 block, F&& launch) {
-  constexpr int kMost = 65535;
-  for (int64_t j0 = 0; j0 < nj; j0 += (int64_t)kMost * block.z)
-    for (int64_t k0 = 0; k0 < nk; k0 += (int64_t)kMost * block.y)
-      launch(dim3((unsigned)div_up(ni, block.x),
-                  (unsigned)std::min<int64_t>(kMost, div_up(nk - k0, block.y)),
-                  (unsigned)std::min<int64_t>(kMost, div_up(nj - j0, block.z))),
-             (int)k0, (int)j0);
+  constexpr int64_t kMost = 65535;
+  const int64_t sk = std::min<int64_t>(nk, kMost * block.y), sj = std::min<int64_t>(nj, kMost * block.z);
+  const dim3 grid((unsigned)div_up(ni, block.x), (unsigned)div_up(sk, block.y),
+                  (unsigned)div_up(sj, block.z));
+  for (int64_t j = 0; j < nj; j += sj)
+    for (int64_t k = 0; k < nk; k += sk)
+      launch(grid, (int)std::min(k, nk - sk), (int)std::min(j, nj - sj));
 }
 
 template <typename T, int NH, int VEC>
@@ -1164,9 +1165,8 @@ void launch_gather(SlArgs<T> a, bool qm, bool def, cudaStream_t s) {
   const dim3 block(kGatherX, kGatherY, kGatherZ);
   const SlArgs<T> all = a;
   over_points(a.ni, a.nk, a.nja, block, [&](dim3 grid, int k0, int j0) {
+    // a slab's pointers start at its first point; the counts stay the call's
     const int64_t first = ((int64_t)k0 * a.nja + j0) * a.ni;
-    a.nkl = a.nk - k0;
-    a.njl = a.nja - j0;
     a.xi = all.xi + first;
     a.phi = all.phi + first;
     a.lev = all.lev + first;
