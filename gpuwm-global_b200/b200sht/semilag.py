@@ -354,14 +354,21 @@ def gather_batch(fields: Sequence[torch.Tensor], stencil: Stencil, *, monotone: 
         window.clear_escape()
     out: list = []
     for start in range(0, len(fields), int(batch)):
-        chunk = [f.contiguous() for f in fields[start:start + int(batch)]]
+        chunk = fields[start:start + int(batch)]
         count = len(chunk)
-        dst = torch.empty((count, *stencil.shape), dtype=chunk[0].dtype, device=chunk[0].device)
+        like = chunk[0]
+        if all(f.is_contiguous() for f in chunk):
+            at = [f.data_ptr() for f in chunk]
+        else:  # one launch lays them all out
+            block = _source_block(chunk)
+            step = block.stride(0) * block.element_size()
+            at = [block.data_ptr() + i * step for i in range(count)]
+        dst = torch.empty((count, *stencil.shape), dtype=like.dtype, device=like.device)
         cut = torch.empty_like(dst) if deficit else None
         # room for the fields interleaved (a single one is read in place)
         packed = (torch.empty((count, *stencil.source_shape), dtype=dst.dtype, device=dst.device)
                   if count > 1 else None)
-        ptrs = (ctypes.c_void_p * count)(*[f.data_ptr() for f in chunk])
+        ptrs = (ctypes.c_void_p * count)(*at)
         tables = stencil.tables if window is None else window.tables
         _lib.call("sht_sl_gather_fields", tables._handle,
                   None if window is None else window._handle, order, lim, 1 if deficit else 0,

@@ -190,6 +190,13 @@ struct SlArgs {
   int* esc;
 };
 
+// The same with F volumes of their own in place of src.
+constexpr int kEachFields = 5;
+template <typename T>
+struct SlEachArgs : SlArgs<T> {
+  const T* each[kEachFields];
+};
+
 // The in-plane offset of extended row r: an offset of -1 (a row outside a
 // band's held rows) raises the escape flag and reads the first held row,
 // so the access stays in bounds while the caller refuses the result.
@@ -295,10 +302,10 @@ __global__ void __launch_bounds__(256) sl_pack_kernel(const __grid_constant__ Pa
 // bytes a clock would take 5.4 ms: it waits for the taps at 16 warps an SM), 9.3
 // ms in CTAs of 128 points, five to an SM (FP64: four); and 0.98 ms to interleave
 // against 0.89 ms for the copy.
-template <typename T, int NH, int VEC, bool QM, bool DEF>
+template <typename T, int NH, int VEC, bool EACH, bool QM, bool DEF>
 __global__ void __launch_bounds__(kGatherX * kGatherY * kGatherZ,
                                   NH == 6 || sizeof(T) == 8 ? 4 : (VEC == 4 ? 5 : 6))
-    sl_gather_kernel(const SlArgs<T> a) {
+    sl_gather_kernel(const std::conditional_t<EACH, SlEachArgs<T>, SlArgs<T>> a) {
   using P = Pack<T, VEC>;
   constexpr int G = NH / 2 - 1;  // zonal lead and meridional start offset
   constexpr int MID = NH / 2 - 1;
@@ -393,7 +400,8 @@ __global__ void __launch_bounds__(kGatherX * kGatherY * kGatherZ,
     P base[NB], acc[NB], lo[NB], hi[NB], f_edge[NB], f_next[NB];
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
-      s[b] = reinterpret_cast<const P*>(a.src) + (f0 + b) * sstride;
+      if constexpr (EACH) s[b] = reinterpret_cast<const P*>(a.each[f0 + b]);
+      else s[b] = reinterpret_cast<const P*>(a.src) + (f0 + b) * sstride;
       base[b] = load_pack<T, VEC>(s[b] + cofs);
 #pragma unroll
       for (int e = 0; e < VEC; ++e)
@@ -1160,8 +1168,8 @@ void over_points(int ni, int nk, int nj, dim3 block, F&& launch) {
       launch(grid, (int)std::min(k, nk - sk), (int)std::min(j, nj - sj));
 }
 
-template <typename T, int NH, int VEC>
-void launch_gather(SlArgs<T> a, bool qm, bool def, cudaStream_t s) {
+template <typename T, int NH, int VEC, bool EACH, class Args>
+void launch_gather(Args a, bool qm, bool def, cudaStream_t s) {
   const dim3 block(kGatherX, kGatherY, kGatherZ);
   const SlArgs<T> all = a;
   over_points(a.ni, a.nk, a.nja, block, [&](dim3 grid, int k0, int j0) {
@@ -1173,20 +1181,20 @@ void launch_gather(SlArgs<T> a, bool qm, bool def, cudaStream_t s) {
     a.out = all.out + first;
     a.cut = all.cut ? all.cut + first : nullptr;
     if constexpr (NH == 6) {
-      if (qm) sl_gather_kernel<T, 6, VEC, true, false><<<grid, block, 0, s>>>(a);
-      else sl_gather_kernel<T, 6, VEC, false, false><<<grid, block, 0, s>>>(a);
+      if (qm) sl_gather_kernel<T, 6, VEC, EACH, true, false><<<grid, block, 0, s>>>(a);
+      else sl_gather_kernel<T, 6, VEC, EACH, false, false><<<grid, block, 0, s>>>(a);
     } else {
-      if (def) sl_gather_kernel<T, 4, VEC, true, true><<<grid, block, 0, s>>>(a);
-      else if (qm) sl_gather_kernel<T, 4, VEC, true, false><<<grid, block, 0, s>>>(a);
-      else sl_gather_kernel<T, 4, VEC, false, false><<<grid, block, 0, s>>>(a);
+      if (def) sl_gather_kernel<T, 4, VEC, EACH, true, true><<<grid, block, 0, s>>>(a);
+      else if (qm) sl_gather_kernel<T, 4, VEC, EACH, true, false><<<grid, block, 0, s>>>(a);
+      else sl_gather_kernel<T, 4, VEC, EACH, false, false><<<grid, block, 0, s>>>(a);
     }
     SHT_CUDA_OR_THROW(cudaGetLastError());
   });
 }
-template <typename T, int VEC>
-void launch_gather_order(const SlArgs<T>& a, int order, bool qm, bool def, cudaStream_t s) {
-  if (order == 6) launch_gather<T, 6, VEC>(a, qm, def, s);
-  else launch_gather<T, 4, VEC>(a, qm, def, s);
+template <typename T, int VEC, bool EACH = false, class Args>
+void launch_gather_order(const Args& a, int order, bool qm, bool def, cudaStream_t s) {
+  if (order == 6) launch_gather<T, 6, VEC, EACH>(a, qm, def, s);
+  else launch_gather<T, 4, VEC, EACH>(a, qm, def, s);
 }
 
 // Interleaves `groups` groups of VEC fields into `packed` and gathers them
@@ -1210,28 +1218,48 @@ void gather_groups(SlArgs<T> a, const void* const* fields, int groups, T* packed
   launch_gather_order<T, VEC>(a, order, qm, def, s);
 }
 
-// All fields of a call: groups of 16 bytes, then (FP32) one group of two, then
-// a single field read in place.
+// All fields of a call: groups of 16 bytes, then (FP32) one group of two or a
+// single field in place.  Three left-over FP32 fields, and FP64 calls of three
+// or five, are read in place by one launch: a launch for the groups and another
+// for the odd field work every point's indices and weights out twice.
+// Microseconds in two launches, in place, and as one block copied together
+// first: three limited FP32 fields, T511 x 12 levels 1152 / 1067 / 1178, T62 x 20
+// levels 41.0 / 32.6 / 37.0; unlimited FP64, T62, three fields 55.4 / 41.0 / 49.3,
+// five 73.8 / 59.5 / 68.2.  The quintic of five FP64 fields is faster in groups
+// where the fields pass the L2 (T511 unlimited 5621 / 5840 / 5739, limited 5650
+// / 6443 / 6680; T62 unlimited 161 / 143 / 155).
 template <typename T>
 void gather_fields(SlArgs<T> a, const void* const* fields, int count, T* packed, int order,
                    bool qm, bool def, cudaStream_t s) {
   constexpr int V = 16 / (int)sizeof(T);
+  constexpr int64_t kL2 = 126 << 20;
   const int64_t n_src = (int64_t)a.nk * a.njs * a.ni, n_out = (int64_t)a.nk * a.nja * a.ni;
   T* const out = a.out;
   T* const cut = a.cut;
-  int f = count / V * V;
-  gather_groups<T, V>(a, fields, count / V, packed, order, qm, def, s);
+  auto from = [&](int f) {
+    a.out = out + f * n_out;
+    a.cut = cut ? cut + f * n_out : nullptr;
+  };
+  const bool in_place = sizeof(T) == 8
+                            ? count == 3 || (count == 5 && (order == 4 || (!qm && 40 * n_src < kL2)))
+                            : count % V == 3;
+  int f = in_place && sizeof(T) == 8 ? 0 : count / V * V;
+  gather_groups<T, V>(a, fields, f / V, packed, order, qm, def, s);
+  from(f);
+  if (in_place) {
+    SlEachArgs<T> b{a, {}};
+    b.F = count - f;
+    for (int e = 0; e < b.F; ++e) b.each[e] = static_cast<const T*>(fields[f + e]);
+    launch_gather_order<T, 1, true>(b, order, qm, def, s);
+    return;
+  }
   if constexpr (V == 4) {
-    if (count - f >= 2) {
-      a.out = out + f * n_out;
-      a.cut = cut ? cut + f * n_out : nullptr;
+    if (count - f == 2) {
       gather_groups<T, 2>(a, fields + f, 1, packed + f * n_src, order, qm, def, s);
-      f += 2;
+      return;
     }
   }
   if (f < count) {
-    a.out = out + f * n_out;
-    a.cut = cut ? cut + f * n_out : nullptr;
     a.src = static_cast<const T*>(fields[f]);
     a.F = 1;
     launch_gather_order<T, 1>(a, order, qm, def, s);
