@@ -319,6 +319,9 @@ def _check_fields(fields, stencil: Stencil) -> None:
                 f"not the wrong answer")
         if not field.is_cuda:
             raise ValueError(f"field {index} must be a CUDA tensor")
+        if field.device != fields[0].device:
+            raise ValueError(f"field {index} is on {field.device} where field 0 is on "
+                             f"{fields[0].device}")
 
 
 def _source_block(chunk):

@@ -58,3 +58,20 @@ def test_band_window_geometry_and_escape_text():
     err = HaloEscape(win, "gather")
     assert isinstance(err, ValueError)
     assert "rows 12..20" in str(err) and "rows 8..24" in str(err)
+
+
+def test_fields_of_a_gather_share_a_device():
+    """The gather reads separate fields where they are, so one on another
+    device is refused before its address reaches a kernel."""
+    from types import SimpleNamespace
+
+    import torch
+
+    from b200sht.semilag import _check_fields
+
+    stencil = SimpleNamespace(source_shape=(4, 6, 8), tables=SimpleNamespace(dtype=torch.float32))
+    on = lambda k: SimpleNamespace(shape=(4, 6, 8), dtype=torch.float32, is_cuda=True,  # noqa: E731
+                                   device=torch.device("cuda", k))
+    _check_fields([on(0), on(0)], stencil)
+    with pytest.raises(ValueError, match="field 1 is on cuda:1 where field 0 is on cuda:0"):
+        _check_fields([on(0), on(1)], stencil)
