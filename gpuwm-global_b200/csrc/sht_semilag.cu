@@ -1440,6 +1440,10 @@ int sht_sl_gather_fields(const sht_sl_tables* tables, const sht_sl_window* win, 
     sht::set_error("fields must point to 1 to 2^20 source arrays");
     return SHT_ERR_ARG;
   }
+  if (reinterpret_cast<uintptr_t>(packed) % 16 != 0) {
+    sht::set_error("packed must be 16-byte aligned");
+    return SHT_ERR_ARG;
+  }
   if (win != nullptr && win->tables != tables) {
     sht::set_error("the band window belongs to other tables");
     return SHT_ERR_ARG;
@@ -1643,6 +1647,10 @@ int sht_sl_departure_maxima(const sht_sl_tables* tables, const sht_sl_window* wi
                             void* maxima, void* stream) {
   if (maxima == nullptr) {
     sht::set_error("maxima is NULL");
+    return SHT_ERR_ARG;
+  }
+  if (reinterpret_cast<uintptr_t>(maxima) % 16 != 0) {
+    sht::set_error("maxima must be 16-byte aligned");
     return SHT_ERR_ARG;
   }
   if (win != nullptr && win->tables != tables) {

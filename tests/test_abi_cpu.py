@@ -118,3 +118,16 @@ def test_latitude_band_edges_tile_the_grid():
         latitude_band_edges(0, 1)
     with pytest.raises(ValueError):
         latitude_band_edges(10, 0)
+
+
+def test_sl_buffers_that_vector_accesses_touch_must_be_aligned(lib):
+    from b200sht import _lib
+
+    null = [None] * 8
+    st = lib.sht_sl_departure_maxima(None, None, 0, 4, *null, 3, 300.0, 6.4e6, None, None, None,
+                                     ctypes.c_void_p(8), None)
+    assert st == _lib.SHT_ERR_ARG and b"maxima must be 16-byte aligned" in lib.sht_last_error()
+    one = (ctypes.c_void_p * 2)(16, 16)
+    st = lib.sht_sl_gather_fields(None, None, 4, 0, 0, one, 2, ctypes.c_void_p(24), 4, None, None,
+                                  None, None, None, None)
+    assert st == _lib.SHT_ERR_ARG and b"packed must be 16-byte aligned" in lib.sht_last_error()
