@@ -64,13 +64,16 @@ def _candidates(transform) -> list[dict]:
         pass
     finally:
         set_tuning(transform, fft=current["fft"])
+    # the default FP32 tile and the other one (128 columns from 256 latitude
+    # pairs on, 64 below)
+    tiles = [0, 1 if (transform.grid.nlat + 1) // 2 >= 256 else 2]
     fp32 = transform.precision != "float64"
     out = []
     for contraction, fft, order, simt_tile in itertools.product(
-            [0, 1] if split else [0], ffts, [0, 1] if split else [0], [0, 1] if fp32 else [0]):
+            [0, 1] if split else [0], ffts, [0, 1] if split else [0], tiles if fp32 else [0]):
         if contraction == 1 and order == 1:
             continue  # the tile order only steers the tensor-core kernel
-        if split and contraction == 0 and simt_tile == 1:
+        if split and contraction == 0 and simt_tile != 0:
             continue  # the SIMT tile shape only steers the SIMT contraction
         out.append({"contraction": contraction, "fft": fft, "tile_order": order, "tc_ctas": 0,
                     "accumulators": current["accumulators"], "simt_tile": simt_tile})

@@ -1518,9 +1518,9 @@ int sht_plan_set_tuning(sht_plan* plan, int key, int value) {
         plan->tune_accumulators = value;
         break;
       case SHT_TUNE_SIMT_TILE:
-        SHT_REQUIRE(value == 0 || value == 1, "SHT_TUNE_SIMT_TILE is 0 or 1");
+        SHT_REQUIRE(value >= 0 && value <= 2, "SHT_TUNE_SIMT_TILE is 0, 1 or 2");
         SHT_REQUIRE(value == 0 || plan->prec != SHT_PREC_F64,
-                    "SHT_TUNE_SIMT_TILE 1 (64-wide column tiles) is an FP32 tile shape");
+                    "SHT_TUNE_SIMT_TILE 1 and 2 (64- and 128-wide column tiles) are each an FP32 tile shape");
         plan->tune_simt_tile = value;
         break;
       default:

@@ -455,7 +455,8 @@ void launch_gemm_simt_groups(const sht_plan* p, int direction, int ngroups, cons
   // many CTAs; from 256 latitude pairs on the 128-wide ones' fewer table and
   // data reloads make up for it (T511 x 200 planes 1921 against 1955 us; T255 x
   // 161 planes 292 against 264, T126 x 200 planes 76 against 70).
-  const bool narrow = std::is_same<T, float>::value && (p->tune_simt_tile == 1 || p->H < 256);
+  const bool narrow = std::is_same<T, float>::value &&
+                      (p->tune_simt_tile == 1 || (p->tune_simt_tile == 0 && p->H < 256));
   const bool skinny = skinny_folded<T>(R);
   const int n_items = narrow && !skinny ? p->n_items_narrow[direction] : p->n_items[direction];
   if (n_items == 0 || R == 0) return;

@@ -67,7 +67,7 @@ struct sht_plan {
   int tune_contraction = 0;  // 1: FP32 SIMT contraction on a split16 plan
   int tune_tile_order = 0;   // tensor-core tile order (0: row blocks innermost, 1: column tiles)
   int tune_tc_ctas = 0;      // tensor-core CTAs per launch (0: one per SM)
-  int tune_simt_tile = 0;    // FP32 SIMT column tile (0: by size, 128 or 64 wide; 1: 64 wide)
+  int tune_simt_tile = 0;    // FP32 SIMT column tile (0: by size, 128 or 64 wide; 1: 64; 2: 128)
   int tune_accumulators = 0; // tensor-core accumulators (0: three K segments; 1: one, double-buffered;
                              // 2: two K segments, data operand in TMEM)
 

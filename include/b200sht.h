@@ -336,8 +336,9 @@ int sht_helmholtz_synthesis(sht_plan* plan, const sht_vertical* op, double tau_w
  *   SHT_TUNE_SIMT_TILE   FP32 SIMT contraction tile shape (columns x rows):
  *                        0: 128 x 64 from 256 latitude pairs on, 64 x 64
  *                        below; 1: 64 x 64 (less padding on the ragged
- *                        analysis blocks, more table loads); FP64 plans have
- *                        the one shape 64 x 32
+ *                        analysis blocks, more table loads); 2: 128 x 64; the
+ *                        results are the same bits; FP64 plans have the one
+ *                        shape 64 x 32
  * Set between calls, not while a call of the plan is in flight. */
 #define SHT_TUNE_CONTRACTION 0
 #define SHT_TUNE_FFT 1

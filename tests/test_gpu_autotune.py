@@ -41,6 +41,17 @@ def test_every_setting_meets_the_bar_and_tune_keeps_the_fastest(tmp_path):
     t.check_device()
 
 
+@pytest.mark.parametrize("T, nlat, tiles", [(62, 95, {0, 2}), (341, 514, {0, 1})])
+def test_candidate_tiles_differ(T, nlat, tiles):
+    """Both FP32 tile shapes are offered, each once, on either side of the
+    size where the default changes."""
+    from b200sht import SphericalHarmonicTransform
+    from b200sht.autotune import _candidates
+
+    t = SphericalHarmonicTransform.create(T, nlat=nlat, nlon=2 * nlat, precision="float32")
+    assert {c["simt_tile"] for c in _candidates(t)} == tiles
+
+
 def test_tuning_errors():
     from b200sht import SphericalHarmonicTransform
     from b200sht.autotune import set_tuning
@@ -80,9 +91,9 @@ def test_accumulator_plans_meet_the_bar_at_t255(acc):
 
 @pytest.mark.parametrize("precision", ["float32", "split16"])
 def test_simt_tile_shapes_agree_bit_for_bit(precision):
-    """The two FP32 SIMT tile shapes run every output's FFMA chain in the same
+    """The FP32 SIMT tile shapes run every output's FFMA chain in the same
     order, so they return the same bits (on a split16 plan through the SIMT
-    contraction switch)."""
+    contraction switch); the default is the narrow one at this size."""
     import torch
 
     from b200sht import SphericalHarmonicTransform
@@ -94,12 +105,14 @@ def test_simt_tile_shapes_agree_bit_for_bit(precision):
         set_tuning(t, contraction=1)
     coeff = red_spectrum(127, 5)
     out = []
-    for tile in (0, 1):
+    for tile in (0, 1, 2):
         set_tuning(t, simt_tile=tile)
         g = t.inverse(coeff)
         out.append((g.clone(), t.forward(g).clone()))
-    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+    for g, c in out[1:]:
+        assert torch.equal(out[0][0], g) and torch.equal(out[0][1], c)
     f64 = SphericalHarmonicTransform.create(21, precision="float64")
-    with pytest.raises(ValueError, match="FP32 tile shape"):
-        set_tuning(f64, simt_tile=1)
+    for tile in (1, 2):
+        with pytest.raises(ValueError, match="FP32 tile shape"):
+            set_tuning(f64, simt_tile=tile)
     t.check_device()

@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("precision", ["float64", "float32"])
 @pytest.mark.parametrize("T, nlat, nlon", [(9, 15, 30), (48, 74, 150), (62, 95, 192), (90, 137, 288),
-                                           (200, 302, 640)])
+                                           (200, 302, 640), (341, 514, 1026)])
 def test_a_plane_has_the_same_bits_in_every_batch(T, nlat, nlon, precision):
     import torch
 
