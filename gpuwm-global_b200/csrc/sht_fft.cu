@@ -483,10 +483,11 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) inverse_unfold_ke
     const V2<T>* D2 = reinterpret_cast<const V2<T>*>(wD) + (int64_t)h * a.ldc + plane * FW;
     const int64_t dsd = (int64_t)a.H * a.ldc;  // S row -> D row of the same order
     const T inv_a = T(1.0 / a.radius);
-    T ie[2] = {T(0), T(0)};  // 1 / (a cos phi) of the two sides
+    Reciprocal<T> over_a{}, ie[2]{};  // 1 / a, and 1 / (a cos phi) of the two sides
+    if constexpr (NF == 2) over_a = reciprocal(T(a.radius));
     if constexpr (NF != 1) {
-      ie[0] = T(1) / (T(a.radius) * T(coslat[h]));
-      ie[1] = T(1) / (T(a.radius) * T(coslat[a.nlat - 1 - h]));
+      ie[0] = reciprocal(T(a.radius) * T(coslat[h]));
+      ie[1] = reciprocal(T(a.radius) * T(coslat[a.nlat - 1 - h]));
     }
     // x[o][sd]: order m of output field o on side sd
     auto order_values = [&](int m, V2<T>(&x)[NO][2]) {
@@ -508,12 +509,12 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) inverse_unfold_ke
           x[0][sd] = a.zonal ? mk2<T>(-mf * v[0].y, mf * v[0].x) : v[0];
         } else if constexpr (NF == 2) {
           // east: i m P / (a cos phi); north: dP / a
-          x[0][sd] = mk2<T>(-mf * v[0].y * ie[sd], mf * v[0].x * ie[sd]);
-          x[1][sd] = mk2<T>(v[1].x * inv_a, v[1].y * inv_a);
+          x[0][sd] = mk2<T>(times(-mf * v[0].y, ie[sd]), times(mf * v[0].x, ie[sd]));
+          x[1][sd] = mk2<T>(times(v[1].x, over_a), times(v[1].y, over_a));
         } else {
           // v = {P psi, P chi, dP psi, dP chi}: u = -dpsi/a + i m chi/(a cos),
           // v = i m psi/(a cos) + dchi/a
-          const T im = mf * ie[sd];
+          const T im = times(mf, ie[sd]);
           x[0][sd] = mk2<T>(-v[2].x * inv_a - im * v[1].y, -v[2].y * inv_a + im * v[1].x);
           x[1][sd] = mk2<T>(-im * v[0].y + v[3].x * inv_a, im * v[0].x + v[3].y * inv_a);
         }

@@ -492,7 +492,7 @@ __global__ void __launch_bounds__(InvCfg<NF>::W * 32, 16 / InvCfg<NF>::W)
   for (int k = threadIdx.x; k < 32 * FF; k += blockDim.x) twn[k] = twN[k];
   // warp w: slots w, w + kW, ...; slot s = (gg * NO + o) * 2 + side
   const int side = warp & 1, o = (warp >> 1) % NO, gp = (warp >> 1) / NO;
-  const float inv_a = 1.0f / a.radius;
+  const Reciprocal<float> over_a = reciprocal(a.radius);
   for (; item < n_items; item += gridDim.x) {
     const int h = (int)(item / n_pb);
     const int64_t p0 = (item - (int64_t)h * n_pb) * GI;
@@ -503,10 +503,10 @@ __global__ void __launch_bounds__(InvCfg<NF>::W * 32, 16 / InvCfg<NF>::W)
     const int T = TC >= 0 ? TC : a.T;
     const int T1 = T + 1;
     // Row scale factors of the two sides: 1 / (a cos phi) (gradient, wind).
-    float ie[2] = {0.f, 0.f};
+    Reciprocal<float> ie[2] = {};
     if constexpr (NF != 1) {
-      ie[0] = 1.0f / (a.radius * (float)coslat[h]);
-      ie[1] = 1.0f / (a.radius * (float)coslat[jmir]);
+      ie[0] = reciprocal(a.radius * (float)coslat[h]);
+      ie[1] = reciprocal(a.radius * (float)coslat[jmir]);
     }
     // x[o][sd]: the spectrum of order j (j <= T) of output field o on side
     // sd, from the symmetric and antisymmetric parts of plane g.
@@ -531,11 +531,11 @@ __global__ void __launch_bounds__(InvCfg<NF>::W * 32, 16 / InvCfg<NF>::W)
         } else if constexpr (NF == 2) {
           // gradient: (i m P) / (a cos phi) east, (dP) / a north; the
           // divisions applied here, ahead of the (linear) FFT
-          x[0][sd] = make_float2(-mf * v[0].y * ie[sd], mf * v[0].x * ie[sd]);
-          x[1][sd] = make_float2(v[1].x * inv_a, v[1].y * inv_a);
+          x[0][sd] = make_float2(times(-mf * v[0].y, ie[sd]), times(mf * v[0].x, ie[sd]));
+          x[1][sd] = make_float2(times(v[1].x, over_a), times(v[1].y, over_a));
         } else {
           // v = {P psi, P chi, dP psi, dP chi}
-          const float im_over = mf * ie[sd];
+          const float im_over = mf * ie[sd].hi, inv_a = over_a.hi;
           x[0][sd] = make_float2(-v[2].x * inv_a - im_over * v[1].y, -v[2].y * inv_a + im_over * v[1].x);
           x[1][sd] = make_float2(-im_over * v[0].y + v[3].x * inv_a, im_over * v[0].x + v[3].y * inv_a);
         }
