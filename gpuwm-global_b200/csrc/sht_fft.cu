@@ -166,6 +166,12 @@ __device__ __forceinline__ void dft_odd(V2<T>* v) {
       const T s = T(e <= H ? OddTrig<R>::s(e) : -OddTrig<R>::s(R - e));
       a.x += c * t[i - 1].x;
       a.y += c * t[i - 1].y;
+      if constexpr (R == 3) {  // the product rounds with the sum it goes into
+        const T t = INV ? -s : s;
+        v[1] = mk2<T>(fma(t, u[0].y, a.x), fma(-t, u[0].x, a.y));
+        v[2] = mk2<T>(fma(-t, u[0].y, a.x), fma(t, u[0].x, a.y));
+        return;
+      }
       b.x += s * u[i - 1].x;
       b.y += s * u[i - 1].y;
     }
