@@ -489,23 +489,27 @@ int sht_sl_gather_linear(const sht_sl_tables* tables, const void* src, int64_t f
  * (continuous zonal index), phi (radians), level (continuous level index,
  * clamped to [-1/2, nlev - 1/2]) and the last iteration's move in metres
  * and in levels.  radius: the sphere's radius in metres. */
+int sht_sl_departure(const sht_sl_tables* tables, int nlev, const void* vx, const void* vy,
+                     const void* vz, const void* level_rate, const void* vx_ex,
+                     const void* vy_ex, const void* vz_ex, const void* level_rate_ex,
+                     int iterations, double dt, double radius, void* xi, void* phi,
+                     void* level, void* move_m, void* move_k, void* stream);
 /* The search with the trajectory diagnostics in place of the move arrays, on
  * the whole grid or (window) a band, by solver 0 (fixed point), 1 (Newton) or
  * 2 (line-search Newton): maxima[6], device memory of the tables' element type,
- * 16-byte aligned and zeroed by the caller, receives the largest last move in metres, in meridional
- * grid lengths and in levels, then the largest displacement in the same three
- * (NaN where one is NaN). */
+ * 16-byte aligned and zeroed by the caller, receives the largest last move in
+ * metres, in meridional grid lengths and in levels, then the largest
+ * displacement in the same three.
+ * A wind that is not finite leaves its points' xi and phi NaN, and with them the
+ * displacement in metres and grid lengths; the last move is NaN only from the
+ * line-search solver (the others count such a point's as 0), and level values
+ * never are: a NaN level is the lowest interface, -1/2. */
 int sht_sl_departure_maxima(const sht_sl_tables* tables, const struct sht_sl_window* window,
                             int solver, int nlev, const void* vx, const void* vy, const void* vz,
                             const void* level_rate, const void* vx_ex, const void* vy_ex,
                             const void* vz_ex, const void* level_rate_ex, int iterations,
                             double dt, double radius, void* xi, void* phi, void* level,
                             void* maxima, void* stream);
-int sht_sl_departure(const sht_sl_tables* tables, int nlev, const void* vx, const void* vy,
-                     const void* vz, const void* level_rate, const void* vx_ex,
-                     const void* vy_ex, const void* vz_ex, const void* level_rate_ex,
-                     int iterations, double dt, double radius, void* xi, void* phi,
-                     void* level, void* move_m, void* move_k, void* stream);
 /* The same search solved by Newton's method (the reference's opt-in
  * "newton" solver of trajectory.departure_points): per iteration the
  * residual of the fixed-point map in the local east / north / level frame

@@ -82,10 +82,19 @@ def test_search_maxima_match_the_move_arrays(dtype, tol, solver):
     got = [d.move_max_m, d.move_max_cells, d.move_max_levels, d.displacement_max_m,
            d.displacement_max_cells, d.displacement_max_levels]
     np.testing.assert_allclose(got, want, rtol=tol)
-    wind[3][2, 5, 6] = float("nan")  # a NaN level rate reaches the level maxima
-    _, d = departure_points(CartesianWind(*wind), tables, 300.0, solver=solver)
-    assert np.isnan(d.displacement_max_levels) == bool(torch.isnan(
-        departure_points(CartesianWind(*wind), tables, 300.0, solver=solver)[0].level).any())
+    # a NaN level rate is clamped to the lowest interface, no NaN in any level
+    wind[3][2, 5, 6] = float("nan")
+    st, d = departure_points(CartesianWind(*wind), tables, 300.0, solver=solver)
+    assert float(st.level[2, 5, 6]) == -0.5 and not bool(torch.isnan(st.level).any())
+    assert 2.5 <= d.displacement_max_levels < lev.shape[0]
+    # a NaN horizontal wind leaves the displacement NaN, whatever the solver,
+    # and the last move only where the line search reports the step at the point
+    wind[0][3, 9, 12] = float("nan")
+    st, d = departure_points(CartesianWind(*wind), tables, 300.0, solver=solver)
+    assert bool(torch.isnan(st.xi[3, 9, 12])) and bool(torch.isnan(st.phi[3, 9, 12]))
+    assert np.isnan(d.displacement_max_m) and np.isnan(d.displacement_max_cells)
+    assert np.isnan(d.move_max_m) == np.isnan(d.move_max_cells) == (solver == "newton_ls")
+    assert np.isfinite([d.move_max_levels, d.displacement_max_levels]).all()
 
 
 @pytest.mark.parametrize("dtype", ["float64", "float32"])
