@@ -163,3 +163,40 @@ def test_more_levels_or_rows_than_a_grid_dimension(shape):
                        [:, None, None].expand(shape))
     assert float((st.phi - torch.as_tensor(lat, device="cuda")[None, :, None]).abs().max()) < 1e-12
     assert d.displacement_max_levels == 0.0 and d.displacement_max_m < 1e-6
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+def test_block_and_move_array_entries(dtype):
+    """The C entries beside the ones the Python calls take: gathers of one
+    contiguous block and the band search with move arrays, bit for bit."""
+    import torch
+
+    from b200sht import _lib
+    from b200sht.semilag import CartesianWind, Stencil, departure_points, gather_batch
+
+    tables, at, field = _setup(getattr(torch, dtype))
+    block = torch.stack([field() for _ in range(3)])
+    ptr = lambda t: t.data_ptr()  # noqa: E731
+    stream = torch.cuda.current_stream().cuda_stream
+    nlev = block.shape[1]
+    band = tables.window(slice(4, 30), slice(9, 24))
+    for window in (None, band):
+        pts = [x if window is None else x[:, 9:24].contiguous() for x in at]
+        src = block if window is None else block[:, :, 4:30].contiguous()
+        want = gather_batch(list(src), Stencil(*pts, tables=tables, window=window))
+        got = torch.empty((3, *pts[0].shape), dtype=block.dtype, device="cuda")
+        name, handle = (("sht_sl_gather", tables._handle) if window is None
+                        else ("sht_sl_gather_band", window._handle))
+        _lib.call(name, handle, 4, _lib.SHT_SL_QUASI_MONOTONE, 0, ptr(src), 3, nlev,
+                  *[ptr(x) for x in pts], ptr(got), None, stream)
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+    wind = [30.0 * field()[:, 4:30].contiguous() for _ in range(3)]
+    wind.append(1e-3 * field()[:, 4:30].contiguous())
+    ahead = [w[:, band.local].contiguous() for w in wind]
+    st, d = departure_points(CartesianWind(*wind), tables, 300.0, window=band,
+                             extrapolated=CartesianWind(*ahead))
+    outs = [torch.empty_like(st.xi) for _ in range(5)]
+    _lib.call("sht_sl_departure_band", band._handle, 0, nlev, *[ptr(x) for x in wind + ahead], 3,
+              300.0, tables.radius_m, *[ptr(x) for x in outs], stream)
+    assert all(torch.equal(a, b) for a, b in zip((st.xi, st.phi, st.level), outs))
+    assert d.move_max_m == float(outs[3].max()) and d.move_max_levels == float(outs[4].max())
