@@ -7,13 +7,13 @@ semilag/interpolate.py:87-500) and the fixed-point departure search of
 ``arwen_global.semilag.trajectory`` (``CartesianWind``, ``cartesian_wind``,
 ``local_wind``, ``departure_points``, ``TrajectoryDiagnostics``) with the same
 argument meaning and the same ``ValueError`` wording; the interpolation and
-the search run in ``libb200sht.so`` (``sht_sl_gather``,
-``sht_sl_gather_linear``, ``sht_sl_departure``).  Arrays are CUDA tensors:
+the search run in ``libb200sht.so`` (``sht_sl_gather_fields``,
+``sht_sl_gather_linear``, ``sht_sl_departure_maxima``).  Arrays are CUDA tensors:
 fields and departure coordinates ``(nlev, nlat, nlon)`` in the tables'
 dtype (float32 or float64).  Latitude-band windows (the reference's
 ``BandWindow``, ``HaloEscape``, ``SphericalGridTables.window``) give the
 banded step's gathers and searches over a band's rows from fields that hold
-the band and its halo (``sht_sl_gather_band``, ``sht_sl_departure_band``).
+the band and its halo (the same calls with the window's handle).
 The search's gate is the reference's too (trajectory.py:121-155, 755-1560):
 ``lipschitz`` (the flow deformation, one kernel: ``sht_sl_lipschitz``),
 ``LipschitzDiagnostics``, ``refuse_trajectory_fold``, ``convergence``,

@@ -635,7 +635,7 @@ void destroy(sht_plan* p) {
   }
   for (cudaEvent_t e : p->event_pool) cudaEventDestroy(e);
   void* ptrs[] = {p->d_mu, p->d_w, p->d_coslat, p->basis, p->dbasis, p->analysis, p->rot,
-                  p->shear, p->tw_l, p->tw_n, p->tw_lane, p->d_radices, p->d_items[0], p->d_items[1],
+                  p->shear, p->tw_l, p->tw_n, p->tw_lane, p->d_items[0], p->d_items[1],
                   p->d_items_narrow[0], p->d_items_narrow[1],
                   p->d_desc[0][0], p->d_desc[0][1], p->d_desc[1][0], p->d_desc[1][1],
                   p->wfold[0], p->wfold[1], p->cfold[0], p->cfold[1], p->rowmax, p->d_err};

@@ -60,7 +60,6 @@ struct sht_plan {
   void* tw_n = nullptr;
   void* tw_lane = nullptr;         // [k1][lane] table of the register kernels
   std::vector<int> radices;
-  int* d_radices = nullptr;
   bool fast_fft = false;           // register-resident kernels (sht_fft_fast.cu)
   bool force_generic_fft = false;  // SHT_FLAG_GENERIC_FFT
   // Autotuner settings (sht_plan_set_tuning).

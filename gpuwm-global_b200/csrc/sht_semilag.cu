@@ -552,7 +552,6 @@ struct SlDepArgs {
   // (the same three), in place of the move arrays.
   T* maxima;
   int iters, nk, nj, ni, nb;
-  double dlam;  // 2 pi / nlon (the arrival longitudes are formed in double)
   T dt, radius, inv_dlam, lut_scale;
   // Latitude-band form: the advecting wind holds njs rows starting `lead`
   // rows above the first arrival row, grid row ja0; the extrapolated wind
@@ -676,7 +675,7 @@ __global__ void __launch_bounds__(256) sl_departure_kernel(const SlDepArgs<T> a)
   const int64_t gid = ((int64_t)k * a.nja + j) * a.ni + i;
   // the arrival point in the advecting wind's held rows
   const int64_t here = ((int64_t)k * a.njs + (j + a.lead)) * a.ni + i;
-  // the arrival point (its longitude is i * dlam formed in double, as the
+  // the arrival point, from the table (its longitudes formed in double, as the
   // host computes the grid's)
   const T sph = __ldg(a.trig + a.ja0 + j), cph = __ldg(a.trig + a.nj + a.ja0 + j);
   const T sla = __ldg(a.trig + 2 * a.nj + i), cla = __ldg(a.trig + 2 * a.nj + a.ni + i);
@@ -1606,7 +1605,7 @@ static int departure_entry(int solver, const sht_sl_window* win, const sht_sl_ta
       a->iters = iterations; a->nk = nlev; a->nj = tables->nlat; a->ni = tables->nlon;
       a->nb = w.bins;
       const double dlam = 2.0 * kPi / tables->nlon;
-      a->dt = (T)dt; a->radius = (T)radius; a->dlam = dlam; a->inv_dlam = (T)(1.0 / dlam);
+      a->dt = (T)dt; a->radius = (T)radius; a->inv_dlam = (T)(1.0 / dlam);
       a->lut_scale = (T)w.lut_scale;
       a->njs = a->nja = tables->nlat;
       a->ja0 = a->lead = 0;
