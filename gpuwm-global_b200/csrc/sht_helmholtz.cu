@@ -474,8 +474,8 @@ __global__ void __launch_bounds__(256) semi_implicit_kernel(
 // serves 4 columns and a loaded coefficient RT rows; the general kernel above
 // holds 6 rows x 1 column and reads a 16-byte matrix piece per 8 multiply-adds.
 // The next item's x comes in by cp.async behind the products.  Blocks above the
-// triangle are zeroed by the same launch.  T255 x 40 levels FP32: 88 -> 64 us,
-// T511 288 -> 249 us; what is left waits for instructions and for the serial
+// triangle are zeroed by the same launch.  T255 x 40 levels FP32: 87 -> 62 us,
+// T511 268 -> 217 us (launches of a graph); what is left waits for instructions and for the serial
 // products (6 warps an SM, 25 % of the FMA pipe).
 template <typename T> struct SolveCfg { static constexpr int RT = sizeof(T) == 4 ? 8 : 4; };
 constexpr int kSolveCols = 64;
@@ -791,6 +791,29 @@ __global__ void __launch_bounds__(224) semi_solve_kernel(
   }
 }
 
+// A CTA of the solve kernel first lays out the operators and then takes 64
+// coefficients at a time on few warps, so a wave of it costs several items of
+// the general kernel on every SM: it is the faster one from so many general items
+// per SM and wave on (fewer where the general kernel, too, has an SM to a CTA
+// and two passes over its rows), and in FP32 from a third of a wave on.  Solve
+// and general kernel, us on the device: FP32 L40 T126 35 / 32, T170 35 / 42, T191
+// (a second wave nearly empty) 50 / 46, T255 62 / 87; L8 T62 17 / 7, T191 18 / 16,
+// T255 18 / 30; L41 (one CTA to an SM) T511 322 / 285; L60 T62 36 / 30, T85 37 /
+// 51; FP64 L16 T85 17 / 14, T126 20 / 23, L40 T85 33 / 31, T106 33 / 44.
+template <typename T>
+bool solve_is_faster(int64_t items, int fit, int64_t pairs, int slots) {
+  int dev = 0, sms = 0;
+  SHT_CUDA_OR_THROW(cudaGetDevice(&dev));
+  SHT_CUDA_OR_THROW(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  if (slots == 0) return false;
+  const int64_t waves = div_up(pairs, slots);
+  const double per_wave = (double)items / (double)(sms * waves);
+  const bool alone = fit <= sms;
+  if (sizeof(T) == 8) return per_wave >= (alone ? 2.5 : 3.4);
+  if (alone) return per_wave >= 1.5;
+  return per_wave >= (waves == 1 ? 5.0 : 6.0) && 3 * pairs >= slots;
+}
+
 }  // namespace
 
 template <typename T>
@@ -805,28 +828,27 @@ void launch_semi_implicit(const sht_plan* p, int nlev, const T* mats, bool has_t
   SHT_REQUIRE(mode != kSemiHalf || has_thermo,
               "half_apply needs the thermodynamic block's modes (sht_vertical_create_modes)");
   const SemiArgs a{p->T, nlev, mode, p->radius, dt, alpha, ldc};
-  // The stage solve by its own kernel while its operators and three vectors fit
-  // an SM (FP32 to about 66 levels, FP64 to about 40); the general kernel keeps
-  // the other maps and more levels.
-  int threads = 0;
-  const size_t solve = solve_smem<T>(nlev, &threads);
-  if (mode == kSemiSolve && threads <= 224 && solve + 2048 <= 227 * 1024) {
-    const int fit = resident_ctas((const void*)semi_solve_kernel<T>, threads, solve);
-    SHT_REQUIRE(fit > 0, "semi-implicit solve does not fit on an SM at this nlev");
-    const int64_t nmb = div_up(p->T + 1, 32);
-    const int64_t items = div_up(nmb * (p->T + 1) - 16 * nmb * (nmb - 1), 2);
-    const int ctas = (int)std::min<int64_t>(items, fit);
-    semi_solve_kernel<T><<<ctas, threads, solve, s>>>(
-        a, mats, (const V2<T>*)div, (const V2<T>*)theta, (const V2<T>*)lnps, (V2<T>*)odiv,
-        (V2<T>*)otheta, (V2<T>*)olnps, metric, (V2<T>*)cfold, rowmax);
-    SHT_CUDA_OR_THROW(cudaGetLastError());
-    return;
-  }
   const SmemPlan sp = smem_plan(nlev, mode);
   const size_t sm = sizeof(T) * (size_t)sp.nmat + sizeof(V2<T>) * 32 * (size_t)(sp.nvec * sp.vp);
   const int fit = resident_ctas((const void*)semi_implicit_kernel<T>, 256, sm);
   SHT_REQUIRE(fit > 0, "semi-implicit kernel does not fit on an SM at this nlev");
-  const int64_t items = div_up(p->T + 1, 32) * (int64_t)(p->T + 1);
+  const int64_t nmb = div_up(p->T + 1, 32), items = nmb * (p->T + 1);
+  // The stage solve by its own kernel where its operators and three vectors fit
+  // an SM (FP32 to about 66 levels, FP64 to about 40) and where it is faster.
+  int threads = 0;
+  const size_t solve = solve_smem<T>(nlev, &threads);
+  if (mode == kSemiSolve && threads <= 224 && solve + 2048 <= 227 * 1024) {
+    const int slots = resident_ctas((const void*)semi_solve_kernel<T>, threads, solve);
+    const int64_t pairs = div_up(items - 16 * nmb * (nmb - 1), 2);
+    if (solve_is_faster<T>(items, fit, pairs, slots)) {
+      const int ctas = (int)std::min<int64_t>(pairs, slots);
+      semi_solve_kernel<T><<<ctas, threads, solve, s>>>(
+          a, mats, (const V2<T>*)div, (const V2<T>*)theta, (const V2<T>*)lnps, (V2<T>*)odiv,
+          (V2<T>*)otheta, (V2<T>*)olnps, metric, (V2<T>*)cfold, rowmax);
+      SHT_CUDA_OR_THROW(cudaGetLastError());
+      return;
+    }
+  }
   const int ctas = (int)std::min<int64_t>(items, fit);
   semi_implicit_kernel<T><<<ctas, dim3(32, 8), sm, s>>>(
       a, mats, (const V2<T>*)div, (const V2<T>*)theta, (const V2<T>*)lnps, (V2<T>*)odiv,

@@ -1,6 +1,7 @@
 """The stage solve at level counts around its row tiles and its shared-memory
-limit (beyond which the general kernel runs), and at truncations around its
-32-order blocks, against the oracle; and fused onto the synthesis."""
+limit, and at truncations around its 32-order blocks, on both sides of the
+sizes from which its own kernel runs, against the oracle; and fused onto the
+synthesis."""
 from __future__ import annotations
 
 import numpy as np
@@ -11,7 +12,10 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("precision, tol", [("float64", 1e-11), ("float32", 1e-5)])
 @pytest.mark.parametrize("T, nlev", [(5, 1), (31, 7), (32, 8), (33, 9), (63, 15), (40, 16),
-                                     (21, 47), (21, 48), (21, 75), (21, 80)])
+                                     (21, 47), (21, 48), (21, 75), (21, 80),
+                                     # by the kernel of its own
+                                     (223, 1), (223, 7), (224, 8), (223, 9), (223, 15), (160, 16),
+                                     (170, 40), (170, 41), (96, 50), (96, 66)])
 def test_solve_against_the_oracle(T, nlev, precision, tol):
     import torch
 
