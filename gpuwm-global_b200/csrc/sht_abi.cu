@@ -497,7 +497,8 @@ void contract_batch(sht_batch* b, int kind, T* const* data, T* const* out, cudaS
       return;
     }
   }
-  for (int i = 0; i < n; ++i) contract<T>(b->plans[i], kind, data[i], out[i], 2 * padded_cols(b->planes[i]), s);
+  for (int i = 0; i < n; ++i)
+    contract<T>(b->plans[i], kind, data[i], out[i], 2 * padded_cols(b->planes[i]), s);
 }
 
 template <typename T>
@@ -519,7 +520,7 @@ void do_batch_forward(sht_batch* b, const void* const* grids, void* const* coeff
   for (int i = 0; i < n; ++i) {
     KernelScope k(b->plans[i], SHT_KIND_UNPACK, s);
     launch_unpack<T>(b->plans[i], kUnpackScalar, c[i], nullptr, b->planes[i],
-                     padded_cols(b->planes[i]),                     static_cast<T*>(coeffs[i]), nullptr, s);
+                     padded_cols(b->planes[i]), static_cast<T*>(coeffs[i]), nullptr, s);
   }
 }
 
@@ -542,7 +543,7 @@ void do_batch_inverse(sht_batch* b, const void* const* coeffs, void* const* grid
   for (int i = 0; i < n; ++i) {
     KernelScope k(b->plans[i], SHT_KIND_FFT_INVERSE, s);
     launch_inverse_unfold<T>(b->plans[i], kUnfoldScalar, w[i], nullptr, b->planes[i],
-                             padded_cols(b->planes[i]),                             static_cast<T*>(grids[i]), nullptr, s);
+                             padded_cols(b->planes[i]), static_cast<T*>(grids[i]), nullptr, s);
   }
 }
 

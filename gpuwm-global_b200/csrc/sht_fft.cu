@@ -657,7 +657,7 @@ FftShape make_shape(const sht_plan* p, int64_t cols, int no, size_t* smem, int* 
   const size_t table = (size_t)p->L * sizeof(V2<T>);
   int lc = 0;
   while (lc < 3 && ((int64_t)1 << lc) < cols && bytes(lc + 1) + table <= kTarget) ++lc;
-  while (lc > 0 && p->H * div_up(cols, (int64_t)1 << lc) < 2 * 148) --lc;
+  while (lc > 0 && p->H * div_up(cols, (int64_t)1 << lc) < 2 * 148) --lc;  // two to an SM
   f.lc = lc;
   f.rs = stride(lc);
   f.tw_shared = bytes(lc) + table <= kMost ? 1 : 0;

@@ -26,10 +26,11 @@ namespace {
 // (fma.rn.f32x2), which halves the issue slots of the multiply-adds, and 8 x 8
 // outputs per thread leave 16 warps on an SM; 8 x 16 with 8 warps measured the
 // same at T511 and 10 to 25 % slower at T255 and T126, where the chain per tile
-// is short.  Analysis + synthesis against one element per instruction in
-// 128 x 128 tiles of 256 threads loaded through registers: T511 x 200 planes
-// 2716 -> 1921 us (42 TF/s), T255 x 161 planes 444 -> 264 us, T126 x 200 planes
-// 103 -> 70 us.  Each output element is one chain of fused multiply-adds over
+// is short.  (The 128-wide FP32 tile spills 56 bytes a thread at its 128
+// registers, the 64-wide one 24.)  Analysis + synthesis against one element per
+// instruction in 128 x 128 tiles of 256 threads loaded through registers, by
+// events around the launches: T511 x 200 planes 2716 -> 2002 us (40 TF/s), T255 x
+// 161 planes 444 -> 278 us, T126 x 200 planes 103 -> 73 us.  Each output element is one chain of fused multiply-adds over
 // ascending k from zero, whatever the tile, so every tile shape returns the
 // same bits.
 template <typename T> struct SimtCfg {
@@ -70,7 +71,9 @@ __device__ __forceinline__ void cp_async(uint32_t dst, const void* src, bool liv
 }
 
 // One CTA tile.  DB: bytes of a data-row copy, 16 where every data row starts
-// on a 16-byte boundary and 8 otherwise (FP32 with an odd plane count).
+// on a 16-byte boundary and 8 otherwise (FP32 with an odd plane count, which only
+// the static-scratch forward has: its fixed buffer holds the exact columns, and a
+// padded one would refuse calls that fit).
 template <typename T, int WX, int GN, int DB>
 __device__ __forceinline__ void simt_tile(const SimtGroup<T>& G, const ShtGemmDesc& d, int x0,
                                           int64_t r0, int64_t R, T* smem) {
@@ -453,8 +456,9 @@ void launch_gemm_simt_groups(const sht_plan* p, int direction, int ngroups, cons
                              int64_t R, cudaStream_t s) {
   // 64-wide tiles waste less of the ragged analysis blocks and hold twice as
   // many CTAs; from 256 latitude pairs on the 128-wide ones' fewer table and
-  // data reloads make up for it (T511 x 200 planes 1921 against 1955 us; T255 x
-  // 161 planes 292 against 264, T126 x 200 planes 76 against 70).
+  // data reloads make up for it (128 and 64 wide, us: T511 x 200 planes 2002 and
+  // 2023, T341 x 100 planes 438 and 443; T255 x 161 planes 302 and 278, T126 x 200
+  // planes 77 and 73).
   const bool narrow = std::is_same<T, float>::value &&
                       (p->tune_simt_tile == 1 || (p->tune_simt_tile == 0 && p->H < 256));
   const bool skinny = skinny_folded<T>(R);

@@ -301,7 +301,12 @@ __global__ void __launch_bounds__(256) sl_pack_kernel(const __grid_constant__ Pa
 // limiter at T511 L40: 16.2 ms one float per load, 9.9 ms four (the L1's 128
 // bytes a clock would take 5.4 ms: it waits for the taps at 16 warps an SM), 9.3
 // ms in CTAs of 128 points, five to an SM (FP64: four); and 0.98 ms to interleave
-// against 0.89 ms for the copy.
+// against 0.89 ms for the copy.  The quintic in groups keeps to 128 registers and
+// spills (FP32 to 276 bytes a thread, FP64 to 344) and is faster all the same:
+// 16 fields at T511 x 12 levels, copy or interleaving included, one value a load
+// -> groups: cubic limited 5.16 -> 3.17 ms, unlimited 4.96 -> 2.83, quintic
+// limited 11.1 -> 7.1, unlimited 13.0 -> 7.2; FP64 8.7 -> 6.7, 7.4 -> 6.0, 20.1 ->
+// 14.8, 17.1 -> 14.9.
 template <typename T, int NH, int VEC, bool EACH, bool QM, bool DEF>
 __global__ void __launch_bounds__(kGatherX * kGatherY * kGatherZ,
                                   NH == 6 || sizeof(T) == 8 ? 4 : (VEC == 4 ? 5 : 6))

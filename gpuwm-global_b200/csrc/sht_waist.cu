@@ -29,7 +29,8 @@ template <typename T>
 __global__ void __launch_bounds__(256) waist_export_kernel(int Tn, int H, int nlat, int nlat_odd,
                                                            double c, int zonal,
                                                            const V2<T>* __restrict__ wf,
-                                                           int64_t planes, int64_t ldc, V2<T>* __restrict__ out) {
+                                                           int64_t planes, int64_t ldc,
+                                                           V2<T>* __restrict__ out) {
   __shared__ V2<T> tile[2][32][33];  // [side][plane][order]
   const int m0 = blockIdx.x * 32;
   const int h = blockIdx.y;
@@ -139,8 +140,8 @@ __global__ void __launch_bounds__(256) waist_import_kernel(int Tn, int H, int nl
 }  // namespace
 
 template <typename T>
-void launch_waist_export(const sht_plan* p, const T* wfold, int64_t planes, int64_t ldc, double c, int zonal,
-                         T* waist, cudaStream_t s) {
+void launch_waist_export(const sht_plan* p, const T* wfold, int64_t planes, int64_t ldc, double c,
+                         int zonal, T* waist, cudaStream_t s) {
   if (planes == 0) return;
   dim3 grid((unsigned)div_up(p->T + 1, 32), (unsigned)p->H, (unsigned)div_up(planes, 32));
   SHT_REQUIRE(grid.z <= 65535, "too many planes for one waist launch");
@@ -151,8 +152,8 @@ void launch_waist_export(const sht_plan* p, const T* wfold, int64_t planes, int6
 }
 
 template <typename T>
-void launch_waist_import(const sht_plan* p, const T* waist, int64_t planes, int64_t ldc, double c, T* wfold,
-                         float* rowmax, cudaStream_t s, int fields) {
+void launch_waist_import(const sht_plan* p, const T* waist, int64_t planes, int64_t ldc, double c,
+                         T* wfold, float* rowmax, cudaStream_t s, int fields) {
   if (planes == 0) return;
   SHT_REQUIRE(fields >= 1 && planes % fields == 0, "waist import: planes not a multiple of fields");
   dim3 grid((unsigned)div_up(p->T + 1, 32), (unsigned)p->H, (unsigned)div_up(planes, 32));
@@ -164,10 +165,10 @@ void launch_waist_import(const sht_plan* p, const T* waist, int64_t planes, int6
 }
 
 #define INST(T)                                                                                  \
-  template void launch_waist_export<T>(const sht_plan*, const T*, int64_t, int64_t, double, int, T*,     \
-                                       cudaStream_t);                                           \
-  template void launch_waist_import<T>(const sht_plan*, const T*, int64_t, int64_t, double, T*, float*,  \
-                                       cudaStream_t, int);
+  template void launch_waist_export<T>(const sht_plan*, const T*, int64_t, int64_t, double, int, \
+                                       T*, cudaStream_t);                                       \
+  template void launch_waist_import<T>(const sht_plan*, const T*, int64_t, int64_t, double, T*, \
+                                       float*, cudaStream_t, int);
 INST(float)
 INST(double)
 #undef INST

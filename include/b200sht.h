@@ -421,7 +421,8 @@ int sht_batch_inverse(sht_batch* batch, const void* const* coeffs, void* const* 
  * their own (fields: host array of device pointers), on the whole grid or,
  * with a window, on its band: the volumes are interleaved into `packed`
  * (count source volumes of room, 16-byte aligned; not needed for count 1,
- * whose volume is read in place) and gathered several to a load.
+ * whose volume is read in place) and gathered several to a load; three odd
+ * volumes, and three or five of double, are read where they are.
  * Stream-ordered; every pointer is device memory the caller owns. */
 typedef struct sht_sl_tables sht_sl_tables;
 #define SHT_SL_NONE 0
