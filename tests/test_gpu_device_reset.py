@@ -59,3 +59,22 @@ def test_plans_made_after_a_device_reset_launch():
     done = subprocess.run([sys.executable, "-c", CHILD, str(build.LIB_PATH)], capture_output=True,
                           text=True, timeout=300)
     assert done.returncode == 0, done.stderr
+
+
+def test_a_capture_may_raise_the_limits():
+    """A plan made after another was warm marks the limits as not raised; the
+    warm plan's next launches raise them inside a stream capture."""
+    import torch
+
+    from b200sht import SphericalHarmonicTransform
+
+    t = SphericalHarmonicTransform.create(169, nlat=256, nlon=512)
+    grid = torch.randn(6, 256, 512, device="cuda")
+    want = t.inverse(t.forward(grid))
+    SphericalHarmonicTransform.create(21, nlat=33, nlon=66)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = t.inverse(t.forward(grid))
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
